@@ -34,6 +34,7 @@ constexpr int NT_CTA = 256;   // threads per CTA of every tile kernel
 constexpr int KC     = 32;    // k-extent of one pipeline stage
 constexpr int IB     = 64;    // inner block of POTRF / TRSM (inverted diagonal blocks)
 constexpr int LDD    = IB + 1;// leading dimension of the inner block in shared memory
+constexpr int LEAF_LD = IB + 4;   // the same in the 64 x 64 leaf (rec.cuh)
 
 enum SplitKind : int { SPLIT_BF16X3 = 0, SPLIT_TF32X3 = 1 };
 
@@ -523,11 +524,11 @@ __device__ __forceinline__ void store_inv(T *g, const T *sInv) {
 // L lower n x n with inverted diagonal blocks invd[b] (IB x IB, ld IB,
 // column-major) -- the panel TRSM Right/Lower/Trans/NonUnit of
 // coreblas/compute/core_ztrsm.c as used by compute/pzpotrf.c:100-105.
-// Left-looking over inner blocks; all work in cta_gemm.
+// Left-looking over inner blocks; all work in cta_gemm (C: its tile, as many
+// rows as X has at most).
 // ---------------------------------------------------------------------------
-template <class T, int SP>
+template <class T, int SP, class C = Cfg12864<T, SP>>
 __device__ inline void trsm_rows(const ViewT<T> &X, int rows, const ViewT<T> &L, int n, const T *invd, T *smem) {
-    using C = Cfg12864<T, SP>;
     for (int jb = 0; jb < n; jb += IB) {
         const int nbk = min(IB, n - jb);
         Acc<C> acc;
@@ -585,9 +586,9 @@ __device__ inline void trsm_left(const ViewT<T> &X, int w, const ViewT<T> &L, in
 
 template <class T, int SP = SPLIT_BF16X3>
 constexpr size_t tile_smem_elems() {
-    return (Cfg128<T, SP>::SMEM_ELEMS > (Cfg12864<T, SP>::SMEM_ELEMS + 2 * IB * LDD)
+    return (Cfg128<T, SP>::SMEM_ELEMS > (Cfg12864<T, SP>::SMEM_ELEMS + 2 * IB * LEAF_LD)
                 ? Cfg128<T, SP>::SMEM_ELEMS
-                : (Cfg12864<T, SP>::SMEM_ELEMS + 2 * IB * LDD));
+                : (Cfg12864<T, SP>::SMEM_ELEMS + 2 * IB * LEAF_LD));
 }
 template <class T, int SP = SPLIT_BF16X3>
 constexpr size_t tile_smem_bytes() {

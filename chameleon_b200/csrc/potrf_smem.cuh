@@ -12,8 +12,8 @@
 //
 // Layout: the lower triangle by 64-wide block columns; block column b holds
 // rows 64 b .. n-1, column-major with a padded leading dimension (blk_ld).  Right-looking over block columns:
-//   leaf:     D_bb = L_bb L_bb^T and X_b = L_bb^-1 (the warp-level 64 x 64
-//             leaf of rec.cuh on a staged copy of the block)
+//   leaf:     D_bb = L_bb L_bb^T and X_b = L_bb^-1 (the 64 x 64 leaf of
+//             rec.cuh on a staged copy of the block)
 //   panel:    L_ib = A_ib X_b^T                      (i > b)
 //   trailing: A_ij -= L_ib L_jb^T                    (i >= j > b)
 // (the panel and trailing products on the tensor cores as 3xTF32)
@@ -30,8 +30,7 @@ namespace psm {
 
 constexpr int MAXN = 256;   // largest tile order
 constexpr int BW = 64;      // block-column width (= IB)
-constexpr int LDI = 65;     // leading dimension of the staged block and its inverse
-static_assert(LDI == rec::LDS, "the staged leaf uses the leading dimension of rec.cuh");
+constexpr int LDI = rec::LDS;   // leading dimension of the staged block and its inverse
 
 // Leading dimension of block column b: its rows rounded up to 32, plus 8
 // (8 mod 32: the tensor-core fragment loads -- 8 consecutive rows at 4
@@ -51,9 +50,8 @@ constexpr size_t SMEM_BYTES = (size_t)SMEM_FLOATS * sizeof(float);
 // Cholesky of the nbk x nbk block (nbk <= 64) at D (column-major, ld ldd,
 // lower triangle) in place, and its inverse into Xs (ld LDI, 64 x 64: zeros
 // above the diagonal and outside nbk).  The block is staged, identity-padded,
-// into sD (64 x LDI) for the warp-level 64 x 64 leaf of rec.cuh (32 x 32
-// Cholesky and inverse kernels in rolled form).  Returns LAPACK info.  All 256
-// threads; ends with a barrier.
+// into sD (64 x LDI) for the 64 x 64 leaf of rec.cuh.  Returns LAPACK info.
+// All 256 threads; ends with a barrier.
 static __device__ __noinline__ int leaf(float *D, int ldd, int nbk, float *sD) {
     float *Xs = sD + BW * LDI;   // the leaf's inverse follows the staged block
     for (int idx = threadIdx.x; idx < 64 * 64; idx += NT_CTA) {
@@ -63,7 +61,7 @@ static __device__ __noinline__ int leaf(float *D, int ldd, int nbk, float *sD) {
         sD[c * LDI + r] = v;
     }
     __syncthreads();
-    const int info = rec::leaf64_core<float, true>(sD);
+    const int info = rec::leaf64_core<float, true>(sD, Xs, nbk);
     if (info) return info;
     for (int idx = threadIdx.x; idx < 64 * 64; idx += NT_CTA) {
         const int r = idx & 63, c = idx >> 6;

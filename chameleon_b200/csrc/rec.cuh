@@ -13,8 +13,7 @@
 //     X21 = -X22 (L21 X11),
 //
 // so that every off-diagonal step is one GEMM-shaped pass (cta_gemm on the
-// tensor cores).  The recursion ends in a 64 x 64 leaf made of two warp-level
-// 32 x 32 Cholesky / inverse kernels that keep a column per lane in registers.
+// tensor cores).  The recursion ends in a 64 x 64 leaf (leaf64_core).
 // With the full inverse, the panel solve A(m,k) <- A(m,k) L(k,k)^-T and the
 // diagonal solves of the forward / backward substitutions are one GEMM each
 // (apply_inv_right / apply_inv_left), done in place by ordering the output
@@ -29,202 +28,360 @@
 namespace chb {
 namespace rec {
 
-constexpr int LDS = IB + 1;   // leaf shared-memory leading dimension (65)
-constexpr unsigned FULL = 0xffffffffu;
+// ---------------------------------------------------------------------------
+// The 64 x 64 leaf: Cholesky factor and inverse of one diagonal block held in
+// shared memory, by the whole CTA.
+//
+// It is the longest serial chain of every factorization here, so what bounds
+// it is latency: 64 dependent pivots.  The block is factored by 8-wide panels,
+// and the pivot chain is kept in registers.  Warp 0 owns the chain: every lane
+// reads the panel's 8 x 8 diagonal block (36 broadcast loads) and factors it
+// redundantly, so that consecutive pivots need no exchange between lanes (one
+// reciprocal, one product and one FMA each), while it carries two rows of the panel along.
+// After panel p the other warps bring block column p + 1 up to date, one 8 x 8
+// tile each, and hand it to warp 0; while warp 0 factors panel p + 1 they
+// update the remaining tiles (FP64 products on DMMA, FP32 ones on FMA).  The
+// inverse trails the factorization by one panel and hides behind it: W(I, J) =
+// sum_k L(I, k) X(k, J) is accumulated in the place of X(I, J), and block row
+// p is finished as X(p, J) = -L(p,p)^-1 W(p, J) once panel p is factored.  The
+// tiles stay in shared memory and are dealt out over the warps: with a row of
+// tiles in each warp's registers the static register indices made every pass
+// a chain of branches, and the warp with the longest row set the time.
+// ---------------------------------------------------------------------------
+constexpr int LDS = LEAF_LD;  // leaf leading dimension: 4 mod 16 doubles (and 4 mod 32
+                              // floats), so that MMA fragments and 16-byte column reads
+                              // are free of bank conflicts
+constexpr int PW = 8;         // panel width
 
-// 1/sqrt(d) to working precision: hardware estimate + one Newton step.
-__device__ __forceinline__ float rsqrt_wp(float d) {
-    const float r = rsqrtf(d);
-    return r * fmaf(-0.5f * d * r, r, 1.5f);
-}
-__device__ __forceinline__ double rsqrt_wp(double d) {
-    const double r = rsqrt(d);
-    return r * fma(-0.5 * d * r, r, 1.5);
-}
-
-// Cholesky of the 32 x 32 lower block at S (shared, ld LDS) by one warp, in
-// place: lane i keeps row i in registers.  Each of the 32 steps needs the
-// pivot, one reciprocal square root and the broadcast of column j.  Entries
-// above the diagonal are updated too (no per-element predicates): they are
-// never read back.  The block must be identity-padded beyond the matrix.
-// Returns 0 or the 1-based column of the first non-positive pivot (uniform
-// across the warp); after a failure the remaining steps run on a unit pivot
-// so that the loop stays branch-free.  The loop is rolled (its ~1-2 KB of
-// code stays in the instruction cache); register indices stay static by
-// shifting: at step j, slot k of a lane holds the entry of column (row)
-// j + k, and the update of slot k writes slot k - 1, so slot 0 is always the
-// current column (row) and the shift costs no moves.
+// The same pointer with its address space known: a function that is not inlined
+// and takes a generic pointer would otherwise compile every access to a generic
+// load or store, which takes about twice the latency of a shared one.
 template <class T>
-__device__ __noinline__ int warp_chol32r(T *S, T *bc) {
+__device__ __forceinline__ T *in_shared(T *p) {
+    return static_cast<T *>(__cvta_shared_to_generic(__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void bar_sync(int id) { asm volatile("bar.sync %0, 256;\n" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, 256;\n" ::"r"(id) : "memory"); }
+
+// Reciprocal (rc) and reciprocal square root (rs) of a pivot to working
+// precision: the hardware estimates (20 bits for FP64, 22 for FP32) and one
+// step of a third-order (FP64) or second-order (FP32) iteration on the
+// residuals 1 - d r and 1 - d r^2.  The next pivot waits for rc only.  The
+// estimates flush to zero or overflow near the ends of the exponent range:
+// false outside (and for a pivot that is not positive, or NaN).
+__device__ __forceinline__ bool pivot_recip(double d, double &rc, double &rs) {
+    double c, q;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(c) : "d"(d));
+    const double e = fma(-d, c, 1.0);
+    rc = fma(c * e, 1.0 + e, c);
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(d));
+    const double h = fma(-d * q, q, 1.0);
+    rs = fma(q * h, fma(0.375, h, 0.5), q);
+    return d > 1e-280 && d < 1e280;
+}
+__device__ __forceinline__ bool pivot_recip(float d, float &rc, float &rs) {
+    float c, q;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(c) : "f"(d));
+    rc = fmaf(c, fmaf(-d, c, 1.f), c);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(d));
+    rs = fmaf(0.5f * q, fmaf(-d * q, q, 1.f), q);
+    return d > 1e-30f && d < 1e30f;
+}
+
+// Panel p (columns 8 p .. 8 p + 7) of the block at S by one warp: L in place,
+// the reciprocals of its diagonal to rd, and for p > 0 the inverse of its
+// diagonal block to X (same place): lane k < 8 then carries the unit row e_k
+// instead of the finished row k, which the column operations turn into column
+// k of the inverse.  The pivots run on d and its reciprocal (an LDL^T
+// recurrence on the unscaled columns); the square roots stay off the chain.
+// SAFE: any pivot; the first one that is not positive (NaN included) is
+// reported in info (1-based) and replaced by 1.  !SAFE: returns false, with
+// nothing written, when a pivot is not positive or too extreme for the
+// estimates.
+template <class T, bool SAFE>
+__device__ __forceinline__ bool leaf_panel(T *S, T *X, int p, T *rd, int &info) {
     const int lane = threadIdx.x & 31;
-    T a[32];   // a[k]: entry (lane, j + k)
+    T *P = S + PW * p * LDS;
+    const T *D0 = P + PW * p;
+    T d[PW][PW];
 #pragma unroll
-    for (int c = 0; c < 32; ++c) a[c] = (c <= lane) ? S[lane + c * LDS] : T(0);
-    int info = 0;
-    // pivot and reciprocal square root of step 0; every step computes those of
-    // the next one right after the entry that holds it, so that the shuffle
-    // and the square root overlap the rest of the update
-    T d = __shfl_sync(FULL, a[0], 0);
-    if (!(d > T(0))) {   // also catches NaN
-        info = 1;
-        d = T(1);
+    for (int k = 0; k < PW; ++k)
+#pragma unroll
+        for (int i = k; i < PW; ++i) d[i][k] = D0[i + k * LDS];
+    const bool unit = p > 0 && lane < PW;
+    T a0[PW], a1[PW];
+#pragma unroll
+    for (int k = 0; k < PW; ++k) {
+        a0[k] = P[lane + k * LDS];
+        a1[k] = P[lane + 32 + k * LDS];
+        if (unit) a0[k] = (k == lane) ? T(1) : T(0);
     }
-    T r = rsqrt_wp(d);
-#pragma unroll 1
-    for (int j = 0; j < 32; ++j) {
-        const T l = (lane == j) ? d * r : a[0] * r;
-        if (lane >= j) S[lane + j * LDS] = l;
-        // column j broadcast through bc (two buffers of 64 entries, by step
-        // parity): buf[m] = l of lane m & 31, so that slot k reads buf[j + k]
-        // at a fixed offset (one shared load per entry, no lane arithmetic);
-        // the wrapped slots read the unused lanes' values, as shuffles would,
-        // and are never read back
-        T *buf = bc + ((j & 1) << 6);
-        buf[lane] = l;
-        buf[lane + 32] = l;
-        __syncwarp();
-        const T *col = buf + j;
-        a[0] = a[1] - l * col[1];
-        T dn = __shfl_sync(FULL, a[0], (j + 1) & 31);
+    __syncwarp();   // every lane has read the diagonal block before it is overwritten
+    T rs[PW];
+    bool ok = true;
 #pragma unroll
-        for (int k = 2; k < 32; ++k) a[k - 1] = a[k] - l * col[k];
-        a[31] = T(0);
-        if (!(dn > T(0))) {
-            if (info == 0 && j + 1 < 32) info = j + 2;
-            dn = T(1);
+    for (int c = 0; c < PW; ++c) {
+        T rc;
+        if (SAFE) {
+            T dc = d[c][c];
+            if (!(dc > T(0))) {
+                if (info == 0) info = PW * p + c + 1;
+                dc = T(1);
+            }
+            rc = T(1) / dc;
+            rs[c] = T(1) / sqrt(dc);
+        } else {
+            ok = pivot_recip(d[c][c], rc, rs[c]) && ok;
         }
-        d = dn;
-        r = rsqrt_wp(dn);
+        // (w first: a product of two unscaled entries could leave the exponent range)
+#pragma unroll
+        for (int k = c + 1; k < PW; ++k) {
+            const T w = d[k][c] * rc;
+#pragma unroll
+            for (int i = k; i < PW; ++i) d[i][k] -= d[i][c] * w;
+            a0[k] -= a0[c] * w;
+            a1[k] -= a1[c] * w;
+        }
     }
-    __syncwarp();
+    if (!SAFE && !ok) return false;
+    // one guarded store per entry through a per-lane pointer and stride
+    // (separate branches for the two destinations cost twice the panel's time)
+    T *q = unit ? X + PW * p * (LDS + 1) + lane * LDS : P + lane;
+    const int st = unit ? 1 : LDS, last0 = unit ? PW : lane - PW * p, last1 = lane + 32 - PW * p;
+#pragma unroll
+    for (int c = 0; c < PW; ++c) {
+        const T v0 = a0[c] * rs[c], v1 = a1[c] * rs[c];
+        if (c <= last0) q[c * st] = v0;
+        if (c <= last1) P[lane + 32 + c * LDS] = v1;
+    }
+    T r = rs[0];
+#pragma unroll
+    for (int c = 1; c < PW; ++c)
+        if (lane == c) r = rs[c];
+    if (lane < PW) rd[PW * p + lane] = r;
+    return true;
+}
+template <class T>
+__device__ __noinline__ int leaf_panel_safe(T *S, T *X, int p, T *rd, int info) {
+    leaf_panel<T, true>(in_shared(S), in_shared(X), p, in_shared(rd), info);
     return info;
 }
 
-// X = L^-1 for the 32 x 32 lower block at S, lane c = column c of X, slot k =
-// row i + k at step i (the entries of columns of L are broadcast loads at
-// fixed offsets from S(i, i): rows i + 1 .. i + 31, so up to 31 entries past
-// row 31 of column i -- the wrapped slots, never read back; the caller keeps
-// that range inside its shared memory: leaf64_core's sX follows sD).
+// Inverse of the 8 x 8 lower block L(p, p) into X (full, zeros above the
+// diagonal), by one warp: lane c < 8 solves for column c.
 template <class T>
-__device__ __noinline__ void warp_trinv32r(const T *S, T *Xs) {
+__device__ __forceinline__ void leaf_dinv(const T *S, T *X, int p, const T *rd) {
     const int lane = threadIdx.x & 31;
-    T x[32];
+    const T *D0 = S + PW * p * (LDS + 1);
+    T *X0 = X + PW * p * (LDS + 1);
+    T s[PW];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) x[k] = (k == lane) ? T(1) : T(0);
-    // the 32 diagonal reciprocals at once, off the step chain (lane i: 1 / L(i, i))
-    const T rdl = T(1) / S[lane + lane * LDS];
-#pragma unroll 1
-    for (int i = 0; i < 32; ++i) {
-        const T xi = x[0] * __shfl_sync(FULL, rdl, i);   // X(i, lane), final (zero above the diagonal)
-        Xs[i + lane * LDS] = xi;
-        const T *col = S + i * (LDS + 1);                 // S(i, i)
+    for (int i = 0; i < PW; ++i) s[i] = (i == lane) ? T(1) : T(0);
 #pragma unroll
-        for (int k = 1; k < 32; ++k) x[k - 1] = x[k] - col[k] * xi;
-        x[31] = T(0);
+    for (int i = 0; i < PW; ++i) {
+        s[i] *= rd[PW * p + i];
+#pragma unroll
+        for (int m = i + 1; m < PW; ++m) s[m] -= D0[m + i * LDS] * s[i];
+    }
+    if (lane < PW) {
+#pragma unroll
+        for (int i = 0; i < PW; ++i) X0[i + lane * LDS] = s[i];
     }
     __syncwarp();
 }
 
-// out(i, c) = sum_{k<32} P[i + k*LDS] * Q[c + k*LDS] (ROWS_Q: Q read as
-// rows) or Q[k + c*LDS] (Q read as columns), 32 x 32 outputs spread over the
-// CTA: thread (i = tid & 31, cg = tid >> 5) owns columns 4cg .. 4cg+3.
-template <class T, bool QROWS>
-__device__ __forceinline__ void small_mm32(const T *P, const T *Q, T (&o)[4]) {
-    const int i = threadIdx.x & 31, cg = threadIdx.x >> 5;
+// An 8 x 8 tile in the registers of one warp, with the DMMA accumulator's
+// layout for both types: lane (g, t) = (lane / 4, lane % 4) holds the entries
+// (g, 2 t) and (g, 2 t + 1).  LeafA is the left operand of a product, K = 8;
+// the right operand is read from shared memory, B(k, n) at q[n + k LDS] (rows
+// of L) or q[k + n LDS] (columns of X).
+template <class T>
+struct LeafA;
+template <>
+struct LeafA<double> {
+    double a0, a1;
+    __device__ __forceinline__ void load(const double *q, double sign) {
+        const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+        a0 = sign * q[g + t * LDS];
+        a1 = sign * q[g + (t + 4) * LDS];
+    }
+};
+template <>
+struct LeafA<float> {
+    float a[PW];
+    __device__ __forceinline__ void load(const float *q, float sign) {
+        const int g = (threadIdx.x & 31) >> 2;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) o[q] = T(0);
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-        const T p = P[i + k * LDS];
+        for (int k = 0; k < PW; ++k) a[k] = sign * q[g + k * LDS];
+    }
+};
+__device__ __forceinline__ void leaf_mm_l(double (&c)[2], const LeafA<double> &a, const double *q) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    dmma884(c, a.a0, q[g + t * LDS]);
+    dmma884(c, a.a1, q[g + (t + 4) * LDS]);
+}
+__device__ __forceinline__ void leaf_mm_x(double (&c)[2], const LeafA<double> &a, const double *q) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    dmma884(c, a.a0, q[t + g * LDS]);
+    dmma884(c, a.a1, q[t + 4 + g * LDS]);
+}
+__device__ __forceinline__ void leaf_mm_l(float (&c)[2], const LeafA<float> &a, const float *q) {
+    const int t = threadIdx.x & 3;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = 4 * cg + q;
-            o[q] += p * (QROWS ? Q[c + k * LDS] : Q[k + c * LDS]);
-        }
+    for (int k = 0; k < PW; ++k) {
+        const float2 b = *reinterpret_cast<const float2 *>(q + 2 * t + k * LDS);
+        c[0] = fmaf(a.a[k], b.x, c[0]);
+        c[1] = fmaf(a.a[k], b.y, c[1]);
     }
 }
+__device__ __forceinline__ void leaf_mm_x(float (&c)[2], const LeafA<float> &a, const float *q) {
+    const int t = threadIdx.x & 3;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const float4 x = *reinterpret_cast<const float4 *>(q + (2 * t + e) * LDS);
+        const float4 y = *reinterpret_cast<const float4 *>(q + (2 * t + e) * LDS + 4);
+        c[e] = fmaf(a.a[0], x.x, c[e]);
+        c[e] = fmaf(a.a[1], x.y, c[e]);
+        c[e] = fmaf(a.a[2], x.z, c[e]);
+        c[e] = fmaf(a.a[3], x.w, c[e]);
+        c[e] = fmaf(a.a[4], y.x, c[e]);
+        c[e] = fmaf(a.a[5], y.y, c[e]);
+        c[e] = fmaf(a.a[6], y.z, c[e]);
+        c[e] = fmaf(a.a[7], y.w, c[e]);
+    }
+}
+template <class T>
+__device__ __forceinline__ void leaf_get(const T *q, T (&c)[2]) {   // q: the tile's (0, 0), ld LDS
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    c[0] = q[g + 2 * t * LDS];
+    c[1] = q[g + (2 * t + 1) * LDS];
+}
+template <class T>
+__device__ __forceinline__ void leaf_put(T *q, const T (&c)[2]) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    q[g + 2 * t * LDS] = c[0];
+    q[g + (2 * t + 1) * LDS] = c[1];
+}
+// Tile (I, J) of S -= L(I, p) L(J, p)^T
+template <class T>
+__device__ __forceinline__ void leaf_tile_c(T *S, int p, int I, int J) {
+    const T *P = S + PW * p * LDS;
+    LeafA<T> a;
+    T c[2];
+    a.load(P + PW * I, T(-1));
+    leaf_get(S + PW * I + PW * J * LDS, c);
+    leaf_mm_l(c, a, P + PW * J);
+    leaf_put(S + PW * I + PW * J * LDS, c);
+}
+// Tile (I, J) of W += L(I, k) X(k, J)
+template <class T>
+__device__ __forceinline__ void leaf_tile_w(const T *S, T *X, int k, int I, int J) {
+    LeafA<T> a;
+    T c[2];
+    a.load(S + PW * k * LDS + PW * I, T(1));
+    leaf_get(X + PW * I + PW * J * LDS, c);
+    leaf_mm_x(c, a, X + PW * k + PW * J * LDS);
+    leaf_put(X + PW * I + PW * J * LDS, c);
+}
+// Tile (p, J) of X = -X(p, p) W(p, J)
+template <class T>
+__device__ __forceinline__ void leaf_tile_x(T *X, int p, int J) {
+    T *q = X + PW * p + PW * J * LDS;
+    LeafA<T> a;
+    T c[2] = {T(0), T(0)};
+    a.load(X + PW * p * (LDS + 1), T(-1));
+    leaf_mm_x(c, a, q);
+    __syncwarp();   // every lane has read W
+    leaf_put(q, c);
+}
+// q-th tile (row, column) of a lower triangle of tiles, row-major
+__device__ __forceinline__ void leaf_tri(int q, int &i, int &j) {
+    i = (q >= 1) + (q >= 3) + (q >= 6) + (q >= 10) + (q >= 15) + (q >= 21);
+    j = q - i * (i + 1) / 2;
+}
 
-// 64 x 64 leaf on shared memory.  sD (ld LDS) holds the block, lower
-// triangle, identity-padded beyond the matrix and zero above the diagonal.
-// FACT: sD is factored in place (L), else it already holds L.  sX = sD + 64
-// LDS (ld LDS) receives the full inverse (zeros above the diagonal); the
-// inverse kernel's column reads run up to 29 entries past the end of sD, into
-// sX.  Returns LAPACK info.  Called by all threads; ends with a barrier.
+// 64 x 64 leaf on shared memory.  sD (ld LDS, 16-byte aligned) holds the
+// block's lower triangle, identity-padded from n to the next multiple of 8.
+// FACT: sD is factored in place (L), else it already holds L (unit: with an
+// implied unit diagonal).  sX (ld LDS) receives the inverse of
+// the leading 8 ceil(n / 8) rows and columns, lower triangle, with zeros
+// above the diagonal and everywhere else.  Returns LAPACK info.  Called by all
+// threads; ends with a barrier.
 template <class T, bool FACT>
-__device__ __noinline__ int leaf64_core(T *sD) {
-    T *sX = sD + 64 * LDS;
+__device__ __noinline__ int leaf64_core(T *sD, T *sX, int n, bool unit = false) {
+    sD = in_shared(sD);
+    sX = in_shared(sX);
     __shared__ int s_info;
+    __shared__ T s_rd[64];
     const int tid = threadIdx.x, warp = tid >> 5;
-    if (tid == 0) s_info = 0;
+    const int nblk = (n + PW - 1) / PW;
+    __syncthreads();   // the callers' last writes of the block
+    if (!FACT && tid < PW * nblk) s_rd[tid] = unit ? T(1) : T(1) / sD[tid + tid * LDS];
+#pragma unroll 4
+    for (int idx = tid; idx < 64 * 64; idx += NT_CTA) sX[(idx & 63) + (idx >> 6) * LDS] = T(0);
     __syncthreads();
-    if (FACT) {
-        if (warp == 0) {
-            const int info = warp_chol32r(sD, sX);   // sX (2 columns) is free until the inverse
-            if (tid == 0) s_info = info;
+    if (FACT && warp == 0) {
+        int info = 0;
+        for (int p = 0; p < nblk; ++p) {
+            if (p > 0) bar_sync(1);   // block column p is up to date in sD
+            if (!leaf_panel<T, false>(sD, sX, p, s_rd, info)) info = leaf_panel_safe<T>(sD, sX, p, s_rd, info);
+            if (p == nblk - 1 && tid == 0) s_info = info;
+            bar_arrive(2);
         }
-        __syncthreads();
-        if (s_info) return s_info;
-    }
-    if (warp == 0) warp_trinv32r(sD, sX);
-    __syncthreads();
-    T o[4];
-    const int i = tid & 31, cg = tid >> 5;
-    if (FACT) {
-        // L21 = A21 X11^T
-        small_mm32<T, true>(sD + 32, sX, o);
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) sD[32 + i + (4 * cg + q) * LDS] = o[q];
-        __syncthreads();
-        // A22 -= L21 L21^T (lower)
-        small_mm32<T, true>(sD + 32, sD + 32, o);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int c = 4 * cg + q;
-            if (c <= i) sD[32 + i + (32 + c) * LDS] -= o[q];
+    } else {
+        const int nw = FACT ? 7 : 8, w = FACT ? warp - 1 : warp;
+        if (!FACT && w < nblk) leaf_dinv(sD, sX, w, s_rd);
+        for (int p = 0; p < nblk; ++p) {
+            if (FACT) bar_sync(2);   // panel p is factored; rows < p of the inverse are done
+            else __syncthreads();
+            if (FACT) {
+                if (p + 1 + w < nblk) leaf_tile_c(sD, p, p + 1 + w, p + 1);   // gates the next panel
+                if (p + 1 < nblk) bar_arrive(1);
+            }
+            if (w < p) {   // block row p of the inverse, one tile per warp
+                leaf_tile_w(sD, sX, p - 1, p, w);
+                __syncwarp();
+                leaf_tile_x(sX, p, w);
+            }
+            const int m = FACT ? max(0, nblk - p - 2) : 0, nc = m * (m + 1) / 2;
+            const int rows = nblk - 1 - p;
+            // the first tiles go to the warps that had none above
+            for (int q = nw - 1 - w; q < nc + rows * p; q += nw) {
+                if (q < nc) {
+                    int i, j;
+                    leaf_tri(q, i, j);
+                    leaf_tile_c(sD, p, p + 2 + i, p + 2 + j);
+                } else {
+                    const int q2 = q - nc;
+                    leaf_tile_w(sD, sX, p - 1, p + 1 + q2 / p, q2 % p);
+                }
+            }
+            // the diagonal block of the inverse comes with the panel, except panel 0's
+            if (FACT && p == 0 && w == 6) leaf_dinv(sD, sX, 0, s_rd);
         }
-        __syncthreads();
-        if (warp == 0) {
-            // the columns 32, 33 of sX are free until X22 and W are written
-            const int info = warp_chol32r(sD + 32 + 32 * LDS, sX + 32 * LDS);
-            if (tid == 0) s_info = info ? 32 + info : 0;
-        }
-        __syncthreads();
-        if (s_info) return s_info;
     }
-    if (warp == 1) warp_trinv32r(sD + 32 + 32 * LDS, sX + 32 + 32 * LDS);
     __syncthreads();
-    // W = L21 X11 into the upper-right block of sX (zero in the inverse)
-    small_mm32<T, false>(sD + 32, sX, o);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sX[i + (32 + 4 * cg + q) * LDS] = o[q];
-    __syncthreads();
-    // X21 = -X22 W
-#pragma unroll
-    for (int q = 0; q < 4; ++q) o[q] = T(0);
-#pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-        const T p = sX[32 + i + (32 + k) * LDS];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) o[q] += p * sX[k + (32 + 4 * cg + q) * LDS];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sX[32 + i + (4 * cg + q) * LDS] = -o[q];
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sX[i + (32 + 4 * cg + q) * LDS] = T(0);
-    __syncthreads();
-    return 0;
+    return FACT ? s_info : 0;
 }
 
-// Identity-padded load of the lower n x n block of A (n <= 64) into sD.
+// Identity-padded load of the lower n x n block of A (n <= 64) into sD (its
+// first 8 ceil(n / 8) columns).
 template <class T>
 __device__ __forceinline__ void leaf64_load(const ViewT<T> &A, int n, T *sD) {
-    for (int idx = threadIdx.x; idx < 64 * 64; idx += NT_CTA) {
-        const int r = idx & 63, c = idx >> 6;
-        T v = (r == c) ? T(1) : T(0);
-        if (r < n && c < n) v = (r >= c) ? *A.at(r, c) : T(0);
-        sD[r + c * LDS] = v;
+    const int np = (n + PW - 1) / PW * PW;
+    const bool cm = A.rs == 1;   // along the contiguous direction, all loads in flight together
+    T v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int idx = threadIdx.x + u * NT_CTA;
+        const int r = cm ? idx & 63 : idx >> 6, c = cm ? idx >> 6 : idx & 63;
+        v[u] = (r < n && c < n) ? ((r >= c) ? *A.at(r, c) : T(0)) : (r == c ? T(1) : T(0));
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int idx = threadIdx.x + u * NT_CTA;
+        const int r = cm ? idx & 63 : idx >> 6, c = cm ? idx >> 6 : idx & 63;
+        if (c < np) sD[r + c * LDS] = v[u];
     }
     __syncthreads();
 }
@@ -236,7 +393,7 @@ __device__ __noinline__ int leaf64(const ViewT<T> &A, const ViewT<T> &X, int n, 
     T *sD = smem;              // 64 x LDS
     T *sX = smem + 64 * LDS;   // 64 x LDS
     leaf64_load(A, n, sD);
-    const int info = leaf64_core<T, FACT>(sD);
+    const int info = leaf64_core<T, FACT>(sD, sX, n);
     if (info) return info;
     for (int idx = threadIdx.x; idx < n * n; idx += NT_CTA) {
         const int r = idx % n, c = idx / n;
@@ -289,7 +446,7 @@ __device__ int tile_potrf_blk(const ViewT<T> &Tv, int n, T *invd, T *smem, unsig
             if (r < nbk && c < nbk && r >= c) sD[r + c * LDS] -= v;
         });
         lap(0);
-        const int info = leaf64_core<T, true>(sD);
+        const int info = leaf64_core<T, true>(sD, sX, nbk);
         lap(1);
         if (info) return jb + info;
         T *inv = invd + (int64_t)(jb / IB) * IB * IB;
@@ -320,6 +477,106 @@ __device__ int tile_potrf_blk(const ViewT<T> &Tv, int n, T *invd, T *smem, unsig
     return 0;
 }
 
+// acc (rows x 64) = P X^T for the 64 x 64 blocks P and X (lower) in shared
+// memory (ld LDS), on DMMA: warp w owns rows 8 w .. 8 w + 7, all 64 columns.
+struct RowAcc {
+    double v[8][2];   // tile J: entries (8 w + g, 8 J + 2 t), (.., + 1)
+    template <class F>
+    __device__ __forceinline__ void for_each(F &&f) const {
+        const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll
+        for (int J = 0; J < 8; ++J)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) f(8 * w + g, 8 * J + 2 * t + e, v[J][e]);
+    }
+};
+static __device__ __forceinline__ void mul_xt64(RowAcc &acc, const double *P, const double *X) {
+    const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll
+    for (int J = 0; J < 8; ++J) acc.v[J][0] = acc.v[J][1] = 0.0;
+#pragma unroll
+    for (int kb = 0; kb < 8; ++kb) {   // X(c, k) is zero for k > c
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = 8 * kb + 4 * h + t;
+            const double a = P[8 * w + g + k * LDS];
+#pragma unroll
+            for (int J = 0; J < 8; ++J)
+                if (J >= kb) dmma884(acc.v[J], a, X[8 * J + g + k * LDS]);
+        }
+    }
+}
+
+// tile_potrf_blk for FP64 with the work between the leaves kept on chip: the
+// leaf's inverse stays in shared memory beside the GEMM staging area (which
+// the leaf block and the panel block alias in turn), so that a 64-row panel
+// step is one product with the columns to its left, one subtraction into
+// shared memory and one product with the inverse from there -- instead of two
+// products with a write and two reads of global memory between them.  Same
+// contract; smem: fused_smem_elems() doubles, two CTAs per SM.
+constexpr int fused_smem_elems() { return Cfg64<double>::SMEM_ELEMS + IB * LDS; }
+static_assert(2 * IB * LDS <= Cfg64<double>::SMEM_ELEMS, "leaf and panel block inside the staging area");
+static __device__ int tile_potrf_fused(const View &Tv, int n, double *invd, double *smem, unsigned *ph = nullptr) {
+    using C = Cfg64<double>;
+    double *sD = smem, *sP = smem + IB * LDS, *sX = smem + C::SMEM_ELEMS;
+    long long c0 = (ph && threadIdx.x == 0) ? clock64() : 0;
+    auto lap = [&](int i) {
+        if (ph && threadIdx.x == 0) {
+            const long long c1 = clock64();
+            ph[i] += (unsigned)(c1 - c0);
+            c0 = c1;
+        }
+    };
+    for (int jb = 0; jb < n; jb += IB) {
+        const int nbk = min(IB, n - jb);
+        Acc<C> acc;
+        acc.zero();
+        if (jb > 0) cta_gemm(acc, Tv.sub(jb, 0), Tv.sub(jb, 0), nbk, nbk, jb, smem);
+        leaf64_load(Tv.sub(jb, jb), nbk, sD);
+        if (jb > 0)
+            acc.for_each([&](int r, int c, double v) {
+                if (r < nbk && c < nbk && r >= c) sD[r + c * LDS] -= v;
+            });
+        lap(0);
+        const int info = leaf64_core<double, true>(sD, sX, nbk);
+        lap(1);
+        if (info) return jb + info;
+        double *inv = invd + (int64_t)(jb / IB) * IB * IB;
+        const bool cm = Tv.rs == 1;
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < IB * IB; idx += NT_CTA) {
+            const int r = idx % IB, c = idx / IB;
+            inv[idx] = (r < nbk && c < nbk) ? sX[r + c * LDS] : 0.0;
+            const int tr = cm ? r : c, tc = cm ? c : r;   // along the tile's contiguous direction
+            if (tr < nbk && tc < nbk && tr >= tc) *Tv.at(jb + tr, jb + tc) = sD[tr + tc * LDS];
+        }
+        cta_sync();
+        for (int r0 = jb + nbk; r0 < n; r0 += IB) {
+            const int mr = min(IB, n - r0);
+            acc.zero();
+            if (jb > 0) cta_gemm(acc, Tv.sub(r0, 0), Tv.sub(jb, 0), mr, nbk, jb, smem);
+            // (nbk == 64 here: rows below mean the block column is full)
+            const View A = Tv.sub(r0, jb);
+            Acc<C> old;
+            acc.for_each_idx([&](int a, int b, int e, int r, int c, double) {
+                old.v[a][b][e] = r < mr ? __ldcg(A.at(r, c)) : 0.0;
+            });
+            acc.for_each_idx([&](int a, int b, int e, int r, int c, double v) {
+                sP[r + c * LDS] = old.v[a][b][e] - v;
+            });
+            __syncthreads();
+            RowAcc x;
+            mul_xt64(x, sP, sX);
+            x.for_each([&](int r, int c, double v) {
+                if (r < mr) *A.at(r, c) = v;
+            });
+            cta_sync();
+        }
+        lap(2);
+    }
+    return 0;
+}
+
 // Inverted 64 x 64 diagonal blocks of an existing lower factor (n x n), for
 // the solve-only executor mode.
 template <class T>
@@ -329,7 +586,7 @@ __device__ void tile_inv_blk(const ViewT<T> &Tv, int n, T *invd, T *smem) {
     for (int jb = 0; jb < n; jb += IB) {
         const int nbk = min(IB, n - jb);
         leaf64_load(Tv.sub(jb, jb), nbk, sD);
-        leaf64_core<T, false>(sD);
+        leaf64_core<T, false>(sD, sX, nbk);
         T *inv = invd + (int64_t)(jb / IB) * IB * IB;
         for (int idx = threadIdx.x; idx < IB * IB; idx += NT_CTA) {
             const int r = idx % IB, c = idx / IB;
