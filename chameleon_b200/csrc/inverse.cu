@@ -4,14 +4,15 @@
 //
 // Reference: compute/ztrtri.c, zlauum.c, zpotri.c (zpotri = pztrtri then
 // pzlauum, compute/zpotri.c), lapack_api/src/lapack_z{posv,potrf,potrs,potri,
-// trtri,lauum}.c.  On the B200 each one is whole-matrix GPU work on the tile
-// kernels of the tile ABI:
-//   dtrtri: X = op(T)^-1 as the solution of T X = I (CUDA_dtrsm: blocked
-//           substitution with inverted 64 x 64 diagonal blocks, FP64 DMMA),
-//           then the referenced triangle of X into A;
-//   dlauum: A <- L^T L (lower) / U U^T (upper) as one FP64 GEMM of the
-//           triangular factor (zero-filled copy) with its transpose;
-//   dpotri: dtrtri then dlauum, as LAPACK and the reference.
+// trtri,lauum}.c.  All of them work on the lower triangle (an upper one is its
+// transposed view) with FP64 tensor-core products, and skip the zero halves
+// of triangular operands, so that each does its n^3 / 3 operations:
+//   dtrtri: the inverted 64 x 64 diagonal blocks in one launch, then doubling:
+//           at block size h = 64, 128, ... every pair of neighbouring h-blocks
+//           gets X21 = -X22 (L21 X11), two launches for all pairs together;
+//   dlauum: A(i,j) = sum_{k >= i} L(k,i) L(k,j), one launch;
+//   dpotri: dtrtri then dlauum, as LAPACK and the reference; the inverse of
+//           the factor stays in the workspace between the two.
 // LAPACK's contract is kept: only the `uplo` triangle of A is read and
 // written; dtrtri returns info = i when A(i,i) is exactly zero (A untouched),
 // with diag = Unit the diagonal is neither read nor written.
@@ -22,39 +23,104 @@
 
 #include "core.cuh"
 #include "internal.h"
+#include "rec.cuh"
 
 struct cham_b200_handle_s;   // tile_abi.cu
 
 namespace chb {
 
-// dst <- the `uplo` triangle of src (N x N, column-major), zero elsewhere
-// (zero_other) or left untouched; the diagonal is skipped when skip_diag.
-__global__ void tri_copy_kernel(const double *src, int64_t lds, double *dst, int64_t ldd, int N, int upper,
-                                int zero_other, int skip_diag) {
-    const int64_t total = (int64_t)N * N;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(idx % N), j = (int)(idx / N);
-        const bool in = upper ? i <= j : i >= j;
-        if (i == j && skip_diag) continue;
-        if (in) dst[i + j * ldd] = src[i + j * lds];
-        else if (zero_other) dst[i + j * ldd] = 0.0;
+// Block edge of the products.  The k extents of the blocks differ by up to
+// n / 64 times (triangular operands), so blocks are small and the longest come
+// first: a 128-wide block of n = 2500 would run 0.65 ms alone, longer than the
+// whole operation needs.
+constexpr int HB = 64;
+using CfgInv = Cfg64<double>;
+constexpr int INV_CTAS_PER_SM = 3;
+
+// X (column-major, ld ldx) gets the inverted HB x HB diagonal blocks of the
+// lower L (n x n), one CTA each; unit: with an implied unit diagonal.
+__global__ void __launch_bounds__(NT_CTA, 1) diag_inv_kernel(View L, int n, int unit, double *X, int64_t ldx) {
+    extern __shared__ __align__(128) double smem[];
+    const int j0 = blockIdx.x * HB, nb = min(HB, n - j0);
+    rec::leaf64_load(L.sub(j0, j0), nb, smem);
+    double *sX = smem + 64 * rec::LDS;
+    rec::leaf64_core<double, false>(smem, sX, nb, unit != 0);
+    double *D = X + j0 + (int64_t)j0 * ldx;
+    for (int idx = threadIdx.x; idx < nb * nb; idx += NT_CTA)
+        D[idx % nb + (int64_t)(idx / nb) * ldx] = sX[idx % nb + (idx / nb) * rec::LDS];
+}
+
+// One half of a doubling step on the pairs of h-blocks (rows [r, r + h2) below
+// rows [r - h, r), r = h (2 q + 1), h2 = h or the matrix's end): output block
+// (bi, bj) of pair q.  first: W21 = L21 X11, written into T (column-major, ld
+// ldx); else X21 = -X22 W21, from T into X.
+__global__ void __launch_bounds__(NT_CTA, INV_CTAS_PER_SM)
+    trtri_pair_kernel(View L, int n, int h, double *X, double *T, int64_t ldx, int first) {
+    extern __shared__ __align__(128) double smem[];
+    const int r = h * (2 * (int)blockIdx.z + 1), c = r - h, h2 = min(h, n - r);
+    // the longest products first: W needs k >= its column, X22 W k <= its row
+    const int bi = first ? blockIdx.x : gridDim.x - 1 - blockIdx.x, bj = blockIdx.y;
+    const int i0 = bi * HB, j0 = bj * HB;
+    if (i0 >= h2) return;
+    const int rows = min(HB, h2 - i0);
+    Acc<CfgInv> acc;
+    acc.zero();
+    const View Xv{X, 1, ldx}, Tv{T, 1, ldx};
+    if (first) {
+        cta_gemm(acc, L.sub(r + i0, c + j0), Xv.sub(c + j0, c + j0).t(), rows, HB, h - j0, smem);
+        acc.store_to(Tv.sub(r + i0, c + j0), rows, HB);
+    } else {
+        cta_gemm(acc, Xv.sub(r + i0, r), Tv.sub(r, c + j0).t(), rows, HB, i0 + rows, smem);
+        acc.for_each([&](int i, int j, double v) {
+            if (i < rows) *Xv.at(r + i0 + i, c + j0 + j) = -v;
+        });
     }
 }
 
-__global__ void identity_kernel(double *X, int64_t ld, int N) {
-    const int64_t total = (int64_t)N * N;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(idx % N), j = (int)(idx / N);
-        X[i + j * ld] = (i == j) ? 1.0 : 0.0;
-    }
+// C (lower triangle, n x n view) = X^T X for the lower X (column-major, ld
+// ldx): blocks of the lower triangle in row order, so that the longest sums
+// (k from the block's first row to n) start first.  Nothing is written when
+// *skip is a valid index (a singular factor).
+__global__ void __launch_bounds__(NT_CTA, INV_CTAS_PER_SM)
+    lauum_kernel(View X, int n, View C, const int *skip) {
+    extern __shared__ __align__(128) double smem[];
+    if (skip && *skip != INT_MAX) return;
+    int bi = (int)((sqrtf(8.f * (float)blockIdx.x + 1.f) - 1.f) * 0.5f);
+    while ((bi + 1) * (bi + 2) / 2 <= (int)blockIdx.x) ++bi;
+    while (bi * (bi + 1) / 2 > (int)blockIdx.x) --bi;
+    const int bj = (int)blockIdx.x - bi * (bi + 1) / 2;
+    const int i0 = bi * HB, j0 = bj * HB, rows = min(HB, n - i0), cols = min(HB, n - j0);
+    Acc<CfgInv> acc;
+    acc.zero();
+    // k in this block row: X(k, i) is lower there, and is read in full
+    cta_gemm(acc, X.sub(i0, i0).t(), X.sub(i0, j0).t(), rows, cols, n - i0, smem);
+    acc.for_each([&](int i, int j, double v) {
+        if (i < rows && j < cols && i0 + i >= j0 + j) *C.at(i0 + i, j0 + j) = v;
+    });
+}
+
+// D <- the lower triangle of S (views of order n), zeros above it when
+// zero_upper; the diagonal is left out when skip_diag; nothing when *skip is a
+// valid index.  Block (x, y): 64 rows of 4 columns per step, along the
+// destination's contiguous direction.
+__global__ void tri_copy_kernel(View S, View D, int n, int zero_upper, int skip_diag, const int *skip) {
+    if (skip && *skip != INT_MAX) return;
+    const bool cm = D.rs == 1;
+    for (int y = blockIdx.y; y < n; y += gridDim.y)
+        for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
+            const int i = cm ? x : y, j = cm ? y : x;
+            if (i < j ? !zero_upper : (i == j && skip_diag)) continue;
+            *D.at(i, j) = i >= j ? *S.at(i, j) : 0.0;
+        }
 }
 
 // *first = min over i of (i + 1) with A(i,i) == 0 (INT_MAX: none).
-__global__ void zero_diag_kernel(const double *A, int64_t lda, int N, int *first) {
+__global__ void flag_kernel(int *first) {
+    if (threadIdx.x == 0) *first = INT_MAX;
+}
+__global__ void zero_diag_kernel(View A, int N, int *first) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
-        if (A[i + (int64_t)i * lda] == 0.0) atomicMin(first, i + 1);
+        if (*A.at(i, i) == 0.0) atomicMin(first, i + 1);
 }
 
 namespace {
@@ -83,52 +149,92 @@ double *work(double **buf, size_t *cap, size_t bytes) {
 }
 }  // namespace
 
-// The three operations on a device column-major A (ld lda), on the library
-// stream; synchronous.  Return LAPACK's info (> 0) or a CHAMELEON_ERR_* code.
-int trtri_dev(cham_uplo_t uplo, cham_diag_t diag, int N, double *A, int lda) {
-    cudaStream_t s = ctx().stream;
-    cublasHandle_t h = lib_handle();
-    if (!h) return CHAMELEON_ERR_UNEXPECTED;
+// Lower view of the uplo triangle.
+static View lower_view(cham_uplo_t uplo, double *A, int lda) {
+    return uplo == ChamLower ? View{A, 1, lda} : View{A, lda, 1};
+}
+
+static int inv_attrs() {
+    static bool done = false;
+    if (done) return 0;
+    CHB_CUDA(cudaFuncSetAttribute(trtri_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgInv::SMEM_BYTES));
+    CHB_CUDA(cudaFuncSetAttribute(lauum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgInv::SMEM_BYTES));
+    CHB_CUDA(cudaFuncSetAttribute(diag_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(2 * IB * LEAF_LD * sizeof(double))));
+    done = true;
+    return 0;
+}
+
+static void tri_copy(View S, View D, int N, int zero_upper, int skip_diag, const int *skip, cudaStream_t s) {
+    const dim3 grid((N + 255) / 256, std::min(N, 2048));
+    tri_copy_kernel<<<grid, 256, 0, s>>>(S, D, N, zero_upper, skip_diag, skip);
+    CHB_LAUNCHED(1);
+}
+
+// Workspace leading dimension: even (16-byte copies of the products' operands)
+// and not a multiple of a power of two for the common orders.
+static int64_t work_ld(int N) { return (N + 1) / 2 * 2 + 2; }
+
+// The inverse of the lower L (view of order N) into the first workspace
+// (column-major, ld work_ld(N), zeros above the diagonal of every HB-block);
+// g_flag = the first zero diagonal entry (INT_MAX: none, or unit).  Stream
+// operations only; returns the workspace.
+static int trtri_work(View L, cham_diag_t diag, int N, cudaStream_t s, double **Xp) {
+    if (int rc = inv_attrs()) return rc;
     if (!g_flag && !(g_flag = (int *)dev_alloc(sizeof(int)))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+    const int64_t ld = work_ld(N);
+    double *X = work(&g_w1, &g_w1_bytes, (size_t)ld * N * sizeof(double));
+    double *T = N > HB ? work(&g_w2, &g_w2_bytes, (size_t)ld * N * sizeof(double)) : X;
+    if (!X || !T) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+    flag_kernel<<<1, 32, 0, s>>>(g_flag);
+    CHB_LAUNCHED(1);
     if (diag == ChamNonUnit) {
-        const int none = INT_MAX;
-        int first = INT_MAX;
-        CHB_CUDA(cudaMemcpyAsync(g_flag, &none, sizeof(int), cudaMemcpyHostToDevice, s));
-        zero_diag_kernel<<<grid_for(N), 256, 0, s>>>(A, lda, N, g_flag);
+        zero_diag_kernel<<<grid_for(N), 256, 0, s>>>(L, N, g_flag);
         CHB_LAUNCHED(1);
-        CHB_CUDA(cudaMemcpyAsync(&first, g_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CHB_CUDA(cudaStreamSynchronize(s));
-        if (first != INT_MAX) return first;   // singular: A is not modified
     }
-    double *X = work(&g_w1, &g_w1_bytes, (size_t)N * N * sizeof(double));
-    if (!X) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-    identity_kernel<<<grid_for((int64_t)N * N), 256, 0, s>>>(X, N, N);
+    diag_inv_kernel<<<(N + HB - 1) / HB, NT_CTA, 2 * IB * LEAF_LD * sizeof(double), s>>>(L, N, diag == ChamUnit, X, ld);
     CHB_LAUNCHED(1);
-    const double one = 1.0;
-    if (int rc = CUDA_dtrsm(ChamLeft, uplo, ChamNoTrans, diag, N, N, &one, A, lda, X, N, h)) return rc;
-    tri_copy_kernel<<<grid_for((int64_t)N * N), 256, 0, s>>>(X, N, A, lda, N, uplo == ChamUpper, 0,
-                                                             diag == ChamUnit);
-    CHB_LAUNCHED(1);
+    for (int64_t h = HB; h < N; h *= 2) {
+        // pairs with any rows in their second block
+        const int pairs = (int)((N - h + 2 * h - 1) / (2 * h)), nb = (int)(h / HB);
+        for (int first = 1; first >= 0; --first)
+            trtri_pair_kernel<<<dim3(nb, nb, pairs), NT_CTA, CfgInv::SMEM_BYTES, s>>>(L, N, (int)h, X, T, ld, first);
+        CHB_LAUNCHED(2);
+    }
     CHB_CUDA(cudaGetLastError());
+    *Xp = X;
+    return 0;
+}
+
+static int read_flag(int *first, cudaStream_t s) {
+    CHB_CUDA(cudaMemcpyAsync(first, g_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     CHB_CUDA(cudaStreamSynchronize(s));
     return 0;
 }
 
+// The three operations on a device column-major A (ld lda), on the library
+// stream; synchronous.  Return LAPACK's info (> 0) or a CHAMELEON_ERR_* code.
+int trtri_dev(cham_uplo_t uplo, cham_diag_t diag, int N, double *A, int lda) {
+    cudaStream_t s = ctx().stream;
+    const View L = lower_view(uplo, A, lda);
+    double *X = nullptr;
+    if (int rc = trtri_work(L, diag, N, s, &X)) return rc;
+    tri_copy(View{X, 1, work_ld(N)}, L, N, 0, diag == ChamUnit, g_flag, s);
+    int first = INT_MAX;
+    if (int rc = read_flag(&first, s)) return rc;
+    return first != INT_MAX ? first : 0;   // singular: A is not modified
+}
+
 int lauum_dev(cham_uplo_t uplo, int N, double *A, int lda) {
     cudaStream_t s = ctx().stream;
-    cublasHandle_t h = lib_handle();
-    if (!h) return CHAMELEON_ERR_UNEXPECTED;
-    double *T = work(&g_w1, &g_w1_bytes, (size_t)N * N * sizeof(double));
-    double *C = work(&g_w2, &g_w2_bytes, (size_t)N * N * sizeof(double));
-    if (!T || !C) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-    tri_copy_kernel<<<grid_for((int64_t)N * N), 256, 0, s>>>(A, lda, T, N, N, uplo == ChamUpper, 1, 0);
-    CHB_LAUNCHED(1);
-    const double one = 1.0, zero = 0.0;
-    // lower: L^T L; upper: U U^T
-    const cham_trans_t ta = (uplo == ChamLower) ? ChamTrans : ChamNoTrans;
-    const cham_trans_t tb = (uplo == ChamLower) ? ChamNoTrans : ChamTrans;
-    if (int rc = CUDA_dgemm(ta, tb, N, N, N, &one, T, N, T, N, &zero, C, N, h)) return rc;
-    tri_copy_kernel<<<grid_for((int64_t)N * N), 256, 0, s>>>(C, N, A, lda, N, uplo == ChamUpper, 0, 0);
+    if (int rc = inv_attrs()) return rc;
+    const View L = lower_view(uplo, A, lda);
+    const int64_t ld = work_ld(N);
+    double *T = work(&g_w1, &g_w1_bytes, (size_t)ld * N * sizeof(double));
+    if (!T) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+    tri_copy(L, View{T, 1, ld}, N, 1, 0, nullptr, s);
+    const int nb = (N + HB - 1) / HB;
+    lauum_kernel<<<nb * (nb + 1) / 2, NT_CTA, CfgInv::SMEM_BYTES, s>>>(View{T, 1, ld}, N, L, nullptr);
     CHB_LAUNCHED(1);
     CHB_CUDA(cudaGetLastError());
     CHB_CUDA(cudaStreamSynchronize(s));
@@ -136,8 +242,17 @@ int lauum_dev(cham_uplo_t uplo, int N, double *A, int lda) {
 }
 
 int potri_dev(cham_uplo_t uplo, int N, double *A, int lda) {
-    if (int rc = trtri_dev(uplo, ChamNonUnit, N, A, lda)) return rc;
-    return lauum_dev(uplo, N, A, lda);
+    cudaStream_t s = ctx().stream;
+    const View L = lower_view(uplo, A, lda);
+    double *X = nullptr;
+    if (int rc = trtri_work(L, ChamNonUnit, N, s, &X)) return rc;
+    const int nb = (N + HB - 1) / HB;
+    lauum_kernel<<<nb * (nb + 1) / 2, NT_CTA, CfgInv::SMEM_BYTES, s>>>(View{X, 1, work_ld(N)}, N, L, g_flag);
+    CHB_LAUNCHED(1);
+    CHB_CUDA(cudaGetLastError());
+    int first = INT_MAX;
+    if (int rc = read_flag(&first, s)) return rc;
+    return first != INT_MAX ? first : 0;   // singular: A is not modified
 }
 
 // S (N x N, ld N) <- the symmetric matrix whose uplo triangle is in A.
