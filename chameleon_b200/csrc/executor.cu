@@ -89,14 +89,19 @@ struct Schedule {
     const int *d_potrf = nullptr;
 };
 
-template <class NBI>
-std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBI nbi);
+template <class NBU>
+std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBU nbu);
 
 std::vector<Task> build_order(const Shape &s) {
     const int NT = (s.N + s.NB - 1) / s.NB;
     const int NTB = s.nrhs > 0 ? (s.nrhs + s.NBB - 1) / s.NBB : 0;
     auto tm = [&](int m) { return (m == NT - 1) ? s.N - m * s.NB : s.NB; };
-    auto nbi = [&](int m) { return (tm(m) + SUBB - 1) / SUBB; };
+    const int cb = count_blk(s.mode);
+    auto nbi = [&](int m) { return (tm(m) + cb - 1) / cb; };                 // panel-solve row blocks
+    auto nbu = [&](int m, int cnt) {                                         // update blocks, cnt panels
+        const int e = upd_blk(s.mode, cnt);
+        return (tm(m) + e - 1) / e;
+    };
     auto wB = [&](int bn) { return (bn == NTB - 1) ? s.nrhs - bn * s.NBB : s.NBB; };
     const bool fact = s.mode & MODE_FACT, solve = s.mode & MODE_SOLVE;
 
@@ -128,19 +133,30 @@ std::vector<Task> build_order(const Shape &s) {
     // latency-bound and grow linearly with the tile order, not with its flops,
     // so a flop model misorders the list (tasks whose inputs are not ready are
     // claimed first and their CTAs wait).
-    const bool lat = (s.prof == PROF_F32_TC05);
-    auto c_potrf = [&](double t) { return lat ? 1.05 * t : cal.potrf * 6.0 * t * t * t / 3.0; };
+    const bool lat = (s.prof == PROF_F32_TC05), f64 = (s.prof == PROF_FP64);
+    // FP64 path, likewise in microseconds: a latency term plus the products at
+    // the rate of one of an SM's two CTAs
+    const double sub = std::min<double>(nb, cb), us = 2.0 / 0.11e6;   // us per multiply-add
+    auto ub = [&](int cnt) { return std::min<double>(nb, upd_blk(s.mode, cnt)); };
+    auto c_potrf = [&](double t) {
+        return f64 ? 0.24 * t + us * t * t * t / 3.0 : lat ? 1.05 * t : cal.potrf * 6.0 * t * t * t / 3.0;
+    };
     auto c_xinv = [&](double t) { return lat ? 1.5 * t : cal.potrf * 6.0 * t * t * t / 3.0; };
-    auto c_trsm = [&]() { return lat ? 0.27 * nb : cal.trsm * 2.0 * SUBB * nb * nb; };
+    auto c_trsm = [&]() {
+        return f64 ? 4.0 + us * sub * nb * (nb + IB) / 2 : lat ? 0.27 * nb : cal.trsm * 2.0 * SUBB * nb * nb;
+    };
     auto c_upd = [&](int cnt) {
-        return lat ? 5.0 + 0.011 * nb * cnt
-                   : cal.upd * SUBB * SUBB * nb * 2.0 * (cnt + cal.upd_fix) / (1.0 + cal.upd_fix);
+        return f64 ? 4.0 + us * ub(cnt) * ub(cnt) * nb * cnt
+                   : lat ? 5.0 + 0.011 * nb * cnt
+                         : cal.upd * SUBB * SUBB * nb * 2.0 * (cnt + cal.upd_fix) / (1.0 + cal.upd_fix);
     };
     auto c_strsm = [&](double t, double w, int parts) {
-        return lat ? 13.0 + 0.01 * t : cal.strsm * 3.0 * t * t * w / parts;
+        return f64 ? 8.0 * t / IB + us * t * (t + IB) / 2 * std::min(w, 64.0)
+                   : lat ? 13.0 + 0.01 * t : cal.strsm * 3.0 * t * t * w / parts;
     };
     auto c_supd = [&](double t, double w) {
-        return lat ? 8.0 + 0.04 * t : cal.supd * 2.0 * solve_rows(s.mode) * t * w;
+        return f64 ? 4.0 + us * sub * t * std::min(w, 64.0)
+                   : lat ? 8.0 + 0.04 * t : cal.supd * 2.0 * solve_rows(s.mode) * t * w;
     };
     if (cast) {
         // the copy engine delivers the stored triangle one tile column after
@@ -187,9 +203,9 @@ std::vector<Task> build_order(const Shape &s) {
                 upd_group_of(n, k, s.G, s.tail, &k0, &cnt, &gi);
                 if (k0 + cnt - 1 != k) continue;
                 for (int m = n; m < NT; ++m) {
-                    const int sub = (m == n) ? nbi(m) * (nbi(m) + 1) / 2 : nbi(m) * nbi(n);
+                    const int bm = nbu(m, cnt), nsub = (m == n) ? bm * (bm + 1) / 2 : bm * nbu(n, cnt);
                     const double dur = c_upd(cnt);
-                    const int id = add(TK_UPD, m, n, k0, cnt, sub, dur);
+                    const int id = add(TK_UPD, m, n, k0, cnt, nsub, dur);
                     ct[id].grp = gi;
                     if (gi == 0) edge(Cst[m + (size_t)NT * n], id);
                     edge(Tr[m + (size_t)NT * k], id);
@@ -243,13 +259,14 @@ std::vector<Task> build_order(const Shape &s) {
             }
         }
     }
-    return list_schedule(ct, s.P, nbi);
+    return list_schedule(ct, s.P, nbu);
 }
 
 // List scheduling of a coarse DAG (generation order topological) on P
 // workers with critical-path priorities; emits the sub-tasks in start order.
-template <class NBI>
-std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBI nbi) {
+// nbu(m, cnt): row blocks of tile m in an update of cnt panels.
+template <class NBU>
+std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBU nbu) {
     // bottom levels (generation order is topological)
     for (int i = (int)ct.size() - 1; i >= 0; --i) {
         double b = 0;
@@ -286,7 +303,6 @@ std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBI nbi) {
         Task t{};
         t.kind = c.kind; t.m = c.m; t.n = c.n; t.k = c.k; t.bn = c.bn; t.sub = 0; t.grp = c.grp;
         if (c.kind == TK_UPD) {
-            const int a = nbi(c.m);
             int bi = 0, bj = 0;
             if (c.m == c.n) {   // j-th lower sub-block (row-major over bi >= bj)
                 int rem = j;
@@ -294,10 +310,9 @@ std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBI nbi) {
                 while (rem > bi) { rem -= bi + 1; ++bi; }
                 bj = rem;
             } else {
-                bi = j / nbi(c.n);
-                bj = j % nbi(c.n);
+                bi = j / nbu(c.n, c.bn);
+                bj = j % nbu(c.n, c.bn);
             }
-            (void)a;
             t.sub = (int16_t)(bi | (bj << 8));
         } else if (c.kind == TK_TRSM || c.kind == TK_FWD_UPD || c.kind == TK_BWD_UPD || c.kind == TK_FWD_TRSM ||
                    c.kind == TK_BWD_TRSM) {
@@ -415,13 +430,48 @@ void free_exec_ws(ExecWs &w) {
 // the device; its update groups are single panels.
 static thread_local const Schedule *t_given = nullptr;
 
+// A descriptor whose rows are one column-major array: any row tiling of it has
+// the same addressing.
+static bool one_tile(const CHAM_desc_t *d) { return priv(d)->cm_view || d->mt == 1; }
+
+// Tile size of the FP64 executor.  The diagonal-tile factorizations are a
+// serial chain on one CTA each, so tiles of the caller's size (512, say) leave
+// the chip waiting for them: the executor uses tiles of EXEC_NB wherever the
+// storage allows it -- any size when it is column-major, else the largest
+// divisor of the storage tile up to EXEC_NB (multiples of 64 first; 48 at
+// least, below that the tasks are all overhead).  dpotrf of order 8192:
+// storage tile 512 24.9 ms, executor tile 256 12.8 ms, 128 9.8 ms, 64 14.9 ms.
+constexpr int EXEC_NB = 128;
+static int exec_tile(const CHAM_desc_t *A, const CHAM_desc_t *B) {
+    const bool free_a = one_tile(A), free_b = !B || one_tile(B);
+    if (free_a && free_b) return EXEC_NB;
+    const int nb = free_a ? B->mb : A->nb;   // A and B have the same row tile size
+    for (int d = EXEC_NB; d >= 64; d -= 64)
+        if (nb % d == 0) return d;
+    for (int d = std::min(EXEC_NB, nb); d >= 48; --d)
+        if (nb % d == 0) return d;
+    return nb;
+}
+
+// Panels per trailing update of the FP64 executor: a depth of n / 16, at least
+// 512 and at most the configured group (given in tiles of 512).  A deeper
+// group amortizes the C round trip, but a tile's last group only becomes ready
+// a few steps before the tile is factored, and a 128 x 128 x 4096 update takes
+// 0.8 ms on a CTA: order 8192 with depth 4096 21.0 ms, 1024 10.0, 512 9.8,
+// 256 10.4.
+constexpr int GROUP_NB = 512;
+static int group_f64(int N, int NB, int kgroup) {
+    const int depth = std::min(kgroup * GROUP_NB, std::max(512, N / 16));
+    return std::max(1, depth / NB);
+}
+
 int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B, cudaStream_t s,
                      ExecResult *res, int split, ExecWs *wsp, int grid_req, int flags, const CastIn *cin) {
     Context &c = ctx();
     ExecWs &w = wsp ? *wsp : g_ws;
     const int N = A->n;
-    const int NB = A->nb;
-    const int NT = A->nt;
+    const int NB = (t_given || A->dtyp == ChamRealFloat) ? A->nb : exec_tile(A, (mode & MODE_SOLVE) ? B : nullptr);
+    const int NT = (N + NB - 1) / NB;
     const int nrhs = (B && (mode & MODE_SOLVE)) ? B->n : 0;
     const int NBB = B ? B->nb : NB;
     const int NTB = nrhs ? B->nt : 0;
@@ -441,6 +491,7 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     // grid_req counts SMs; FP64 places two executor CTAs on each
     const int cps = f32 ? 1 : 2;
     const int grid = cps * ((grid_req > 0) ? std::min(grid_req, c.num_sms) : c.num_sms);
+    if (!f32 && !t_given) mode |= MODE_FINE;
     const int prof = !f32 ? PROF_FP64 : (tc ? PROF_F32_TC05 : PROF_F32_MMA);
     const bool full_inv = f32 && c.rec_tile && NB <= (64 << rec::MAX_LVL);
     // FP32 substitutions with full diagonal-tile inverses: computed off the
@@ -459,7 +510,7 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     // takes the exact sizes from the parameters): key the cache on that
     // canonical shape so that callers with many distinct N share schedules.
     // (the finer of the update and substitution row blocks decides)
-    const int gran = std::min(SUBB, solve_rows(mode));
+    const int gran = std::min(count_blk(mode), solve_rows(mode));
     const int last_sub = ((N - (NT - 1) * NB) + gran - 1) / gran;
     const int canonN = (NT - 1) * NB + std::min(NB, last_sub * gran);
     // nrhs enters the cost model (not the task list): keep it, with the last
@@ -468,7 +519,9 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     const int canonR = nrhs ? (NTB - 1) * NBB + std::min(NBB, ((nrhs - (NTB - 1) * NBB + 15) / 16) * 16) : 0;
     // update group size: fused k steps amortize the C round trip and the
     // dispatch of an update over G panels (CHAMELEON_B200_UPD_GROUP per path)
-    const int G = t_given ? 1 : std::max(1, prof == PROF_FP64 ? c.kgroup_f64 : (tc ? c.kgroup_tc : c.kgroup_f32));
+    const int G = t_given ? 1
+                          : prof == PROF_FP64 ? group_f64(N, NB, c.kgroup_f64)
+                                              : std::max(1, tc ? c.kgroup_tc : c.kgroup_f32);
     Shape sh{mode, canonN, NB, canonR, NBB, grid, prof, G, cin ? std::max(1, cin->h2d_gbs) : 0, upd_tail(prof)};
     const Schedule *sch = t_given ? t_given : get_schedule(sh);
     if (!sch) return CHAMELEON_ERR_OUT_OF_RESOURCES;
@@ -498,10 +551,14 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     p.A = A->mat;
     p.a_off = priv(A)->dev.off;
     p.a_ld = priv(A)->dev.ld;
+    p.a_nt = A->mt;
+    p.a_r = one_tile(A) ? NT : std::max(1, A->nb / NB);
     p.NTB = NTB; p.nrhs = nrhs; p.NBB = NBB;
     p.B = nrhs ? B->mat : nullptr;
     p.b_off = nrhs ? priv(B)->dev.off : nullptr;
     p.b_ld = nrhs ? priv(B)->dev.ld : nullptr;
+    p.b_nt = nrhs ? B->mt : 1;
+    p.b_r = nrhs ? (one_tile(B) ? NT : std::max(1, B->mb / NB)) : 1;
     int *ctr = (int *)w.ctr;
     p.updA = ctr;
     p.panA = ctr + (size_t)NT * NT;
@@ -829,7 +886,7 @@ static int dag_to_tasks(const cham_b200_dag_s &dag, int N, int NB, int nrhs, int
             return CHAMELEON_ERR_ILLEGAL_VALUE;
         }
     }
-    *out = list_schedule(ct, workers, nbi);
+    *out = list_schedule(ct, workers, [&](int m, int) { return nbi(m); });
     *mode_out = mode;
     if (!replay_ok(*out, mode, N, NB, NTB)) {
         out->clear();

@@ -78,7 +78,15 @@ static_assert(sizeof(Task) == 16, "Task is 16 bytes");
 // MODE_CAST: the FP32 tiles of A are produced inside the launch by TK_CAST
 // tasks from an FP64 column-major copy of A that is still arriving from the
 // host: each tile's first consumer waits for its cast.
-enum ExecMode : int { MODE_FACT = 1, MODE_SOLVE = 2, MODE_XINV = 4, MODE_NOINV = 8, MODE_CAST = 16 };
+// MODE_FINE (FP64): panel solves and substitution updates in 64-row blocks and
+// the updates of a single panel in 64 x 64 blocks.  Those tasks are on the
+// chain from one diagonal tile to the next; a 128-wide block of FP64 products
+// takes 12-25 us on one SM, four 64-wide ones run side by side.  The
+// counters count 64-blocks: an update of several panels, which keeps its
+// 128 x 128 blocks, counts for each 64-block it covers (upd_weight).
+enum ExecMode : int {
+    MODE_FACT = 1, MODE_SOLVE = 2, MODE_XINV = 4, MODE_NOINV = 8, MODE_CAST = 16, MODE_FINE = 32
+};
 
 constexpr int SUBB = 128;      // sub-block edge of trailing updates / row blocks
 // Row block of the substitution tasks (FWD/BWD TRSM and UPD) with full
@@ -86,7 +94,20 @@ constexpr int SUBB = 128;      // sub-block edge of trailing updates / row block
 // chain of 2 NT dependent steps, and 64-row tasks halve each step's latency.
 constexpr int SOLB = 64;
 // Row block of the substitution tasks of a launch mode.
-__host__ __device__ constexpr int solve_rows(int mode) { return (mode & 4 /*MODE_XINV*/) ? SOLB : SUBB; }
+__host__ __device__ constexpr int solve_rows(int mode) { return (mode & (4 | 32) /*XINV, FINE*/) ? SOLB : SUBB; }
+// Edge of the blocks that the counters count, and of an update task's block
+// (cnt panels).
+constexpr int FINEB = 64;
+__host__ __device__ constexpr int count_blk(int mode) { return (mode & 32 /*MODE_FINE*/) ? FINEB : SUBB; }
+__host__ __device__ constexpr int upd_blk(int mode, int cnt) { return cnt == 1 ? count_blk(mode) : SUBB; }
+// Counted blocks of an update task on a rows x cols block (diag: on the
+// diagonal, lower triangle only).
+__host__ __device__ __forceinline__ int upd_weight(int mode, int cnt, int rows, int cols, bool diag) {
+    const int e = count_blk(mode);
+    if (upd_blk(mode, cnt) == e) return 1;
+    const int a = (rows + e - 1) / e, b = (cols + e - 1) / e;
+    return diag ? a * (a + 1) / 2 : a * b;
+}
 
 struct ExecState {
     int next;          // dispatch cursor (alone in its 128-byte line: the contended atomic)
@@ -118,13 +139,18 @@ struct ExecParams {
     int mode;
     int upper;
     int NT, N, NB;          // A: NT x NT tiles, order N, tile size NB (square tiles)
+    // The executor's tiles may be finer than the storage's: a_r x a_r of them
+    // make up one storage tile, column-major inside it (a_r = NT: the matrix
+    // is one column-major array).
     void *A;                // double or float tiles
-    const int64_t *a_off;   // element offset of tile (m,n) at a_off[m + NT*n]
-    const int *a_ld;        // leading dimension of tile row m
-    int NTB, nrhs, NBB;     // B: NT x NTB tiles of NB x NBB
+    const int64_t *a_off;   // element offset of storage tile (M,N) at a_off[M + a_nt*N]
+    const int *a_ld;        // leading dimension of storage tile row M
+    int a_nt, a_r;
+    int NTB, nrhs, NBB;     // B: NT x NTB tiles of NB x NBB (rows likewise, b_r per storage tile)
     void *B;
-    const int64_t *b_off;   // b_off[m + NT*bn]
+    const int64_t *b_off;   // b_off[M + b_nt*bn]
     const int *b_ld;
+    int b_nt, b_r;
     int *updA, *panA, *fwdB, *fwdDone, *bwdB, *bwdDone;
     void *invd;             // full_inv: NT inverted NB x NB diagonal tiles (ld NB);
                             // else NT * NIB inverted IB x IB blocks (element type of A)

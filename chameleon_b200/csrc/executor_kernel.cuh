@@ -31,7 +31,11 @@ template <class T>
 struct Dims {
     const ExecParams &p;
     __device__ int tm(int m) const { return (m == p.NT - 1) ? p.N - m * p.NB : p.NB; }
-    __device__ int nbi(int m) const { return (tm(m) + SUBB - 1) / SUBB; }
+    // Row blocks of tile m that the counters count.
+    __device__ int nbi(int m) const {
+        const int e = count_blk(p.mode);
+        return (tm(m) + e - 1) / e;
+    }
     __device__ int S(int m, int n) const {
         const int a = nbi(m), b = nbi(n);
         return (m == n) ? a * (a + 1) / 2 : a * b;
@@ -39,18 +43,38 @@ struct Dims {
     __device__ int wB(int bn) const { return (bn == p.NTB - 1) ? p.nrhs - bn * p.NBB : p.NBB; }
     // Logical lower tile (m,n), m >= n.
     __device__ ViewT<T> A(int m, int n) const {
-        T *a = static_cast<T *>(p.A);
-        if (!p.upper) return ViewT<T>{a + p.a_off[m + p.NT * n], 1, p.a_ld[m]};
-        return ViewT<T>{a + p.a_off[n + p.NT * m], p.a_ld[n], 1};
+        if (!p.upper) return stored(m, n);
+        return stored(n, m).t();
     }
-    __device__ ViewT<T> Bt(int m, int bn) const {
-        return ViewT<T>{static_cast<T *>(p.B) + p.b_off[m + p.NT * bn], 1, p.b_ld[m]};
+    // Stored tile (P, Q): its place inside the storage tile that holds it.
+    // (FP32 tiles are storage tiles)
+    __device__ ViewT<T> stored(int P, int Q) const {
+        if constexpr (sizeof(T) == 4)
+            return ViewT<T>{static_cast<T *>(p.A) + p.a_off[P + p.a_nt * Q], 1, p.a_ld[P]};
+        const int Pc = P / p.a_r, Qc = Q / p.a_r;
+        const int64_t ld = p.a_ld[Pc];
+        return ViewT<T>{static_cast<T *>(p.A) + p.a_off[Pc + p.a_nt * Qc] + (int64_t)(P - Pc * p.a_r) * p.NB +
+                            (int64_t)(Q - Qc * p.a_r) * p.NB * ld,
+                        1, ld};
     }
+    __device__ ViewT<T> btile(void *B, int m, int bn) const {
+        if constexpr (sizeof(T) == 4)
+            return ViewT<T>{static_cast<T *>(B) + p.b_off[m + p.b_nt * bn], 1, p.b_ld[m]};
+        const int M = m / p.b_r;
+        return ViewT<T>{static_cast<T *>(B) + p.b_off[M + p.b_nt * bn] + (int64_t)(m - M * p.b_r) * p.NB, 1,
+                        p.b_ld[M]};
+    }
+    __device__ ViewT<T> Bt(int m, int bn) const { return btile(p.B, m, bn); }
     // Tile (m, bn) of the forward results (MODE_XINV), layout of B.
-    __device__ ViewT<T> Yt(int m, int bn) const {
-        return ViewT<T>{static_cast<T *>(p.Y) + p.b_off[m + p.NT * bn], 1, p.b_ld[m]};
+    __device__ ViewT<T> Yt(int m, int bn) const { return btile(p.Y, m, bn); }
+    // Panels of A from k on, at most cnt, whose columns follow each other in
+    // one storage tile, and (in K) their total width.
+    __device__ int run(int k, int cnt, int *K) const {
+        const int c = min(cnt, p.a_r - k % p.a_r);
+        *K = min(c * p.NB, p.N - k * p.NB);
+        return c;
     }
-    // Row blocks of tile m in the substitution updates (SOLB rows with MODE_XINV).
+    // Row blocks of tile m in the substitution updates.
     __device__ int nsb(int m) const {
         const int r = solve_rows(p.mode);
         return (tm(m) + r - 1) / r;
@@ -197,8 +221,9 @@ __device__ void cast_tile(const Task &t, const ExecParams &p, const Dims<T> &d, 
     const int rows = d.tm(P), cols = d.tm(Q);
     const bool diag = (P == Q);
     const double *src = p.csrc + (int64_t)P * p.NB + (int64_t)Q * p.NB * p.csrc_ld;
-    T *dst = static_cast<T *>(p.A) + p.a_off[P + p.NT * Q];
-    const int ldd = p.a_ld[P];
+    const ViewT<T> dv = d.stored(P, Q);
+    T *dst = dv.p;
+    const int64_t ldd = dv.cs;
     for (int j = threadIdx.x; j < cols; j += NT_CTA) s_col[j] = 0.0;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -257,9 +282,7 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
             else if (d.tm(t.k) <= psm::MAXN) info = psm::potrf(d.A(t.k, t.k), d.tm(t.k), d.inv(t.k), smem, ph);
             else info = rec::tile_potrf_blk<T, SP>(d.A(t.k, t.k), d.tm(t.k), d.inv(t.k), smem, ph);
         } else {
-            // FP64: the lean form (64-row panels, leaf on the staging area) fits
-            // the two-CTAs-per-SM shared memory
-            info = rec::tile_potrf_blk<T, SP, 64, true>(d.A(t.k, t.k), d.tm(t.k), d.inv(t.k), smem, ph);
+            info = rec::tile_potrf_fused(d.A(t.k, t.k), d.tm(t.k), d.inv(t.k), smem, ph);
         }
         if (info && threadIdx.x == 0) {
             atomicMin(&p.st->info, t.k * p.NB + info);
@@ -277,12 +300,20 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
         rec::tile_inv_blk<T>(d.A(t.k, t.k), d.tm(t.k), d.inv(t.k), smem);
         break;
     case TK_TRSM: {
-        const int r0 = t.sub * SUBB;
-        const int rows = min(SUBB, d.tm(t.m) - r0);
+        const int e = count_blk(p.mode);
+        const int r0 = t.sub * e;
+        const int rows = min(e, d.tm(t.m) - r0);
         bool done = false;
         if constexpr (std::is_same<T, float>::value) {
             if (p.full_inv) {
                 rec::apply_inv_right<T, SP>(d.A(t.m, t.k).sub(r0, 0), rows, d.X(t.k), d.tm(t.k), smem);
+                done = true;
+            }
+        }
+        if constexpr (sizeof(T) == 8) {
+            if (rows <= FINEB) {
+                trsm_rows<T, SP, Cfg64<T, SP>>(d.A(t.m, t.k).sub(r0, 0), rows, d.A(t.k, t.k), d.tm(t.k), d.inv(t.k),
+                                               smem);
                 done = true;
             }
         }
@@ -307,8 +338,9 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
     }
     case TK_UPD: {
         const int bi = t.sub & 0xff, bj = (t.sub >> 8) & 0xff;
-        const int rows = min(SUBB, d.tm(t.m) - bi * SUBB), cols = min(SUBB, d.tm(t.n) - bj * SUBB);
-        const VT C = d.A(t.m, t.n).sub(bi * SUBB, bj * SUBB);
+        const int e = upd_blk(p.mode, t.bn);
+        const int rows = min(e, d.tm(t.m) - bi * e), cols = min(e, d.tm(t.n) - bj * e);
+        const VT C = d.A(t.m, t.n).sub(bi * e, bj * e);
         const bool diag = (t.m == t.n) && (bi == bj);
         if constexpr (TC) {
             // the split tiles of panels k .. k + bn - 1 of one tile row are
@@ -355,18 +387,37 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
             break;
         }
         if constexpr (sizeof(T) == 8) {
+            if (e == FINEB) {   // one panel
+                Acc<Cfg64<T, SP>> acc;
+                acc.zero();
+                cta_gemm(acc, d.A(t.m, t.k).sub(bi * e, 0), d.A(t.n, t.k).sub(bj * e, 0), rows, cols, d.tm(t.k), smem);
+                acc.sub_from(C, rows, cols, diag);
+                break;
+            }
             // FP64: two 128 x 64 halves (the 111 KB of stages that let two
             // CTAs share an SM); on a diagonal block the second half is the
             // 64 x 64 lower block of rows and columns 64..127
             for (int h = 0; h < 2; ++h) {
                 const int c0 = 64 * h, r0 = diag ? c0 : 0;
                 if (c0 >= cols || r0 >= rows) break;
-                Acc<Cfg12864<T, SP>> acc;
-                acc.zero();
-                for (int k = t.k; k < t.k + t.bn; ++k)
-                    cta_gemm(acc, d.A(t.m, k).sub(bi * SUBB + r0, 0), d.A(t.n, k).sub(bj * SUBB + c0, 0), rows - r0,
-                             min(64, cols - c0), d.tm(k), smem);
-                acc.sub_from(C.sub(r0, c0), rows - r0, min(64, cols - c0), diag);
+                const int mr = rows - r0, nc = min(64, cols - c0);
+                auto product = [&](auto &acc) {
+                    acc.zero();
+                    for (int k = t.k, K; k < t.k + t.bn;) {
+                        const int c = d.run(k, t.k + t.bn - k, &K);
+                        cta_gemm(acc, d.A(t.m, k).sub(bi * e + r0, 0), d.A(t.n, k).sub(bj * e + c0, 0), mr, nc, K,
+                                 smem);
+                        k += c;
+                    }
+                    acc.sub_from(C.sub(r0, c0), mr, nc, diag);
+                };
+                if (mr <= 64) {
+                    Acc<Cfg64<T, SP>> acc;
+                    product(acc);
+                } else {
+                    Acc<Cfg12864<T, SP>> acc;
+                    product(acc);
+                }
             }
         } else {
             Acc<Cfg128<T, SP>> acc;
@@ -433,7 +484,7 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
         // MODE_XINV: forward updates read Y_k into B_m, backward ones read B_k
         // into Y_m, in SOLB-row blocks
         const bool y = p.mode & MODE_XINV;
-        const int rb = y ? SOLB : SUBB;
+        const int rb = solve_rows(p.mode);
         const int r0 = t.sub * rb;
         const int rows = min(rb, d.tm(t.m) - r0);
         const int w = d.wB(t.bn);
@@ -442,7 +493,12 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
         const VT L = (t.kind == TK_FWD_UPD) ? d.A(t.m, t.k).sub(r0, 0) : d.A(t.k, t.m).t().sub(r0, 0);
         for (int c0 = 0; c0 < w; c0 += 64) {
             const int wc = min(64, w - c0);
-            if (y) {
+            if (rows <= SOLB && wc <= Cfg64N<T, SP>::BN && sizeof(T) == 8) {   // few right-hand sides
+                Acc<Cfg64N<T, SP>> acc;
+                acc.zero();
+                cta_gemm(acc, L, Bk.sub(0, c0).t(), rows, wc, d.tm(t.k), smem);
+                acc.sub_from(Bm.sub(0, c0), rows, wc, false);
+            } else if (rows <= SOLB) {
                 Acc<Cfg64<T, SP>> acc;
                 acc.zero();
                 cta_gemm(acc, L, Bk.sub(0, c0).t(), rows, wc, d.tm(t.k), smem);
@@ -457,6 +513,15 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
         break;
     }
     }
+}
+
+// What the completion of a task adds to its counter.
+template <class T>
+__device__ __forceinline__ int task_weight(const Task &t, const ExecParams &p, const Dims<T> &d) {
+    if (sizeof(T) == 4 || t.kind != TK_UPD || t.bn == 1) return 1;
+    const int bi = t.sub & 0xff, bj = (t.sub >> 8) & 0xff;
+    return upd_weight(p.mode, t.bn, min(SUBB, d.tm(t.m) - bi * SUBB), min(SUBB, d.tm(t.n) - bj * SUBB),
+                      t.m == t.n && bi == bj);
 }
 
 __device__ inline int *task_counter(const Task &t, const ExecParams &p) {
@@ -542,7 +607,7 @@ __global__ void __launch_bounds__(NT_CTA, dag_ctas_per_sm<T, TC>()) cholesky_dag
         if (threadIdx.x == 0) {
             int *ctr = task_counter(t, p);
             if (TC && ah.ready && ah.t.kind == TK_UPD) ah.rel = ctr;   // released by the next task
-            else red_release_add(ctr, 1);
+            else red_release_add(ctr, task_weight<T>(t, p, d));
             ++ndone;
             if (p.trace) {
                 unsigned smid;
@@ -559,7 +624,10 @@ __global__ void __launch_bounds__(NT_CTA, dag_ctas_per_sm<T, TC>()) cholesky_dag
 template <class T, int SP, bool TC>
 constexpr size_t dag_smem_bytes() {
     // FP64: two CTAs per SM, each task within a 128 x 64 DMMA tile's stages
-    if (sizeof(T) == 8 && !TC) return Cfg12864<T, SP>::SMEM_BYTES + 1024;
+    if (sizeof(T) == 8 && !TC) {
+        static_assert(sizeof(T) == 4 || (size_t)rec::fused_smem_elems() <= Cfg12864<T, SP>::SMEM_ELEMS, "diagonal tile");
+        return Cfg12864<T, SP>::SMEM_BYTES + 1024;
+    }
     // one CTA per SM: every variant may use the shared memory its largest task needs
     // (the tcgen05 stages; FP32: the shared-memory diagonal-tile factorization)
     size_t b = tile_smem_bytes<T, SP>() + 1024;

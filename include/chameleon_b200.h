@@ -69,7 +69,8 @@ typedef enum {
                                              diagonal tiles, kept across refinement solves (default) */
 #define CHAMELEON_B200_POTRF_CTA      108 /* 1: one executor CTA runs all diagonal-tile
                                              factorizations; 0: any CTA (default) */
-#define CHAMELEON_B200_UPD_GROUP_F64  109 /* panels applied per trailing-update task, FP64 path (default 8) */
+#define CHAMELEON_B200_UPD_GROUP_F64  109 /* most panels (of 512 columns) applied per trailing-update task, FP64
+                                             path (default 8) */
 #define CHAMELEON_B200_UPD_GROUP_F32  110 /* the same, FP32 split products on mma.sync (default 1) */
 #define CHAMELEON_B200_UPD_GROUP_TC   111 /* the same, FP32 BF16x3 on tcgen05 (default 8) */
 #define CHAMELEON_B200_FACTOR_NB      112 /* tile size of the mixed solver's FP32 factorization;

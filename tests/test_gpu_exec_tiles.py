@@ -1,0 +1,113 @@
+"""FP64 executor tiles finer than the storage's, and the 64 x 64 leaf.
+
+The executor picks its own tile size inside the storage tiles (any size for
+column-major storage, a divisor of the tile otherwise): every layout, triangle
+and remainder is checked against numpy's factor and solution.  Errors are
+bounded by the backward error of Cholesky and of the two substitutions,
+a small multiple of n eps relative to the norms (Higham, Accuracy and
+Stability of Numerical Algorithms, theorems 10.3 and 10.4): 8 n eps.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+UPPER, LOWER = 121, 122
+
+
+def spd(n, seed, scale=1.0):
+    g = np.random.default_rng(seed)
+    a = g.uniform(-0.5, 0.5, (n, n))
+    return (a + a.T + n * np.eye(n)) * scale
+
+
+@pytest.mark.parametrize("layout", ["tiles", "array"])
+@pytest.mark.parametrize("uplo", [UPPER, LOWER])
+@pytest.mark.parametrize("n,nb,nrhs", [(1, 64, 1), (127, 512, 2), (129, 512, 9), (385, 128, 1), (700, 320, 70),
+                                       (641, 200, 8), (300, 7, 3), (1031, 384, 65), (1152, 512, 33)])
+def test_posv_and_potrs_over_tilings(cb, layout, uplo, n, nb, nrhs):
+    import torch
+    A0 = spd(n, n + nb)
+    B0 = np.random.default_rng(nb).uniform(-0.5, 0.5, (n, nrhs))
+    poisoned = np.where(np.tri(n, k=0 if uplo == LOWER else -1, dtype=bool) == (uplo == LOWER), A0, np.nan)
+    if layout == "array":   # torch (columns, rows): column-major storage
+        tA, tB = torch.from_numpy(poisoned.T.copy()).cuda(), torch.from_numpy(B0.T.copy()).cuda()
+        dA, dB = cb.Desc.create(n, n, nb, mat=tA), cb.Desc.create(n, nrhs, nb, mat=tB)
+    else:
+        dA, dB = cb.Desc.create(n, n, nb), cb.Desc.create(n, nrhs, nb)
+        dA.from_numpy(poisoned)
+        dB.from_numpy(B0)
+    get = (lambda: (tA.cpu().numpy().T, tB.cpu().numpy().T)) if layout == "array" else (
+        lambda: (dA.to_numpy(uplo), dB.to_numpy()))
+    X = np.linalg.solve(A0, B0)
+    for step in ("posv", "potrs"):
+        if step == "potrs":
+            if layout == "array":
+                tB.copy_(torch.from_numpy(B0.T.copy()))
+            else:
+                dB.from_numpy(B0)
+        assert (cb.dposv_Tile if step == "posv" else cb.dpotrs_Tile)(uplo, dA, dB) == 0
+        F, Y = get()
+        L = np.tril(F) if uplo == LOWER else np.triu(F).T
+        assert np.linalg.norm(A0 - L @ L.T) <= 8 * n * EPS * np.linalg.norm(A0)
+        assert np.linalg.norm(Y - X) <= 8 * n * EPS * np.linalg.cond(A0) * np.linalg.norm(X)
+        if layout == "array" and n > 1:   # the other triangle is not written
+            off = np.triu(F, 1) if uplo == LOWER else np.tril(F, -1)
+            assert np.isnan(off[off != 0]).all()
+
+
+@pytest.mark.parametrize("n,scale", [(n, 1.0) for n in (1, 7, 8, 9, 31, 33, 56, 57, 64, 65, 72, 128)] +
+                         [(40, 1e-290), (64, 1e290), (23, 3e-309)])
+@pytest.mark.parametrize("uplo", [UPPER, LOWER])
+def test_tile_potrf_fp64_orders_and_scales(cb, uplo, n, scale):
+    """Every remainder of the 8-wide panels, and pivots beyond the range of
+    the reciprocal estimates (subnormal ones included: absolute errors of a
+    few subnormal units, relative to sqrt of them, bound the last case)."""
+    import torch
+    L = cb.lib()
+    A0 = spd(n, 3 * n, scale)
+    t = torch.from_numpy(A0.T.copy()).cuda()
+    info = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    h = ctypes.c_void_p()
+    assert L.CHAM_B200_Handle_Create(ctypes.byref(h), None) == 0
+    assert L.CUDA_dpotrf(uplo, n, t.data_ptr(), n, None, 0, info.data_ptr(), h) == 0
+    torch.cuda.synchronize()
+    L.CHAM_B200_Handle_Destroy(h)
+    assert int(info) == 0
+    F = t.cpu().numpy().T
+    Lf = np.tril(F) if uplo == LOWER else np.triu(F).T
+    # in units of the scale, so that the squares stay representable
+    r = np.sqrt(scale)
+    err = np.abs(A0 / scale - (Lf / r) @ (Lf / r).T).max() / n
+    assert err <= 8 * n * EPS + 8 * 4.94e-324 / scale
+
+
+@pytest.mark.parametrize("n", [1, 9, 64, 100, 256])
+@pytest.mark.parametrize("scale", [1.0, 1e-34, 1e34])
+def test_tile_potrf_fp32_scales(cb, n, scale):
+    import torch
+    L = cb.lib()
+    A0 = spd(n, 5 * n, scale).astype(np.float32)
+    t = torch.from_numpy(A0.T.copy()).cuda()
+    info = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    h = ctypes.c_void_p()
+    assert L.CHAM_B200_Handle_Create(ctypes.byref(h), None) == 0
+    assert L.CUDA_spotrf(LOWER, n, t.data_ptr(), n, None, 0, info.data_ptr(), h) == 0
+    torch.cuda.synchronize()
+    L.CHAM_B200_Handle_Destroy(h)
+    assert int(info) == 0
+    Lf = np.tril(t.cpu().numpy().T).astype(np.float64)
+    err = np.abs(A0.astype(np.float64) - Lf @ Lf.T).max() / (n * scale)
+    # the panels' 3xTF32 products keep 2^-21 relative to the operands
+    assert err <= 8 * n * 2.0 ** -24 + 2.0 ** -21
+
+
+@pytest.mark.parametrize("n,bad", [(64, 1), (64, 9), (64, 64), (130, 65), (200, 129), (200, 200)])
+def test_first_non_positive_pivot(cb, n, bad):
+    import torch
+    A0 = spd(n, n)
+    A0[bad - 1, bad - 1] = -1.0
+    t = torch.from_numpy(A0.copy()).cuda()
+    assert cb.dpotrf(LOWER, n, t, n) == bad
