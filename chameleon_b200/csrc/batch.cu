@@ -39,10 +39,24 @@
 
 namespace chb {
 
+// Shared memory of the lean shapes: FP64 at two CTAs per SM keeps the leaf's
+// inverse beside the staging area (rec::tile_potrf_fused).
+template <class T, int MINB>
+constexpr bool lean_fused() {
+    return sizeof(T) == 8 && MINB == 2;
+}
+template <class T, int MINB>
+constexpr size_t lean_smem_bytes() {
+    return (lean_fused<T, MINB>() ? sizeof(T) * rec::fused_smem_elems() : sizeof(T) * rec::lean_smem_elems<T, SPLIT_BF16X3>()) +
+           64;
+}
+
 // Generic bin: factor (+ forward and backward solve) of one system per task.
 // LEAN: 64-row panels and the leaf blocks aliased onto the GEMM staging area
 // (rec::lean_smem_elems), MINB CTAs per SM, so that the latency-bound leaf of
-// one system overlaps the GEMMs and leaves of the systems beside it.
+// one system overlaps the GEMMs and leaves of the systems beside it.  Right-
+// hand sides are solved in strips of 8 columns in shared memory where the
+// order allows it.
 template <class T, bool LEAN = false, int MINB = 1>
 __global__ void __launch_bounds__(NT_CTA, MINB) posv_batch_kernel(const BatchItem *items, int count, T *A, T *B,
                                                                   int upper, int *info, int *cursor, T *scratch,
@@ -59,12 +73,31 @@ __global__ void __launch_bounds__(NT_CTA, MINB) posv_batch_kernel(const BatchIte
         if (i >= count) break;
         const BatchItem it = items[i];
         const ViewT<T> Lv = upper ? ViewT<T>{A + it.a_off, it.lda, 1} : ViewT<T>{A + it.a_off, 1, it.lda};
-        const int r = LEAN ? rec::tile_potrf_blk<T, SPLIT_BF16X3, 64, true>(Lv, it.n, invd, smem)
-                           : rec::tile_potrf_blk<T, SPLIT_BF16X3>(Lv, it.n, invd, smem);
+        int r;
+        if constexpr (LEAN && lean_fused<T, MINB>()) r = rec::tile_potrf_fused(Lv, it.n, invd, smem);
+        else if constexpr (LEAN) r = rec::tile_potrf_blk<T, SPLIT_BF16X3, 64, true>(Lv, it.n, invd, smem);
+        else r = rec::tile_potrf_blk<T, SPLIT_BF16X3>(Lv, it.n, invd, smem);
         if (threadIdx.x == 0 && info) info[it.info_idx] = r;
         if (r == 0 && it.nrhs > 0) {
             const ViewT<T> X{B + it.b_off, 1, it.ldb};
-            for (int c0 = 0; c0 < it.nrhs; c0 += IB) {
+            constexpr size_t smem_bytes = LEAN ? lean_smem_bytes<T, MINB>() : tile_smem_bytes<T>();
+            const bool strips = rec::strip_smem_elems(it.n) * sizeof(double) <= smem_bytes;
+            for (int c0 = 0; strips && c0 < it.nrhs; c0 += rec::SW) {
+                const int w = min(rec::SW, it.nrhs - c0), ld = rec::strip_ld(it.n), np = ld - 4;
+                double *sX = reinterpret_cast<double *>(smem_raw), *sR = sX + rec::SW * ld;
+                for (int idx = threadIdx.x; idx < rec::SW * np; idx += NT_CTA) {
+                    const int rr = idx % np, cc = idx / np;
+                    sX[rr + cc * ld] = (rr < it.n && cc < w) ? (double)*X.at(rr, c0 + cc) : 0.0;
+                }
+                rec::strip_sweep<T>(Lv, it.n, invd, sX, ld, sR, false);
+                rec::strip_sweep<T>(Lv, it.n, invd, sX, ld, sR, true);
+                for (int idx = threadIdx.x; idx < w * it.n; idx += NT_CTA) {
+                    const int rr = idx % it.n, cc = idx / it.n;
+                    *X.at(rr, c0 + cc) = (T)sX[rr + cc * ld];
+                }
+                __syncthreads();
+            }
+            for (int c0 = strips ? it.nrhs : 0; c0 < it.nrhs; c0 += IB) {
                 const int w = min(IB, it.nrhs - c0);
                 // a narrow last block (few right-hand sides, the common case)
                 // runs on the narrow tile instead of padding it to 64 columns
@@ -79,11 +112,6 @@ __global__ void __launch_bounds__(NT_CTA, MINB) posv_batch_kernel(const BatchIte
         }
         cta_sync_global();
     }
-}
-
-template <class T>
-constexpr size_t lean_smem_bytes() {
-    return sizeof(T) * rec::lean_smem_elems<T, SPLIT_BF16X3>() + 64;
 }
 
 // Small bin (n <= 64): system in shared memory.  sD holds the identity-padded
@@ -179,8 +207,7 @@ __global__ void __launch_bounds__(NT_CTA, 1) trsm_batch_kernel(const TrsmItem *i
     extern __shared__ __align__(128) double smem[];
     __shared__ int s_i;
     double *invd = scratch + (int64_t)blockIdx.x * nib * IB * IB;
-    double *sD = smem + Cfg12864<double>::SMEM_ELEMS;
-    double *sInv = sD + IB * LDD;
+    double *sD = smem, *sInv = sD + IB * LEAF_LD;
     while (true) {
         if (threadIdx.x == 0) s_i = atomicAdd(cursor, 1);
         __syncthreads();
@@ -198,13 +225,12 @@ __global__ void __launch_bounds__(NT_CTA, 1) trsm_batch_kernel(const TrsmItem *i
         }
         for (int jb = 0; jb < it.na; jb += IB) {
             const int nbk = min(IB, it.na - jb);
-            for (int idx = threadIdx.x; idx < nbk * nbk; idx += NT_CTA) {
-                const int r = idx % nbk, c = idx / nbk;
-                sD[r + c * LDD] = (r >= c) ? *L.at(jb + r, jb + c) : 0.0;
+            rec::leaf64_load(L.sub(jb, jb), nbk, sD);
+            rec::leaf64_core<double, false>(sD, sInv, nbk, unit != 0);
+            for (int idx = threadIdx.x; idx < IB * IB; idx += NT_CTA) {
+                const int r = idx % IB, c = idx / IB;
+                invd[(int64_t)(jb / IB) * IB * IB + idx] = (r < nbk && c < nbk) ? sInv[r + c * LEAF_LD] : 0.0;
             }
-            __syncthreads();
-            blk_inv(sD, sInv, nbk, unit != 0);
-            store_inv(invd + (int64_t)(jb / IB) * IB * IB, sInv);
             __syncthreads();
         }
         cta_sync_global();
@@ -249,13 +275,13 @@ int set_attrs() {
     CHB_CUDA(cudaFuncSetAttribute(posv_batch_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)tile_smem_bytes<float>()));
     CHB_CUDA(cudaFuncSetAttribute(posv_batch_kernel<double, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)lean_smem_bytes<double>()));
+                                  (int)lean_smem_bytes<double, 2>()));
     CHB_CUDA(cudaFuncSetAttribute(posv_batch_kernel<double, true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)lean_smem_bytes<double>()));
+                                  (int)lean_smem_bytes<double, 3>()));
     CHB_CUDA(cudaFuncSetAttribute(posv_batch_kernel<float, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)lean_smem_bytes<float>()));
+                                  (int)lean_smem_bytes<float, 2>()));
     CHB_CUDA(cudaFuncSetAttribute(posv_batch_kernel<float, true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)lean_smem_bytes<float>()));
+                                  (int)lean_smem_bytes<float, 3>()));
 #define CHB_SMALL_ATTR(T, K)                                                                          \
     CHB_CUDA(cudaFuncSetAttribute(posv_small_kernel<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                   (int)small_smem_bytes<T>()))
@@ -320,8 +346,8 @@ bool shape_fits(int shape) {
     case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, posv_small_kernel<T, 1>, NT_CTA, small_smem_bytes<T>()); break;
     case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, posv_small_kernel<T, 2>, NT_CTA, small_smem_bytes<T>()); break;
     case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, posv_small_kernel<T, 3>, NT_CTA, small_smem_bytes<T>()); break;
-    case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, posv_batch_kernel<T, true, 2>, NT_CTA, lean_smem_bytes<T>()); break;
-    case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, posv_batch_kernel<T, true, 3>, NT_CTA, lean_smem_bytes<T>()); break;
+    case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, posv_batch_kernel<T, true, 2>, NT_CTA, lean_smem_bytes<T, 2>()); break;
+    case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, posv_batch_kernel<T, true, 3>, NT_CTA, lean_smem_bytes<T, 3>()); break;
     default: return false;
     }
     cudaGetLastError();
@@ -343,8 +369,8 @@ int launch_shape(int shape, const BatchItem *d_items, int cnt, int nmax, T *A, T
     case 1: posv_small_kernel<T, 1><<<grid, NT_CTA, small_smem_bytes<T>(), st>>>(d_items, cnt, A, B, upper, info, cursor); break;
     case 2: posv_small_kernel<T, 2><<<grid, NT_CTA, small_smem_bytes<T>(), st>>>(d_items, cnt, A, B, upper, info, cursor); break;
     case 3: posv_small_kernel<T, 3><<<grid, NT_CTA, small_smem_bytes<T>(), st>>>(d_items, cnt, A, B, upper, info, cursor); break;
-    case 4: posv_batch_kernel<T, true, 2><<<grid, NT_CTA, lean_smem_bytes<T>(), st>>>(d_items, cnt, A, B, upper, info, cursor, scr, nib); break;
-    case 5: posv_batch_kernel<T, true, 3><<<grid, NT_CTA, lean_smem_bytes<T>(), st>>>(d_items, cnt, A, B, upper, info, cursor, scr, nib); break;
+    case 4: posv_batch_kernel<T, true, 2><<<grid, NT_CTA, lean_smem_bytes<T, 2>(), st>>>(d_items, cnt, A, B, upper, info, cursor, scr, nib); break;
+    case 5: posv_batch_kernel<T, true, 3><<<grid, NT_CTA, lean_smem_bytes<T, 3>(), st>>>(d_items, cnt, A, B, upper, info, cursor, scr, nib); break;
     default: return CHAMELEON_ERR_ILLEGAL_VALUE;
     }
     CHB_LAUNCHED(1);

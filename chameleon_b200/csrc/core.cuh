@@ -3,7 +3,7 @@
 // Every tile operation of the Cholesky path (reference: the POTRF / TRSM /
 // SYRK / GEMM tile kernels of coreblas and gpucublas, e.g.
 // coreblas/compute/core_zpotrf.c:75-81, gpucublas/compute/cuda_zgemm.c:24-45)
-// is expressed with three CTA-wide primitives, generic over the element type:
+// is expressed with two CTA-wide primitives, generic over the element type:
 //
 //   cta_gemm      acc(i,j) += sum_k A(i,k) * B(j,k)  ("NT" form), operands
 //                 staged global -> shared by cp.async (two-stage pipeline, any
@@ -12,8 +12,6 @@
 //                   float : split products on mma.sync with FP32 accumulation,
 //                           BF16x3 (x = hi + lo in bf16, hi*hi + hi*lo + lo*hi,
 //                           m16n8k16) or TF32x3 (same split in tf32, m16n8k8);
-//   blk_inv       the explicit inverse of a <= 64 x 64 triangular block in
-//                 shared memory;
 //   trsm_rows / trsm_left   blocked triangular solves that apply the inverted
 //                 64 x 64 diagonal blocks, so that all bulk work is GEMM-shaped.
 //
@@ -33,8 +31,7 @@ namespace chb {
 constexpr int NT_CTA = 256;   // threads per CTA of every tile kernel
 constexpr int KC     = 32;    // k-extent of one pipeline stage
 constexpr int IB     = 64;    // inner block of POTRF / TRSM (inverted diagonal blocks)
-constexpr int LDD    = IB + 1;// leading dimension of the inner block in shared memory
-constexpr int LEAF_LD = IB + 4;   // the same in the 64 x 64 leaf (rec.cuh)
+constexpr int LEAF_LD = IB + 4;   // leading dimension of an inner block in shared memory (rec.cuh)
 
 enum SplitKind : int { SPLIT_BF16X3 = 0, SPLIT_TF32X3 = 1 };
 
@@ -472,51 +469,6 @@ __device__ void cta_gemm(Acc<C> &acc, const ViewT<typename C::T> &A, const ViewT
     else if (!ak && bk) cta_gemm_impl<C, false, true>(acc, A, B, M, N, K, smem, alA, alB);
     else if (ak && !bk) cta_gemm_impl<C, true, false>(acc, A, B, M, N, K, smem, alA, alB);
     else cta_gemm_impl<C, true, true>(acc, A, B, M, N, K, smem, alA, alB);
-}
-
-// ---------------------------------------------------------------------------
-// Inner-block triangular inverse in shared memory.  sD: n x n (n <= IB)
-// column-major with leading dimension LDD, lower triangle valid.
-// ---------------------------------------------------------------------------
-// sInv = L^{-1} for L = lower triangle of sD (n x n): row sweep, row i from
-// rows < i; 4 threads per column split the dot product (shuffle combine).
-template <class T>
-__device__ inline void blk_inv(const T *sD, T *sInv, int n, bool unit = false) {
-    // sInv has room for IB x LDD elements: the sweep works at stride LDD
-    // (conflict-free column reads), then compacts to stride IB in place.
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < IB * LDD; idx += NT_CTA) sInv[idx] = T(0);
-    __syncthreads();
-    const int c = tid >> 2, part = tid & 3;   // 64 columns x 4 parts
-    for (int i = 0; i < n; ++i) {
-        T s = T(0);
-        if (c < i) {
-            for (int k = c + part; k < i; k += 4) s += sD[i + k * LDD] * sInv[k + c * LDD];
-        }
-        s += __shfl_down_sync(0xffffffffu, s, 2, 4);
-        s += __shfl_down_sync(0xffffffffu, s, 1, 4);
-        if (part == 0 && c <= i) {
-            const T rhs = (c == i) ? T(1) : T(0);
-            sInv[i + c * LDD] = unit ? (rhs - s) : (rhs - s) / sD[i + i * LDD];
-        }
-        __syncthreads();
-    }
-    // compact columns 1..63 from stride LDD to stride IB (ascending: each
-    // destination range starts before its source range, ranges of one column
-    // do not overlap earlier compacted columns)
-    for (int col = 1; col < IB; ++col) {
-        T v = T(0);
-        if (tid < IB) v = sInv[tid + col * LDD];
-        __syncthreads();
-        if (tid < IB) sInv[tid + col * IB] = v;
-        __syncthreads();
-    }
-}
-
-// Copy an IB x IB lower inverse from shared (ld IB) to global (ld IB).
-template <class T>
-__device__ __forceinline__ void store_inv(T *g, const T *sInv) {
-    for (int idx = threadIdx.x; idx < IB * IB; idx += NT_CTA) g[idx] = sInv[idx];
 }
 
 // ---------------------------------------------------------------------------

@@ -151,7 +151,8 @@ std::vector<Task> build_order(const Shape &s) {
                          : cal.upd * SUBB * SUBB * nb * 2.0 * (cnt + cal.upd_fix) / (1.0 + cal.upd_fix);
     };
     auto c_strsm = [&](double t, double w, int parts) {
-        return f64 ? 8.0 * t / IB + us * t * (t + IB) / 2 * std::min(w, 64.0)
+        return f64 ? (xinv ? 5.0 + us * SOLB * 0.75 * t * std::min(w, 64.0)
+                           : 8.0 * t / IB + us * t * (t + IB) / 2 * std::min(w, 64.0))
                    : lat ? 13.0 + 0.01 * t : cal.strsm * 3.0 * t * t * w / parts;
     };
     auto c_supd = [&](double t, double w) {
@@ -384,7 +385,7 @@ ExecWs g_ws;   // workspace of the synchronous API entry points
 // Grow-only workspace buffers, stream-ordered (no device-wide synchronization).
 int ensure_ws(ExecWs &w, size_t ctr_bytes, size_t inv_bytes) {
     if (!w.st) {
-        if (!(w.st = (ExecState *)dev_alloc(sizeof(ExecState)))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+        if (!(w.st = (ExecState *)dev_alloc(2 * sizeof(ExecState)))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
         CHB_CUDA(cudaEventCreate(&w.e0));
         CHB_CUDA(cudaEventCreate(&w.e1));
     }
@@ -465,20 +466,126 @@ static int group_f64(int N, int NB, int kgroup) {
     return std::max(1, depth / NB);
 }
 
-int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B, cudaStream_t s,
-                     ExecResult *res, int split, ExecWs *wsp, int grid_req, int flags, const CastIn *cin) {
+// FP64 substitutions.  The forward and backward sweeps are a chain of 2 N / NB
+// dependent steps of a few microseconds each, so they run on tiles as large as
+// the storage and the inverses allow (SOLVE_NB), each step one product per
+// 64-row block with the tile's full inverse, and on column blocks of SOLVE_NBB
+// whose chains run side by side.  The inverses come from products over all
+// tiles at once (xinv_launch) before the chain starts, on the whole chip.
+// Order 8192, 64 right-hand sides: 6.7 ms on the factor's tiles of 512 with
+// inverted 64-blocks, 5.0 ms on tiles of 128.
+constexpr int SOLVE_NB = 512, SOLVE_NBB = 32;
+
+// Tile size of the substitutions, 0 when the storage allows none from 64 on.
+static int solve_tile(const CHAM_desc_t *A, const CHAM_desc_t *B) {
+    if (one_tile(A) && one_tile(B)) return std::min(SOLVE_NB, (A->n + IB - 1) / IB * IB);
+    const int nb = one_tile(A) ? B->mb : A->nb;
+    for (int d = std::min(SOLVE_NB, nb); d >= IB; --d)
+        if (nb % d == 0) return d;
+    return 0;
+}
+
+// The diagonal tiles (order <= NB, NT of them) of a factor, as lower views.
+struct DiagTiles {
+    double *A;
+    const int64_t *off;
+    const int *ld;
+    int nt, r, NB, N, upper;
+    __device__ int order(int k) const { return min(NB, N - k * NB); }
+    __device__ View L(int k) const {
+        const int K = k / r, i = k - K * r;
+        const int64_t l = ld[K];
+        double *q = A + off[K + nt * K] + (int64_t)i * NB * (1 + l);
+        return upper ? View{q, l, 1} : View{q, 1, l};
+    }
+};
+
+// X(k) (ld NB, NB^2 apart) gets the inverted 64 x 64 diagonal blocks of tile k.
+__global__ void __launch_bounds__(NT_CTA, 2) xinv_diag_kernel(DiagTiles d, double *X) {
+    extern __shared__ __align__(128) double smem[];
+    const int k = blockIdx.y, j0 = blockIdx.x * IB, n = min(IB, d.order(k) - j0);
+    if (n <= 0) return;
+    double *sX = smem + IB * LEAF_LD;
+    rec::leaf64_load(d.L(k).sub(j0, j0), n, smem);
+    rec::leaf64_core<double, false>(smem, sX, n);
+    double *q = X + (int64_t)k * d.NB * d.NB + (int64_t)j0 * (d.NB + 1);
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < n * IB; idx += NT_CTA) {
+        const int r = idx & (IB - 1), c = idx / IB;
+        if (r < n) q[r + (int64_t)c * d.NB] = sX[r + c * LEAF_LD];
+    }
+}
+// One doubling half-step on every tile: the pairs of h-blocks of the tile get
+// W21 = L21 X11 (first) or X21 = -X22 W21; 64 x 64 output blocks.
+__global__ void __launch_bounds__(NT_CTA, 2) xinv_pair_kernel(DiagTiles d, int h, int pairs, double *X, double *W,
+                                                              int first) {
+    extern __shared__ __align__(128) double smem[];
+    const int k = blockIdx.z / pairs, q = blockIdx.z % pairs, n = d.order(k);
+    const int r = h * (2 * q + 1), c = r - h, h2 = min(h, n - r);
+    const int i0 = blockIdx.x * IB, j0 = blockIdx.y * IB;
+    if (i0 >= h2) return;
+    const int rows = min(IB, h2 - i0);
+    const int64_t base = (int64_t)k * d.NB * d.NB;
+    const View Xv{X + base, 1, d.NB}, Wv{W + base, 1, d.NB};
+    Acc<GemmCfg<double, 64, 64, 2, 4, SPLIT_BF16X3, 3>> acc;
+    acc.zero();
+    if (first) {
+        cta_gemm(acc, d.L(k).sub(r + i0, c + j0), Xv.sub(c + j0, c + j0).t(), rows, IB, h - j0, smem);
+        acc.store_to(Wv.sub(r + i0, c + j0), rows, IB);
+    } else {
+        cta_gemm(acc, Xv.sub(r + i0, r), Wv.sub(r, c + j0).t(), rows, IB, i0 + rows, smem);
+        acc.for_each([&](int i, int j, double v) {
+            if (i < rows) *Xv.at(r + i0 + i, c + j0 + j) = -v;
+        });
+    }
+}
+
+// The full inverses of all diagonal tiles into X (W: scratch of the same size).
+static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, cudaStream_t s) {
+    constexpr size_t inv_smem = sizeof(double) * 2 * IB * LEAF_LD;
+    constexpr size_t pair_smem = GemmCfg<double, 64, 64, 2, 4, SPLIT_BF16X3, 3>::SMEM_BYTES;
+    static bool attr = false;
+    if (!attr) {
+        CHB_CUDA(cudaFuncSetAttribute(xinv_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem));
+        CHB_CUDA(cudaFuncSetAttribute(xinv_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem));
+        attr = true;
+    }
+    xinv_diag_kernel<<<dim3((d.NB + IB - 1) / IB, NT), NT_CTA, inv_smem, s>>>(d, X);
+    CHB_LAUNCHED(1);
+    for (int h = IB; h < d.NB; h *= 2) {
+        const int pairs = (d.NB + h - 1) / (2 * h), nb = h / IB;
+        for (int first = 1; first >= 0; --first)
+            xinv_pair_kernel<<<dim3(nb, nb, NT * pairs), NT_CTA, pair_smem, s>>>(d, h, pairs, X, W, first);
+        CHB_LAUNCHED(2);
+    }
+    CHB_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// Enqueue one launch of the executor (mode: factorization, substitutions or
+// both).  xnb > 0 (FP64 substitutions): tiles of xnb with their full inverses.
+// st: its state, initialized by the caller; after: state of an earlier launch
+// that must not have failed.  *xinv_made: the launch computes the FP32 tile
+// inverses of this factor.
+static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B, cudaStream_t s, int split,
+                       ExecWs &w, int grid_req, int flags, const CastIn *cin, int xnb, ExecState *st,
+                       const ExecState *after, bool *xinv_made, int *ntasks) {
     Context &c = ctx();
-    ExecWs &w = wsp ? *wsp : g_ws;
     const int N = A->n;
-    const int NB = (t_given || A->dtyp == ChamRealFloat) ? A->nb : exec_tile(A, (mode & MODE_SOLVE) ? B : nullptr);
+    const bool f32 = (A->dtyp == ChamRealFloat);
+    const int NB = xnb > 0 ? xnb : (t_given || f32) ? A->nb : exec_tile(A, (mode & MODE_SOLVE) ? B : nullptr);
     const int NT = (N + NB - 1) / NB;
     const int nrhs = (B && (mode & MODE_SOLVE)) ? B->n : 0;
-    const int NBB = B ? B->nb : NB;
-    const int NTB = nrhs ? B->nt : 0;
-    const bool f32 = (A->dtyp == ChamRealFloat);
-    res->info = 0; res->error = 0; res->ms = 0.f;
-    if (N == 0) return 0;
-    if (nrhs && B->dtyp != A->dtyp) return CHAMELEON_ERR_ILLEGAL_VALUE;
+    int NBB = B ? B->nb : NB, NTB = nrhs ? B->nt : 0, b_c = 1;
+    if (xnb > 0) {
+        const bool one_col = priv(B)->cm_view || B->nt == 1;
+        const int want = nrhs <= 1024 ? SOLVE_NBB : 2 * SOLVE_NBB;
+        if (one_col || B->nb % want == 0) {
+            b_c = one_col ? (nrhs + want - 1) / want : B->nb / want;
+            NBB = want;
+            NTB = (nrhs + want - 1) / want;
+        }
+    }
     if (cin) {
         if (!f32 || !(mode & MODE_FACT)) return CHAMELEON_ERR_ILLEGAL_VALUE;
         mode |= MODE_CAST;
@@ -497,9 +604,10 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     // FP32 substitutions with full diagonal-tile inverses: computed off the
     // critical path in a factor+solve launch, reused by later solve-only
     // launches on the same factor and workspace (flags & EXEC_REUSE_INV).
-    const bool xinv = f32 && !full_inv && c.xinv_solve && (mode & MODE_SOLVE) && nrhs > 0 &&
-                      NB <= (64 << rec::MAX_LVL);
-    if (xinv) {
+    const bool xinv = xnb > 0 || (f32 && !full_inv && c.xinv_solve && (mode & MODE_SOLVE) && nrhs > 0 &&
+                                  NB <= (64 << rec::MAX_LVL));
+    if (xnb > 0) mode |= MODE_XINV | MODE_NOINV;
+    else if (xinv) {
         mode |= MODE_XINV;
         if (!(mode & MODE_FACT) && (flags & EXEC_REUSE_INV) && w.xinv_owner == A->mat && w.xinv_nt == NT &&
             w.xinv_nb == NB && w.xinv_n == N)
@@ -529,8 +637,9 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     const size_t nctr = (size_t)(cin ? 3 : 2) * NT * NT + (size_t)4 * NT * std::max(NTB, 1) + NT;
     const size_t esz = f32 ? sizeof(float) : sizeof(double);
     const size_t inv_elems = full_inv ? (size_t)NT * NB * NB : (size_t)NT * NIB * IB * IB;
-    rc = ensure_ws(w, nctr * sizeof(int), inv_elems * esz);
+    rc = ensure_ws(w, nctr * sizeof(int), xnb > 0 ? 0 : inv_elems * esz);
     if (rc) return rc;
+    if (!st) st = w.st;
     int rcA = desc_upload(A);
     if (rcA) return rcA;
     if (nrhs) {
@@ -559,6 +668,7 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     p.b_ld = nrhs ? priv(B)->dev.ld : nullptr;
     p.b_nt = nrhs ? B->mt : 1;
     p.b_r = nrhs ? (one_tile(B) ? NT : std::max(1, B->mb / NB)) : 1;
+    p.b_c = b_c;
     int *ctr = (int *)w.ctr;
     p.updA = ctr;
     p.panA = ctr + (size_t)NT * NT;
@@ -582,7 +692,7 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     }
     p.xinv = nullptr;
     if (xinv) {
-        const size_t xbytes = (size_t)NT * NB * NB * sizeof(float);
+        const size_t xelems = (size_t)NT * NB * NB, xbytes = xelems * (f32 ? sizeof(float) : 2 * sizeof(double));
         if (xbytes > w.xinv_bytes) {
             dev_free(w.xinv);
             w.xinv_bytes = 0;
@@ -591,9 +701,13 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
             w.xinv_bytes = xbytes;
         }
         p.xinv = w.xinv;
-        if (!(mode & MODE_NOINV)) w.xinv_owner = nullptr;   // rewritten by this launch
+        if (xnb > 0 || !(mode & MODE_NOINV)) w.xinv_owner = nullptr;   // rewritten by this call
+        if (xnb > 0) {
+            const DiagTiles d{(double *)A->mat, priv(A)->dev.off, priv(A)->dev.ld, p.a_nt, p.a_r, NB, N, p.upper};
+            if ((rc = xinv_launch(d, NT, (double *)w.xinv, (double *)w.xinv + xelems, s))) return rc;
+        }
         // forward-substitution results, same tile layout as B
-        const size_t ybytes = (size_t)(priv(B)->cm_view ? B->lda : B->lm) * B->ln * sizeof(float);
+        const size_t ybytes = (size_t)(priv(B)->cm_view ? B->lda : B->lm) * B->ln * esz;
         if (ybytes > w.y_bytes) {
             dev_free(w.y);
             w.y_bytes = 0;
@@ -602,7 +716,8 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
         }
         p.Y = w.y;
     }
-    p.st = w.st;
+    p.st = st;
+    p.after = after;
     p.trace = (g_trace_buf && g_trace_cap >= p.ntasks) ? g_trace_buf : nullptr;
     p.wait_budget_ns = (unsigned long long)c.wait_budget_us * 1000ull;
     p.kgroup = G;
@@ -620,12 +735,7 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
         }
         p.split = w.split;
     }
-    ExecState init{};
-    init.info = INT_MAX;
-    init.stuck_task = -1;
     CHB_CUDA(cudaMemsetAsync(ctr, 0, nctr * sizeof(int), s));
-    CHB_CUDA(cudaMemcpyAsync(w.st, &init, sizeof(init), cudaMemcpyHostToDevice, s));
-    CHB_CUDA(cudaEventRecord(w.e0, s));
     if (p.ntasks > 0) {
         CHB_LAUNCHED(1);
         if (!f32) rc = launch_dag_f64(p, grid, s);
@@ -634,25 +744,142 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
         else rc = launch_dag_f32(p, grid, s);
         if (rc) return rc;
     }
+    *xinv_made = f32 && xinv && !(mode & MODE_NOINV);
+    *ntasks = p.ntasks;
+    return 0;
+}
+
+int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B, cudaStream_t s,
+                     ExecResult *res, int split, ExecWs *wsp, int grid_req, int flags, const CastIn *cin) {
+    ExecWs &w = wsp ? *wsp : g_ws;
+    const int N = A->n;
+    const bool f32 = (A->dtyp == ChamRealFloat);
+    const int nrhs = (B && (mode & MODE_SOLVE)) ? B->n : 0;
+    res->info = 0; res->error = 0; res->ms = 0.f;
+    if (N == 0) return 0;
+    if (nrhs && B->dtyp != A->dtyp) return CHAMELEON_ERR_ILLEGAL_VALUE;
+    int rc = ensure_ws(w, 0, 0);
+    if (rc) return rc;
+    ExecState init[2] = {};
+    init[0].info = init[1].info = INT_MAX;
+    init[0].stuck_task = init[1].stuck_task = -1;
+    CHB_CUDA(cudaMemcpyAsync(w.st, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    CHB_CUDA(cudaEventRecord(w.e0, s));
+    // FP64 substitutions above one executor tile: a launch of their own, after
+    // the factorization's (which it checks on the device).  With a
+    // factorization of a small matrix they stay in its launch, where the
+    // forward sweep runs beside it (dposv 203: 232 us in one launch, 256 in
+    // two; 2048: 1.70 and 1.73 ms; 5003: 6.16 and 5.95 ms).
+    const bool own = (mode & MODE_FACT) ? N > 3072 : N > EXEC_NB;
+    const int xnb = (!f32 && !t_given && nrhs > 0 && own) ? solve_tile(A, B) : 0;
+    bool xinv_made = false;
+    int ntasks[2] = {0, 0};
+    if (xnb > 0) {
+        if (mode & MODE_FACT)
+            rc = enqueue_dag(MODE_FACT, uplo, A, nullptr, s, split, w, grid_req, flags, nullptr, 0, w.st, nullptr,
+                             &xinv_made, &ntasks[0]);
+        if (!rc)
+            rc = enqueue_dag(MODE_SOLVE, uplo, A, B, s, split, w, grid_req, flags, nullptr, xnb, w.st + 1, w.st,
+                             &xinv_made, &ntasks[1]);
+    } else {
+        rc = enqueue_dag(mode, uplo, A, B, s, split, w, grid_req, flags, cin, 0, w.st, nullptr, &xinv_made, &ntasks[0]);
+    }
+    if (rc) return rc;
     CHB_CUDA(cudaEventRecord(w.e1, s));
-    ExecState out{};
-    CHB_CUDA(cudaMemcpyAsync(&out, w.st, sizeof(out), cudaMemcpyDeviceToHost, s));
+    ExecState out[2] = {};
+    CHB_CUDA(cudaMemcpyAsync(out, w.st, sizeof(out), cudaMemcpyDeviceToHost, s));
     CHB_CUDA(cudaStreamSynchronize(s));
     CHB_CUDA(cudaEventElapsedTime(&res->ms, w.e0, w.e1));
-    res->info = (out.info == INT_MAX) ? 0 : out.info;
-    res->error = out.error;
-    if (xinv && !(mode & MODE_NOINV) && res->info == 0 && res->error == 0) {
+    res->info = (out[0].info == INT_MAX) ? 0 : out[0].info;
+    res->error = out[0].error ? out[0].error : out[1].error;
+    if (xinv_made && res->info == 0 && res->error == 0) {
         w.xinv_owner = A->mat;   // the inverses now match this factor
         w.xinv_n = N;
-        w.xinv_nt = NT;
-        w.xinv_nb = NB;
+        w.xinv_nt = A->nt;
+        w.xinv_nb = A->nb;
     }
-    if (out.error) {
-        char msg[160];
-        snprintf(msg, sizeof msg, "device wait budget exhausted at task %d (%d of %d done)",
-                 out.stuck_task, out.done, p.ntasks);
-        warning("run_cholesky_dag", msg);
+    for (int i = 0; i < 2; ++i)
+        if (out[i].error) {
+            char msg[160];
+            snprintf(msg, sizeof msg, "device wait budget exhausted at task %d (%d of %d done)", out[i].stuck_task,
+                     out[i].done, ntasks[i]);
+            warning("run_cholesky_dag", msg);
+        }
+    return 0;
+}
+
+// Counters, state and the one-entry tile table of dag_potrf_async.
+struct OneTile {
+    int64_t off;
+    int ld, pad;
+};
+__global__ void dag_init_kernel(OneTile *tab, int lda, int *ctr, int nctr, ExecState *st) {
+    for (int i = threadIdx.x; i < nctr; i += blockDim.x) ctr[i] = 0;
+    if (threadIdx.x == 0) {
+        *tab = OneTile{0, lda, 0};
+        *st = ExecState{};
+        st->info = INT_MAX;
+        st->stuck_task = -1;
     }
+}
+__global__ void dag_info_kernel(const ExecState *st, int *info) {
+    *info = st->error ? st->error : (st->info == INT_MAX ? 0 : st->info);
+}
+
+int dag_potrf_async(cham_uplo_t uplo, int n, double *A, int lda, int *d_info, cudaStream_t s, ExecWs &w, bool *ran) {
+    *ran = false;
+    const int NB = EXEC_NB, NT = (n + NB - 1) / NB, mode = MODE_FACT | MODE_FINE;
+    int dev = 0, sms = 0;
+    CHB_CUDA(cudaGetDevice(&dev));
+    CHB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // as many CTAs as the first step has panel-solve and update blocks
+    const int grid = std::min(2 * sms, 2 * NT * NT);
+    const int canon = (NT - 1) * NB + (n - (NT - 1) * NB + FINEB - 1) / FINEB * FINEB;
+    const int G = group_f64(n, NB, ctx().kgroup_f64);
+    const Shape sh{mode, canon, NB, 0, NB, grid, PROF_FP64, G, 0, upd_tail(PROF_FP64)};
+    const size_t nctr = (size_t)2 * NT * NT + (size_t)5 * NT;
+    const size_t ctr_bytes = sizeof(OneTile) + nctr * sizeof(int);
+    const size_t inv_bytes = (size_t)NT * (NB / IB) * IB * IB * sizeof(double);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CHB_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        std::lock_guard<std::mutex> lk(g_sched_mu);
+        if (g_sched.find(sh) == g_sched.end() || !w.st || ctr_bytes > w.ctr_bytes || inv_bytes > w.inv_bytes) return 0;
+    } else if (w.st && (ctr_bytes > w.ctr_bytes || inv_bytes > w.inv_bytes)) {
+        CHB_CUDA(cudaStreamSynchronize(s));   // queued calls still use the buffers that are replaced
+    }
+    const Schedule *sch = get_schedule(sh);
+    if (!sch) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+    if (int rc = ensure_ws(w, ctr_bytes, inv_bytes)) return rc;
+    OneTile *tab = (OneTile *)w.ctr;
+    int *ctr = (int *)(tab + 1);
+    dag_init_kernel<<<1, 256, 0, s>>>(tab, lda, ctr, (int)nctr, w.st);
+    ExecParams p{};
+    p.tasks = sch->d_tasks;
+    p.ntasks = (int)sch->tasks.size();
+    p.mode = mode;
+    p.upper = (uplo == ChamUpper);
+    p.NT = NT; p.N = n; p.NB = NB;
+    p.A = A;
+    p.a_off = &tab->off;
+    p.a_ld = &tab->ld;
+    p.a_nt = 1;
+    p.a_r = NT;
+    p.NBB = NB;
+    p.b_r = p.b_nt = 1;
+    p.updA = ctr;
+    p.panA = ctr + (size_t)NT * NT;
+    p.invd = w.inv;
+    p.NIB = NB / IB;
+    p.st = w.st;
+    p.wait_budget_ns = (unsigned long long)ctx().wait_budget_us * 1000ull;
+    p.kgroup = G;
+    p.utail = sh.tail;
+    if (int rc = launch_dag_f64(p, grid, s)) return rc;
+    if (d_info) dag_info_kernel<<<1, 1, 0, s>>>(w.st, d_info);
+    CHB_LAUNCHED(d_info ? 3 : 2);
+    CHB_CUDA(cudaGetLastError());
+    *ran = true;
     return 0;
 }
 

@@ -150,17 +150,19 @@ struct ExecParams {
     void *B;
     const int64_t *b_off;   // b_off[M + b_nt*bn]
     const int *b_ld;
-    int b_nt, b_r;
+    int b_nt, b_r, b_c;     // b_c: column blocks of NBB per storage tile (1 unless FP64 MODE_XINV)
     int *updA, *panA, *fwdB, *fwdDone, *bwdB, *bwdDone;
     void *invd;             // full_inv: NT inverted NB x NB diagonal tiles (ld NB);
                             // else NT * NIB inverted IB x IB blocks (element type of A)
     int NIB;
     int full_inv;           // FP32 path: recursive tile factorization with full tile inverses
-    void *xinv;             // MODE_XINV: NT full inverses of the diagonal tiles (ld NB)
+    void *xinv;             // MODE_XINV: NT full inverses of the diagonal tiles (ld NB; FP64: only
+                            // the lower triangle of 64-blocks is set)
     void *Y;                // MODE_XINV: forward results (layout of B): the substitutions
                             // read B and write Y (forward), read Y and write B (backward)
     int *xinvDone;          // MODE_XINV: TK_XINV(k) done
     ExecState *st;
+    const ExecState *after;     // state of an earlier launch: do nothing when that one failed (or null)
     TraceRec *trace;        // optional per-task trace (nullptr: off)
     // tcgen05 trailing update of the FP32 factorization (split-BF16 operands):
     // split chunks of panel tile (m,k), m > k, at split + (m(m-1)/2 + k) * tile_split_bytes

@@ -60,9 +60,11 @@ struct Dims {
     __device__ ViewT<T> btile(void *B, int m, int bn) const {
         if constexpr (sizeof(T) == 4)
             return ViewT<T>{static_cast<T *>(B) + p.b_off[m + p.b_nt * bn], 1, p.b_ld[m]};
-        const int M = m / p.b_r;
-        return ViewT<T>{static_cast<T *>(B) + p.b_off[M + p.b_nt * bn] + (int64_t)(m - M * p.b_r) * p.NB, 1,
-                        p.b_ld[M]};
+        const int M = m / p.b_r, C = bn / p.b_c;
+        const int64_t ld = p.b_ld[M];
+        return ViewT<T>{static_cast<T *>(B) + p.b_off[M + p.b_nt * C] + (int64_t)(m - M * p.b_r) * p.NB +
+                            (int64_t)(bn - C * p.b_c) * p.NBB * ld,
+                        1, ld};
     }
     __device__ ViewT<T> Bt(int m, int bn) const { return btile(p.B, m, bn); }
     // Tile (m, bn) of the forward results (MODE_XINV), layout of B.
@@ -270,6 +272,28 @@ struct Ahead {
     Task t;
 };
 
+// A substitution product of 64 rows and w <= 64 columns: f(accumulator) on the
+// narrowest tile.  FP64 pipelines as deep as the launch's shared memory allows
+// (the products are short and wait for L2: order 8192, 64 right-hand sides,
+// two stages 15 us per 64 x 64 x 128 product, 4 us of it on the tensor cores).
+template <class T, int SP, class F>
+__device__ __forceinline__ void solve_cols(int w, F &&f) {
+    if constexpr (sizeof(T) == 8) {
+        if (w <= 8) {
+            Acc<GemmCfg<T, 64, 8, 8, 1, SP, 5>> acc;
+            f(acc);
+            return;
+        }
+        if (w <= 32) {
+            Acc<GemmCfg<T, 64, 32, 4, 2, SP, 4>> acc;
+            f(acc);
+            return;
+        }
+    }
+    Acc<GemmCfg<T, 64, 64, 2, 4, SP, sizeof(T) == 8 ? 3 : 2>> acc;
+    f(acc);
+}
+
 template <class T, int SP, bool TC>
 __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T *smem, tc05::Smem *tsm,
                          uint8_t *stage, unsigned *ph, Ahead *ah) {
@@ -439,28 +463,27 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
     case TK_BWD_TRSM: {
         const VT X = d.Bt(t.k, t.bn);
         const int w = d.wB(t.bn);
-        if constexpr (std::is_same<T, float>::value) {
-            if (p.mode & MODE_XINV) {
-                // row block t.sub (SOLB rows) of the tile: forward Y_k = X_k B_k,
-                // backward B_k = X_k^T Y_k
-                const int r0 = t.sub * SOLB, n = d.tm(t.k);
-                const int mr = min(SOLB, n - r0);
-                const VT Xk = d.XI(t.k);
-                const VT Yk = d.Yt(t.k, t.bn);
-                for (int c0 = 0; c0 < w; c0 += 64) {
-                    const int wc = min(64, w - c0);
-                    Acc<Cfg64<T, SP>> acc;
-                    acc.zero();
-                    if (t.kind == TK_FWD_TRSM) {
-                        cta_gemm(acc, Xk.sub(r0, 0), X.sub(0, c0).t(), mr, wc, r0 + mr, smem);
-                        acc.store_to(Yk.sub(r0, c0), mr, wc);
-                    } else {
-                        cta_gemm(acc, Xk.sub(r0, r0).t(), Yk.sub(r0, c0).t(), mr, wc, n - r0, smem);
-                        acc.store_to(X.sub(r0, c0), mr, wc);
-                    }
+        if (p.mode & MODE_XINV) {
+            // row block t.sub (SOLB rows) of the tile: forward Y_k = X_k B_k,
+            // backward B_k = X_k^T Y_k
+            const int r0 = t.sub * SOLB, n = d.tm(t.k);
+            const int mr = min(SOLB, n - r0);
+            const VT Xk = d.XI(t.k);
+            const VT Yk = d.Yt(t.k, t.bn);
+            auto apply = [&](auto &acc, int c0, int wc) {
+                acc.zero();
+                if (t.kind == TK_FWD_TRSM) {
+                    cta_gemm(acc, Xk.sub(r0, 0), X.sub(0, c0).t(), mr, wc, r0 + mr, smem);
+                    acc.store_to(Yk.sub(r0, c0), mr, wc);
+                } else {
+                    cta_gemm(acc, Xk.sub(r0, r0).t(), Yk.sub(r0, c0).t(), mr, wc, n - r0, smem);
+                    acc.store_to(X.sub(r0, c0), mr, wc);
                 }
-                break;
-            }
+            };
+            for (int c0 = 0; c0 < w; c0 += 64) solve_cols<T, SP>(min(64, w - c0), [&](auto &acc) { apply(acc, c0, min(64, w - c0)); });
+            break;
+        }
+        if constexpr (std::is_same<T, float>::value) {
             if (p.full_inv) {
                 const VT Xk = d.X(t.k);
                 if (t.kind == TK_FWD_TRSM) rec::apply_inv_left<T, SP, false>(X, w, Xk, d.tm(t.k), smem);
@@ -493,16 +516,12 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
         const VT L = (t.kind == TK_FWD_UPD) ? d.A(t.m, t.k).sub(r0, 0) : d.A(t.k, t.m).t().sub(r0, 0);
         for (int c0 = 0; c0 < w; c0 += 64) {
             const int wc = min(64, w - c0);
-            if (rows <= SOLB && wc <= Cfg64N<T, SP>::BN && sizeof(T) == 8) {   // few right-hand sides
-                Acc<Cfg64N<T, SP>> acc;
-                acc.zero();
-                cta_gemm(acc, L, Bk.sub(0, c0).t(), rows, wc, d.tm(t.k), smem);
-                acc.sub_from(Bm.sub(0, c0), rows, wc, false);
-            } else if (rows <= SOLB) {
-                Acc<Cfg64<T, SP>> acc;
-                acc.zero();
-                cta_gemm(acc, L, Bk.sub(0, c0).t(), rows, wc, d.tm(t.k), smem);
-                acc.sub_from(Bm.sub(0, c0), rows, wc, false);
+            if (rows <= SOLB) {
+                solve_cols<T, SP>(wc, [&](auto &acc) {
+                    acc.zero();
+                    cta_gemm(acc, L, Bk.sub(0, c0).t(), rows, wc, d.tm(t.k), smem);
+                    acc.sub_from(Bm.sub(0, c0), rows, wc, false);
+                });
             } else {
                 Acc<Cfg12864<T, SP>> acc;
                 acc.zero();
@@ -554,6 +573,7 @@ __global__ void __launch_bounds__(NT_CTA, dag_ctas_per_sm<T, TC>()) cholesky_dag
     __shared__ tc05::Smem tsm;
     __shared__ unsigned s_ph[3];   // phase cycles of the current task (tracing only)
     const Dims<T> d{p};
+    if (p.after && (p.after->abort || p.after->error)) return;
     if constexpr (TC) tc05::init(&tsm);
     __shared__ Task s_desc;
     uint64_t tg = 0;

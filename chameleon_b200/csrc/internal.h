@@ -216,6 +216,12 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
                      ExecResult *res, int split = 0, ExecWs *ws = nullptr, int grid = 0, int flags = 0,
                      const CastIn *cin = nullptr);
 
+// FP64 Cholesky of a device column-major matrix on the executor, in stream
+// order on s (no synchronization; *d_info, may be null, receives LAPACK's info
+// or an error code).  *ran = false, with nothing launched, when s is being
+// captured and the task list or the workspace w would have to be made first.
+int dag_potrf_async(cham_uplo_t uplo, int n, double *A, int lda, int *d_info, cudaStream_t s, ExecWs &w, bool *ran);
+
 // Tile size of the mixed solver's FP32 factorization for FP64 tile size NB (mixed.cu).
 int factor_tile(int NB);
 

@@ -38,15 +38,16 @@ namespace chb {
 
 static __device__ __align__(256) double g_potrf_scratch[(CHAM_B200_NOALLOC_POTRF_MAXN / IB) * IB * IB];
 
-// The same tile algorithm as CUDA_dpotrf's kernel (blocked left-looking with
-// the 64-wide leaf), so both entry points return the same factor and info.
+// The one-CTA tile algorithm of CUDA_dpotrf (blocked left-looking with the
+// 64-wide leaf).
 __global__ void __launch_bounds__(NT_CTA, 1) potrf_noalloc_kernel(View T, int n, double *invd, int *info) {
     extern __shared__ __align__(128) double smem[];
-    const int r = rec::tile_potrf_blk<double, SPLIT_BF16X3>(T, n, invd, smem);
+    const int r = rec::tile_potrf_fused(T, n, invd, smem);
     if (threadIdx.x == 0 && info) *info = r;
 }
 
 namespace {
+constexpr size_t NOALLOC_SMEM_BYTES = sizeof(double) * rec::fused_smem_elems();
 constexpr int MAX_DEVICES = 64;
 std::mutex g_mu;
 double *g_scratch_addr[MAX_DEVICES] = {};
@@ -67,7 +68,7 @@ int noalloc_setup(int dev, double **addr) {
     }
     if (!g_attr_set[dev]) {
         const cudaError_t e = cudaFuncSetAttribute(potrf_noalloc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)TILE_KERNEL_SMEM_BYTES);
+                                                   (int)NOALLOC_SMEM_BYTES);
         if (e != cudaSuccess) {
             report_cuda_error("cudaFuncSetAttribute(potrf_noalloc_kernel)", e, __FILE__, __LINE__);
             return CHAMELEON_ERR_UNEXPECTED;
@@ -107,7 +108,7 @@ extern "C" int CUDA_dpotrf_noalloc(cham_uplo_t uplo, int n, double *A, int lda, 
     // a launch error left over from unrelated earlier work would otherwise be
     // reported as this launch's failure
     (void)cudaGetLastError();
-    potrf_noalloc_kernel<<<1, NT_CTA, TILE_KERNEL_SMEM_BYTES, s>>>(T, n, scratch, d_info);
+    potrf_noalloc_kernel<<<1, NT_CTA, NOALLOC_SMEM_BYTES, s>>>(T, n, scratch, d_info);
     CHB_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? CHAMELEON_SUCCESS : CHAMELEON_ERR_UNEXPECTED;
 }

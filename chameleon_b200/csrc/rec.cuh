@@ -577,6 +577,70 @@ static __device__ int tile_potrf_fused(const View &Tv, int n, double *invd, doub
     return 0;
 }
 
+// One sweep (forward, or backward with the transpose) of the substitution on a
+// strip of SW columns held in shared memory, X(r, c) at sX[r + c ld], rows n up
+// to the next multiple of 64 zero, with the inverted diagonal blocks invd of
+// the lower L.  The rows of L are used once per strip, so its MMA fragments
+// come straight from L2 into registers, the next ones in flight during the
+// products, and a 64-row step is two products and two barriers without a
+// global round trip of X.  FP32 operands are multiplied in FP64.  sR: SW x
+// LEAF_LD doubles.  All threads; starts and ends with a barrier.
+constexpr int SW = 8;
+__host__ __device__ constexpr int strip_ld(int n) { return (n + IB - 1) / IB * IB + 4; }   // 4 mod 16: no conflicts
+__host__ __device__ constexpr size_t strip_smem_elems(int n) { return (size_t)SW * (strip_ld(n) + LEAF_LD); }
+template <class T>
+__device__ __noinline__ void strip_sweep(const ViewT<T> &L, int n, const T *invd, double *sX, int ld, double *sR,
+                                         bool trans) {
+    sX = in_shared(sX);
+    sR = in_shared(sR);
+    const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const int nblk = (n + IB - 1) / IB, row = 8 * warp + g;   // this lane's row of the 64-row step
+    const int last = ld - 8;   // the strip's last group of four rows
+    __syncthreads();
+    for (int s = 0; s < nblk; ++s) {
+        const int b = trans ? nblk - 1 - s : s, jb = b * IB;
+        const bool live = jb + row < n;
+        // fragments of the inverted diagonal block: independent of the sum below
+        const T *inv = invd + (int64_t)b * IB * IB;
+        T iv[IB / 4];
+#pragma unroll
+        for (int q = 0; q < IB / 4; ++q) iv[q] = trans ? inv[4 * q + t + row * IB] : inv[row + (4 * q + t) * IB];
+        // rows jb .. of the sum over the columns solved so far
+        const int k0 = trans ? jb + IB : 0, k1 = trans ? n : jb;
+        const ViewT<T> Lr = trans ? L.sub(0, jb).t() : L.sub(jb, 0);   // (row, k)
+        const T *lp = Lr.at(live ? row : 0, 0) + (int64_t)t * Lr.cs;
+        const int64_t st = 4 * Lr.cs;
+        double acc[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        constexpr int U = 8;   // fragments of one round: 32 columns
+        auto fetch = [&](T (&a)[U], int k) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) a[u] = (live && k + 4 * u + t < k1) ? lp[(int64_t)(k / 4 + u) * st] : T(0);
+        };
+        T a0[U], a1[U];
+        fetch(a0, k0);
+        for (int k = k0; k < k1; k += 8 * U) {
+            fetch(a1, k + 4 * U);
+#pragma unroll
+            for (int u = 0; u < U; ++u) dmma884(acc[u & 3], (double)a0[u], sX[min(k + 4 * u, last) + t + g * ld]);
+            fetch(a0, k + 8 * U);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                dmma884(acc[u & 3], (double)a1[u], sX[min(k + 4 * (U + u), last) + t + g * ld]);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            sR[row + (2 * t + e) * LEAF_LD] =
+                sX[jb + row + (2 * t + e) * ld] - ((acc[0][e] + acc[1][e]) + (acc[2][e] + acc[3][e]));
+        __syncthreads();
+        double y[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+        for (int q = 0; q < IB / 4; ++q) dmma884(y[q & 1], (double)iv[q], sR[4 * q + t + g * LEAF_LD]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) sX[jb + row + (2 * t + e) * ld] = y[0][e] + y[1][e];
+        __syncthreads();
+    }
+}
+
 // Inverted 64 x 64 diagonal blocks of an existing lower factor (n x n), for
 // the solve-only executor mode.
 template <class T>

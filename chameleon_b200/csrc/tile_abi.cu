@@ -21,6 +21,7 @@ struct cham_b200_handle_s {
     double *ws;          // scratch: inverted diagonal blocks (grown on demand)
     size_t ws_bytes;
     int *flag;           // dlag2s overflow flag (device)
+    chb::ExecWs ews;     // executor workspace of the handle's stream (dpotrf)
 };
 
 namespace chb {
@@ -35,16 +36,25 @@ static int handle_ws(cham_b200_handle_s *h, size_t bytes) {
     return 0;
 }
 
-// C = alpha * sum_k A(i,k) B(j,k) + beta * C over one 128 x 128 block.
-__global__ void __launch_bounds__(NT_CTA, 1) gemm_kernel(View A, View B, View C, int M, int N, int K, double alpha,
-                                                         double beta, int tri /*0 full, 1 lower, 2 upper*/) {
+// C = alpha * sum_k A(i,k) B(j,k) + beta * C over one block of the tile
+// configuration CF.  One tile of a runtime (a few hundred rows) has too few
+// 128-wide blocks for the chip -- 16 at order 512, 67 us each -- so the
+// launcher takes the widest block that still gives every SM work.
+template <int E>
+using CfgTile = typename std::conditional<E == 128, Cfg128<double>,
+                                          typename std::conditional<E == 64, GemmCfg<double, 64, 64, 2, 4, SPLIT_BF16X3, 3>,
+                                                                    GemmCfg<double, 32, 32, 4, 2, SPLIT_BF16X3, 4>>::type>::type;
+template <int E>
+__global__ void __launch_bounds__(NT_CTA, E == 128 ? 1 : 2)
+    gemm_kernel(View A, View B, View C, int M, int N, int K, double alpha, double beta,
+                int tri /*0 full, 1 lower, 2 upper*/) {
     extern __shared__ __align__(128) double smem[];
     const int bi = blockIdx.x, bj = blockIdx.y;
     if (tri == 1 && bj > bi) return;
     if (tri == 2 && bi > bj) return;
-    const int i0 = bi * 128, j0 = bj * 128;
-    const int rows = min(128, M - i0), cols = min(128, N - j0);
-    Acc<Cfg128<double>> acc;
+    const int i0 = bi * E, j0 = bj * E;
+    const int rows = min(E, M - i0), cols = min(E, N - j0);
+    Acc<CfgTile<E>> acc;
     acc.zero();
     cta_gemm(acc, A.sub(i0, 0), B.sub(j0, 0), rows, cols, K, smem);
     const View Cb = C.sub(i0, j0);
@@ -55,6 +65,25 @@ __global__ void __launch_bounds__(NT_CTA, 1) gemm_kernel(View A, View B, View C,
         double *p = Cb.at(r, c);
         *p = (beta == 0.0) ? alpha * v : alpha * v + beta * *p;
     });
+}
+
+template <int E>
+static void launch_gemm(View A, View B, View C, int M, int N, int K, double alpha, double beta, int tri,
+                        cudaStream_t s) {
+    const dim3 grid((M + E - 1) / E, (N + E - 1) / E);
+    gemm_kernel<E><<<grid, NT_CTA, CfgTile<E>::SMEM_BYTES, s>>>(A, B, C, M, N, K, alpha, beta, tri);
+}
+// Block edge: 128 from two blocks per SM on (order 2200: 296 blocks), 64 from
+// one block per SM on, 32 below.
+static void gemm_tile(View A, View B, View C, int M, int N, int K, double alpha, double beta, int tri,
+                      cudaStream_t s) {
+    auto blocks = [&](int64_t e) {
+        const int64_t a = (M + e - 1) / e, b = (N + e - 1) / e;
+        return tri ? a * (a + 1) / 2 : a * b;
+    };
+    if (blocks(128) >= 2 * 148) launch_gemm<128>(A, B, C, M, N, K, alpha, beta, tri, s);
+    else if (blocks(64) >= 148) launch_gemm<64>(A, B, C, M, N, K, alpha, beta, tri, s);
+    else launch_gemm<32>(A, B, C, M, N, K, alpha, beta, tri, s);
 }
 
 __global__ void scale_kernel(View X, int M, int N, double alpha) {
@@ -70,17 +99,46 @@ __global__ void scale_kernel(View X, int M, int N, double alpha) {
 // Invert the IB x IB diagonal blocks of lower-triangular L (n x n) into invd.
 __global__ void __launch_bounds__(NT_CTA, 1) inv_diag_kernel(View L, int n, double *invd, int unit) {
     extern __shared__ __align__(128) double smem[];
-    double *sD = smem;
-    double *sInv = smem + IB * LDD;
+    double *sX = smem + IB * LEAF_LD;
     const int jb = blockIdx.x * IB;
     const int nbk = min(IB, n - jb);
-    for (int idx = threadIdx.x; idx < nbk * nbk; idx += NT_CTA) {
-        const int r = idx % nbk, c = idx / nbk;
-        sD[r + c * LDD] = (r >= c) ? *L.at(jb + r, jb + c) : 0.0;
+    rec::leaf64_load(L.sub(jb, jb), nbk, smem);
+    rec::leaf64_core<double, false>(smem, sX, nbk, unit != 0);
+    double *g = invd + (int64_t)blockIdx.x * IB * IB;
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < IB * IB; idx += NT_CTA) {
+        const int r = idx % IB, c = idx / IB;
+        g[idx] = (r < nbk && c < nbk) ? sX[r + c * LEAF_LD] : 0.0;
+    }
+}
+
+// X <- alpha op(L)^{-1} X on strips of SW columns, one CTA each (strip_sweep).
+// A solve with a tile of order 512 has 64 strips instead of 8 64-column ones.
+// Wide right-hand sides (more than two strips per SM) read L too often this
+// way and keep the 64-column strips of trsm_kernel.  Order 512, 512 columns:
+// 215 us in 64-column strips.
+using rec::SW;
+using rec::strip_ld;
+constexpr int STRIP_MAXN = 3072;
+static size_t strip_smem(int n) { return sizeof(double) * rec::strip_smem_elems(n); }
+
+__global__ void __launch_bounds__(NT_CTA, 1)
+    trsm_strip_kernel(View L, int n, const double *invd, View X, int w, int trans, double alpha) {
+    extern __shared__ __align__(128) double smem[];
+    const int ld = strip_ld(n), np = ld - 4;
+    double *sR = smem + SW * ld;   // right-hand side of one step (ld LEAF_LD)
+    const int c0 = blockIdx.x * SW, wc = min(SW, w - c0);
+    const bool cm = X.rs == 1;
+    for (int idx = threadIdx.x; idx < SW * np; idx += NT_CTA) {
+        const int r = cm ? idx % np : idx / SW, c = cm ? idx / np : idx % SW;
+        smem[r + c * ld] = (r < n && c < wc) ? (alpha == 0.0 ? 0.0 : alpha * *X.at(r, c0 + c)) : 0.0;
     }
     __syncthreads();
-    blk_inv(sD, sInv, nbk, unit != 0);
-    store_inv(invd + (int64_t)blockIdx.x * IB * IB, sInv);
+    rec::strip_sweep(L, n, invd, smem, ld, sR, trans != 0);
+    for (int idx = threadIdx.x; idx < SW * np; idx += NT_CTA) {
+        const int r = cm ? idx % np : idx / SW, c = cm ? idx / np : idx % SW;
+        if (r < n && c < wc) *X.at(r, c0 + c) = smem[r + c * ld];
+    }
 }
 
 // X <- op(L)^{-1} X on column strips of IB.
@@ -93,7 +151,7 @@ __global__ void __launch_bounds__(NT_CTA, 1) trsm_kernel(View L, int n, const do
 
 __global__ void __launch_bounds__(NT_CTA, 1) potrf_kernel(View T, int n, double *invd, int *info) {
     extern __shared__ __align__(128) double smem[];
-    const int r = rec::tile_potrf_blk<double, SPLIT_BF16X3>(T, n, invd, smem);
+    const int r = rec::tile_potrf_fused(T, n, invd, smem);
     if (threadIdx.x == 0 && info) *info = r;
 }
 
@@ -203,17 +261,23 @@ static int ew_grid(int64_t total) {
     return (int)std::min<int64_t>(std::max<int64_t>(b, 1), 148 * 32);
 }
 
+constexpr size_t POTRF_SMEM_BYTES = sizeof(double) * rec::fused_smem_elems();
+constexpr size_t INV_SMEM_BYTES = sizeof(double) * 2 * IB * LEAF_LD;
 static bool smem_attr_done = false;
 static int set_smem_attrs() {
     if (smem_attr_done) return 0;
-    CHB_CUDA(cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg128<double>::SMEM_BYTES));
+    CHB_CUDA(cudaFuncSetAttribute(gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgTile<128>::SMEM_BYTES));
+    CHB_CUDA(cudaFuncSetAttribute(gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgTile<64>::SMEM_BYTES));
+    CHB_CUDA(cudaFuncSetAttribute(gemm_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgTile<32>::SMEM_BYTES));
     CHB_CUDA(cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg64<double>::SMEM_BYTES));
+    CHB_CUDA(cudaFuncSetAttribute(trsm_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)strip_smem(STRIP_MAXN)));
     CHB_CUDA(cudaFuncSetAttribute(potrf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)TILE_KERNEL_SMEM_BYTES));
+                                  (int)POTRF_SMEM_BYTES));
     CHB_CUDA(cudaFuncSetAttribute(spotrf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)SPOTRF_SMEM_BYTES));
     CHB_CUDA(cudaFuncSetAttribute(inv_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * IB * LDD * sizeof(double))));
+                                  (int)INV_SMEM_BYTES));
     smem_attr_done = true;
     return 0;
 }
@@ -242,6 +306,7 @@ int CHAM_B200_Handle_Destroy(cublasHandle_t h) {
     cudaStreamSynchronize(h->stream);
     if (h->ws) cudaFree(h->ws);
     if (h->flag) cudaFree(h->flag);
+    free_exec_ws(h->ews);
     free(h);
     return 0;
 }
@@ -272,8 +337,7 @@ int CUDA_dgemm(cham_trans_t transa, cham_trans_t transb, int m, int n, int k, co
     if (k == 0 || *alpha == 0.0) {
         scale_kernel<<<ew_grid((int64_t)m * n), 256, 0, handle->stream>>>(Cv, m, n, *beta);
     } else {
-        dim3 grid((m + 127) / 128, (n + 127) / 128);
-        gemm_kernel<<<grid, NT_CTA, Cfg128<double>::SMEM_BYTES, handle->stream>>>(Av, Bv, Cv, m, n, k, *alpha, *beta, 0);
+        gemm_tile(Av, Bv, Cv, m, n, k, *alpha, *beta, 0, handle->stream);
     }
     CHB_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? CHAMELEON_SUCCESS : CHAMELEON_ERR_UNEXPECTED;
@@ -289,10 +353,8 @@ int CUDA_dsyrk(cham_uplo_t uplo, cham_trans_t trans, int n, int k, const double 
     if (n == 0) return 0;
     if (int rc = set_smem_attrs()) return rc;
     const View Av = (trans == ChamNoTrans) ? View{const_cast<double *>(A), 1, lda} : View{const_cast<double *>(A), lda, 1};
-    dim3 grid((n + 127) / 128, (n + 127) / 128);
     const View Cv{C, 1, ldc};
-    gemm_kernel<<<grid, NT_CTA, Cfg128<double>::SMEM_BYTES, handle->stream>>>(Av, Av, Cv, n, n, k, (k == 0) ? 0.0 : *alpha,
-                                                                     *beta, uplo == ChamLower ? 1 : 2);
+    gemm_tile(Av, Av, Cv, n, n, k, (k == 0) ? 0.0 : *alpha, *beta, uplo == ChamLower ? 1 : 2, handle->stream);
     CHB_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? CHAMELEON_SUCCESS : CHAMELEON_ERR_UNEXPECTED;
 }
@@ -316,12 +378,18 @@ int CUDA_dtrsm(cham_side_t side, cham_uplo_t uplo, cham_trans_t transa, cham_dia
     const int ns = left ? m : n, w = left ? n : m;
     const int nblk = (ns + IB - 1) / IB;
     if (int rc = handle_ws(handle, (size_t)nblk * IB * IB * sizeof(double))) return rc;
-    if (*alpha != 1.0) scale_kernel<<<ew_grid((int64_t)ns * w), 256, 0, handle->stream>>>(X, ns, w, *alpha);
-    inv_diag_kernel<<<nblk, NT_CTA, 2 * IB * LDD * sizeof(double), handle->stream>>>(L, ns, handle->ws,
-                                                                                     diag == ChamUnit);
-    trsm_kernel<<<(w + IB - 1) / IB, NT_CTA, Cfg64<double>::SMEM_BYTES, handle->stream>>>(L, ns, handle->ws, X, w,
-                                                                                 trans_eff);
-    CHB_LAUNCHED(3);
+    inv_diag_kernel<<<nblk, NT_CTA, INV_SMEM_BYTES, handle->stream>>>(L, ns, handle->ws, diag == ChamUnit);
+    if (ns <= STRIP_MAXN && w <= 2 * 148 * SW) {
+        trsm_strip_kernel<<<(w + SW - 1) / SW, NT_CTA, strip_smem(ns), handle->stream>>>(L, ns, handle->ws, X, w,
+                                                                                       trans_eff, *alpha);
+        CHB_LAUNCHED(2);
+    } else {
+        if (*alpha != 1.0)
+            scale_kernel<<<ew_grid((int64_t)ns * w), 256, 0, handle->stream>>>(X, ns, w, *alpha);
+        trsm_kernel<<<(w + IB - 1) / IB, NT_CTA, Cfg64<double>::SMEM_BYTES, handle->stream>>>(L, ns, handle->ws, X, w,
+                                                                                     trans_eff);
+        CHB_LAUNCHED(3);
+    }
     return cudaGetLastError() == cudaSuccess ? CHAMELEON_SUCCESS : CHAMELEON_ERR_UNEXPECTED;
 }
 
@@ -338,10 +406,18 @@ int CUDA_dpotrf(cham_uplo_t uplo, int n, double *A, int lda, double *WORK, int l
         return 0;
     }
     if (int rc = set_smem_attrs()) return rc;
+    // Above one executor tile the tile DAG runs on many CTAs (order 512: one
+    // CTA 532 us); a stream under capture takes it only when nothing has to be
+    // allocated or uploaded for it.
+    if (n > 128) {
+        bool ran = false;
+        if (int rc = dag_potrf_async(uplo, n, A, lda, d_info, handle->stream, handle->ews, &ran)) return rc;
+        if (ran) return CHAMELEON_SUCCESS;
+    }
     const int nblk = (n + IB - 1) / IB;
     if (int rc = handle_ws(handle, (size_t)nblk * IB * IB * sizeof(double))) return rc;
     const View T = (uplo == ChamLower) ? View{A, 1, lda} : View{A, lda, 1};
-    potrf_kernel<<<1, NT_CTA, TILE_KERNEL_SMEM_BYTES, handle->stream>>>(T, n, handle->ws, d_info);
+    potrf_kernel<<<1, NT_CTA, POTRF_SMEM_BYTES, handle->stream>>>(T, n, handle->ws, d_info);
     CHB_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? CHAMELEON_SUCCESS : CHAMELEON_ERR_UNEXPECTED;
 }
