@@ -16,7 +16,7 @@
 //             rec.cuh on a staged copy of the block)
 //   panel:    L_ib = A_ib X_b^T                      (i > b)
 //   trailing: A_ij -= L_ib L_jb^T                    (i >= j > b)
-// (the panel and trailing products on the tensor cores as 3xTF32)
+// (the panel and trailing products in FP32 FMA from shared memory)
 // Same contract as CORE_spotrf on a lower view (coreblas/compute/core_zpotrf.c
 // :75-81): lower triangle overwritten by L, upper untouched, LAPACK info; the
 // inverted blocks go to invd (IB x IB, ld IB, zero outside the block), as the
@@ -32,10 +32,8 @@ constexpr int MAXN = 256;   // largest tile order
 constexpr int BW = 64;      // block-column width (= IB)
 constexpr int LDI = rec::LDS;   // leading dimension of the staged block and its inverse
 
-// Leading dimension of block column b: its rows rounded up to 32, plus 8
-// (8 mod 32: the tensor-core fragment loads -- 8 consecutive rows at 4
-// columns -- then hit 32 distinct banks; a multiple of 4 keeps the columns
-// 16-byte aligned for the vectorized load and write-back).
+// Leading dimension of block column b: its rows rounded up to 32, plus 8 (a
+// multiple of 4: the columns stay 16-byte aligned for the vector accesses).
 __host__ __device__ constexpr int blk_ld(int n, int b) { return (((n - BW * b) + 31) & ~31) + 8; }
 __host__ __device__ constexpr int blk_off(int n, int b) {
     int o = 0;
@@ -75,78 +73,77 @@ static __device__ __noinline__ int leaf(float *D, int ldd, int nbk, float *sD) {
     return 0;
 }
 
-// acc(i, c) = sum_{k < K} Xm(i, k) Ym(c, k) for rows i < M (M <= 192) and
-// columns c < 64 on the tensor cores: mma.sync m16n8k8 TF32 with each operand
-// split in two TF32 parts and three products (hi*hi + hi*lo + lo*hi, close to
-// FP32 accuracy).  Xm: column-major (ld ldx), Ym(c, k) at Ym[k * ldy + c].
-// Warp w owns rows 48 (w & 3) .. +47 (three 16-row tiles) and columns
-// 32 (w >> 2) .. +31 (four 8-column tiles); rows >= M and k >= K read as
-// zero, so no operand entry outside them is read.
+// acc(i, c) = sum_{k < 64} Xm(i, k) Ym(c, k) for rows i < M (M <= 192) and
+// columns c < 64, in FP32 FMA.  Xm: column-major (ld ldx), Ym(c, k) at
+// Ym[k * ldy + c]; 16-byte aligned columns.  Thread (r = tid % 16, q = tid /
+// 16) owns rows 4 r + 64 i .. + 3 (i < 3) and columns 4 q .. + 3, so that four
+// 16-byte loads feed 48 FMAs.  The products are small and their operands are
+// in shared memory: FMA takes 2 K cycles per 64^3 block, where the tensor-core
+// form (three TF32 products per pair, both operands split on the way) took
+// 12 K.  Rows >= M of the last 64-row group are computed from whatever follows
+// and are not stored.
 struct Frag {
-    float v[3][4][4];   // [row tile][column tile][mma accumulator]
+    float v[3][4][4];   // [row group][column][row]
 };
-static __device__ __forceinline__ void gemm64(Frag &acc, const float *Xm, int ldx, int M, const float *Ym, int ldy,
-                                              int K) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int r0 = 48 * (w & 3), c0 = 32 * (w >> 2);
+static __device__ __forceinline__ void gemm64(Frag &acc, const float *Xm, int ldx, int M, const float *Ym, int ldy) {
+    const float *x = Xm + 4 * (threadIdx.x & 15), *y = Ym + 4 * (threadIdx.x >> 4);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc.v[i][j][e] = 0.f;
-    const int nm = M > r0 ? min(3, (M - r0 + 15) / 16) : 0;   // row tiles with rows < M (warp-uniform)
-    if (nm == 0) return;
-#pragma unroll 1
-    for (int k8 = 0; k8 < K; k8 += 8) {
-        const int ka = k8 + t, kb = k8 + t + 4;
-        const bool va = ka < K, vb = kb < K;
-        // the four column tiles' fragments stay live; each row tile's are
-        // loaded just before its products (fewer live registers)
-        uint32_t bh[4][2], bl[4][2];
+    const int ng = (M + 63) / 64;   // row groups (uniform across the CTA)
+    auto sweep = [&](auto groups) {
+        constexpr int G = decltype(groups)::value;
+#pragma unroll 4
+        for (int k = 0; k < BW; ++k) {
+            const float4 b = *reinterpret_cast<const float4 *>(y + k * ldy);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = c0 + 8 * j + g;
-            split_tf32(va ? Ym[ka * ldy + c] : 0.f, bh[j][0], bl[j][0]);
-            split_tf32(vb ? Ym[kb * ldy + c] : 0.f, bh[j][1], bl[j][1]);
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            if (i < nm) {
-                const int ra = r0 + 16 * i + g, rb = ra + 8;
-                uint32_t ah[4], al[4];
-                split_tf32((va && ra < M) ? Xm[ka * ldx + ra] : 0.f, ah[0], al[0]);
-                split_tf32((va && rb < M) ? Xm[ka * ldx + rb] : 0.f, ah[1], al[1]);
-                split_tf32((vb && ra < M) ? Xm[kb * ldx + ra] : 0.f, ah[2], al[2]);
-                split_tf32((vb && rb < M) ? Xm[kb * ldx + rb] : 0.f, ah[3], al[3]);
+            for (int i = 0; i < G; ++i) {
+                const float4 a = *reinterpret_cast<const float4 *>(x + 64 * i + k * ldx);
+                const float bb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    mma_tf32_1688(acc.v[i][j], al, bh[j]);
-                    mma_tf32_1688(acc.v[i][j], ah, bl[j]);
-                    mma_tf32_1688(acc.v[i][j], ah, bh[j]);
+                    acc.v[i][j][0] = fmaf(a.x, bb[j], acc.v[i][j][0]);
+                    acc.v[i][j][1] = fmaf(a.y, bb[j], acc.v[i][j][1]);
+                    acc.v[i][j][2] = fmaf(a.z, bb[j], acc.v[i][j][2]);
+                    acc.v[i][j][3] = fmaf(a.w, bb[j], acc.v[i][j][3]);
                 }
             }
         }
-    }
+    };
+    if (ng == 1) sweep(std::integral_constant<int, 1>{});
+    else if (ng == 2) sweep(std::integral_constant<int, 2>{});
+    else sweep(std::integral_constant<int, 3>{});
 }
 
-// f(row, column, value) over this thread's accumulators (rows may be >= M:
-// their values are zero and the caller's row guard skips them).
-template <class F>
-static __device__ __forceinline__ void frag_each(const Frag &acc, F &&f) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int r0 = 48 * (w & 3), c0 = 32 * (w >> 2);
+// C(r, c) = acc (SUB: C -= acc) for r < M, c < N (and r >= c when lower), C
+// column-major in shared memory (ld ldc, 16-byte aligned columns): four rows
+// as one 16-byte access where all of them are stored.
+template <bool SUB>
+static __device__ __forceinline__ void frag_store(const Frag &acc, float *C, int ldc, int M, int N, bool lower) {
+    const int r0 = 4 * (threadIdx.x & 15), c0 = 4 * (threadIdx.x >> 4);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int r = r0 + 16 * i + g, c = c0 + 8 * j + 2 * t;
-            f(r, c, acc.v[i][j][0]);
-            f(r, c + 1, acc.v[i][j][1]);
-            f(r + 8, c, acc.v[i][j][2]);
-            f(r + 8, c + 1, acc.v[i][j][3]);
+            const int r = r0 + 64 * i, c = c0 + j;
+            if (r >= M || c >= N) continue;
+            const float(&v)[4] = acc.v[i][j];
+            float *q = C + c * ldc + r;
+            if (r + 3 < M && (!lower || r >= c)) {
+                float4 o = make_float4(v[0], v[1], v[2], v[3]);
+                if (SUB) {
+                    const float4 w = *reinterpret_cast<const float4 *>(q);
+                    o = make_float4(w.x - v[0], w.y - v[1], w.z - v[2], w.w - v[3]);
+                }
+                *reinterpret_cast<float4 *>(q) = o;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (r + e < M && (!lower || r + e >= c)) q[e] = SUB ? q[e] - v[e] : v[e];
+            }
         }
 }
 
@@ -228,11 +225,9 @@ static __device__ __noinline__ int potrf(const ViewF &T, int n, float *invd, flo
         // panel: L_ib = A_ib X_b^T, computed in registers, then stored in place
         {
             Frag acc;
-            gemm64(acc, Sb + BW, ldb, M, Xs, LDI, nbk);   // X_b(c, k) at Xs[k * LDI + c]
+            gemm64(acc, Sb + BW, ldb, M, Xs, LDI);   // X_b(c, k) at Xs[k * LDI + c]
             __syncthreads();
-            frag_each(acc, [&](int r, int c, float v) {
-                if (r < M && c < nbk) Sb[c * ldb + BW + r] = v;
-            });
+            frag_store<false>(acc, Sb + BW, ldb, M, nbk, false);
             __syncthreads();
         }
         lap(1);
@@ -242,10 +237,8 @@ static __device__ __noinline__ int potrf(const ViewF &T, int n, float *invd, flo
             const int ldc = blk_ld(n, cb), Mc = n - BW * cb, wc = min(BW, n - BW * cb);
             Frag acc;
             // rows i >= 64 cb of panel b, against its rows 64 cb .. 64 cb + 63
-            gemm64(acc, Sb + BW * (cb - b), ldb, Mc, Sb + BW * (cb - b), ldb, nbk);
-            frag_each(acc, [&](int r, int c, float v) {
-                if (r < Mc && c < wc && r >= c) Sc[c * ldc + r] -= v;
-            });
+            gemm64(acc, Sb + BW * (cb - b), ldb, Mc, Sb + BW * (cb - b), ldb);
+            frag_store<true>(acc, Sc, ldc, Mc, wc, true);
         }
         __syncthreads();
         lap(2);
