@@ -14,7 +14,8 @@
 //   * lean generic: the same routines with 64-row panels and the leaf blocks
 //     aliased onto the GEMM staging area (74 KB for FP64), 2 or 3 CTAs per SM,
 //     so that the latency-bound leaf of one system overlaps the work of the
-//     systems beside it;
+//     systems beside it; FP64 at 2 CTAs per SM keeps the leaf's inverse on chip
+//     too (109 KB);
 //   * small (n <= 64): the whole system in shared memory -- leaf Cholesky +
 //     inverse, then X = L^-T L^-1 B by two small products over the live
 //     right-hand-side columns -- at 1..3 CTAs per SM.

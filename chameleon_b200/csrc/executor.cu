@@ -97,7 +97,8 @@ std::vector<Task> build_order(const Shape &s) {
     const int NTB = s.nrhs > 0 ? (s.nrhs + s.NBB - 1) / s.NBB : 0;
     auto tm = [&](int m) { return (m == NT - 1) ? s.N - m * s.NB : s.NB; };
     const int cb = count_blk(s.mode);
-    auto nbi = [&](int m) { return (tm(m) + cb - 1) / cb; };                 // panel-solve row blocks
+    const int pb = panel_blk(s.mode);
+    auto nbp = [&](int m) { return (tm(m) + pb - 1) / pb; };                 // panel-solve row blocks
     auto nbu = [&](int m, int cnt) {                                         // update blocks, cnt panels
         const int e = upd_blk(s.mode, cnt);
         return (tm(m) + e - 1) / e;
@@ -143,7 +144,7 @@ std::vector<Task> build_order(const Shape &s) {
     };
     auto c_xinv = [&](double t) { return lat ? 1.5 * t : cal.potrf * 6.0 * t * t * t / 3.0; };
     auto c_trsm = [&]() {
-        return f64 ? 4.0 + us * sub * nb * (nb + IB) / 2 : lat ? 0.27 * nb : cal.trsm * 2.0 * SUBB * nb * nb;
+        return f64 ? 4.0 + us * sub * nb * (nb + IB) / 2 : lat ? (pb < SUBB ? 0.15 : 0.27) * nb : cal.trsm * 2.0 * SUBB * nb * nb;
     };
     auto c_upd = [&](int cnt) {
         return f64 ? 4.0 + us * ub(cnt) * ub(cnt) * nb * cnt
@@ -191,7 +192,7 @@ std::vector<Task> build_order(const Shape &s) {
                 edge(P[k], XI[k]);
             }
             for (int m = k + 1; m < NT; ++m) {
-                const int id = add(TK_TRSM, m, k, k, 0, nbi(m), c_trsm());
+                const int id = add(TK_TRSM, m, k, k, 0, nbp(m), c_trsm());
                 edge(P[k], id);
                 edge(lastU[m + (size_t)NT * k], id);
                 if (k == 0) edge(Cst[m], id);
@@ -562,6 +563,8 @@ static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, cudaStr
     return 0;
 }
 
+constexpr int TC_CHAIN_N = 20480;
+
 // Enqueue one launch of the executor (mode: factorization, substitutions or
 // both).  xnb > 0 (FP64 substitutions): tiles of xnb with their full inverses.
 // st: its state, initialized by the caller; after: state of an earlier launch
@@ -598,9 +601,18 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     // grid_req counts SMs; FP64 places two executor CTAs on each
     const int cps = f32 ? 1 : 2;
     const int grid = cps * ((grid_req > 0) ? std::min(grid_req, c.num_sms) : c.num_sms);
-    if (!f32 && !t_given) mode |= MODE_FINE;
-    const int prof = !f32 ? PROF_FP64 : (tc ? PROF_F32_TC05 : PROF_F32_MMA);
     const bool full_inv = f32 && c.rec_tile && NB <= (64 << rec::MAX_LVL);
+    if (!f32 && !t_given) mode |= MODE_FINE;
+    // The tcgen05 path is bound by the chain of diagonal tiles up to about 80
+    // tiles of 256 and by its updates (L2 operand traffic) beyond: the chain's
+    // panel solves are split in two and the update groups kept short there
+    // (order 16384: 16.9 -> 15.4 ms, 4096: 3.5 -> 3.05), while a chain that
+    // runs further ahead only costs the updates locality at larger orders
+    // (32768: 61 -> 65 ms), where deeper groups save C round trips instead
+    // (8 panels 61.0 ms, 12 panels 59.3).
+    const bool chain_bound = N <= TC_CHAIN_N;
+    if (tc && !full_inv && chain_bound) mode |= MODE_HALF;
+    const int prof = !f32 ? PROF_FP64 : (tc ? PROF_F32_TC05 : PROF_F32_MMA);
     // FP32 substitutions with full diagonal-tile inverses: computed off the
     // critical path in a factor+solve launch, reused by later solve-only
     // launches on the same factor and workspace (flags & EXEC_REUSE_INV).
@@ -618,7 +630,7 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     // takes the exact sizes from the parameters): key the cache on that
     // canonical shape so that callers with many distinct N share schedules.
     // (the finer of the update and substitution row blocks decides)
-    const int gran = std::min(count_blk(mode), solve_rows(mode));
+    const int gran = std::min(panel_blk(mode), solve_rows(mode));
     const int last_sub = ((N - (NT - 1) * NB) + gran - 1) / gran;
     const int canonN = (NT - 1) * NB + std::min(NB, last_sub * gran);
     // nrhs enters the cost model (not the task list): keep it, with the last
@@ -629,7 +641,8 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     // dispatch of an update over G panels (CHAMELEON_B200_UPD_GROUP per path)
     const int G = t_given ? 1
                           : prof == PROF_FP64 ? group_f64(N, NB, c.kgroup_f64)
-                                              : std::max(1, tc ? c.kgroup_tc : c.kgroup_f32);
+                                              : std::max(1, !tc ? c.kgroup_f32
+                                                                : chain_bound ? c.kgroup_tc : c.kgroup_tc + c.kgroup_tc / 2);
     Shape sh{mode, canonN, NB, canonR, NBB, grid, prof, G, cin ? std::max(1, cin->h2d_gbs) : 0, upd_tail(prof)};
     const Schedule *sch = t_given ? t_given : get_schedule(sh);
     if (!sch) return CHAMELEON_ERR_OUT_OF_RESOURCES;

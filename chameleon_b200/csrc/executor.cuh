@@ -84,8 +84,10 @@ static_assert(sizeof(Task) == 16, "Task is 16 bytes");
 // takes 12-25 us on one SM, four 64-wide ones run side by side.  The
 // counters count 64-blocks: an update of several panels, which keeps its
 // 128 x 128 blocks, counts for each 64-block it covers (upd_weight).
+// MODE_HALF (FP32): panel solves alone in 64-row blocks, two side by side for
+// each 128-row block of the tcgen05 updates.
 enum ExecMode : int {
-    MODE_FACT = 1, MODE_SOLVE = 2, MODE_XINV = 4, MODE_NOINV = 8, MODE_CAST = 16, MODE_FINE = 32
+    MODE_FACT = 1, MODE_SOLVE = 2, MODE_XINV = 4, MODE_NOINV = 8, MODE_CAST = 16, MODE_FINE = 32, MODE_HALF = 64
 };
 
 constexpr int SUBB = 128;      // sub-block edge of trailing updates / row blocks
@@ -99,6 +101,7 @@ __host__ __device__ constexpr int solve_rows(int mode) { return (mode & (4 | 32)
 // (cnt panels).
 constexpr int FINEB = 64;
 __host__ __device__ constexpr int count_blk(int mode) { return (mode & 32 /*MODE_FINE*/) ? FINEB : SUBB; }
+__host__ __device__ constexpr int panel_blk(int mode) { return (mode & (32 | 64) /*FINE, HALF*/) ? FINEB : SUBB; }
 __host__ __device__ constexpr int upd_blk(int mode, int cnt) { return cnt == 1 ? count_blk(mode) : SUBB; }
 // Counted blocks of an update task on a rows x cols block (diag: on the
 // diagonal, lower triangle only).

@@ -36,6 +36,11 @@ struct Dims {
         const int e = count_blk(p.mode);
         return (tm(m) + e - 1) / e;
     }
+    // Row blocks of a panel solve of tile row m.
+    __device__ int nbp(int m) const {
+        const int e = panel_blk(p.mode);
+        return (tm(m) + e - 1) / e;
+    }
     __device__ int S(int m, int n) const {
         const int a = nbi(m), b = nbi(n);
         return (m == n) ? a * (a + 1) / 2 : a * b;
@@ -130,8 +135,8 @@ __device__ Deps task_deps(const Task &t, const ExecParams &p, const Dims<T> &d) 
         // the group's last panel being solved implies the earlier ones are
         // (each panel solve waits for the previous panels' updates of its tile)
         const int kl = t.k + t.bn - 1;
-        need(0, &p.panA[t.m + p.NT * kl], d.nbi(t.m));
-        need(1, &p.panA[t.n + p.NT * kl], d.nbi(t.n));
+        need(0, &p.panA[t.m + p.NT * kl], d.nbp(t.m));
+        need(1, &p.panA[t.n + p.NT * kl], d.nbp(t.n));
         need(2, &p.updA[t.m + p.NT * t.n], t.grp * d.S(t.m, t.n));
         // the first update of a tile is its first reader: wait for its cast
         if ((p.mode & MODE_CAST) && t.grp == 0) need(2, &p.castDone[t.m + p.NT * t.n], 1);
@@ -149,7 +154,7 @@ __device__ Deps task_deps(const Task &t, const ExecParams &p, const Dims<T> &d) 
         break;
     case TK_FWD_UPD:
         need(0, &p.fwdDone[t.k + p.NT * t.bn], d.nsolve(t.k));
-        if (fact) need(1, &p.panA[t.m + p.NT * t.k], d.nbi(t.m));
+        if (fact) need(1, &p.panA[t.m + p.NT * t.k], d.nbp(t.m));
         need(2, &p.fwdB[t.m + p.NT * t.bn], t.k * d.nsb(t.m));
         break;
     case TK_BWD_TRSM:
@@ -324,7 +329,7 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
         rec::tile_inv_blk<T>(d.A(t.k, t.k), d.tm(t.k), d.inv(t.k), smem);
         break;
     case TK_TRSM: {
-        const int e = count_blk(p.mode);
+        const int e = panel_blk(p.mode);
         const int r0 = t.sub * e;
         const int rows = min(e, d.tm(t.m) - r0);
         bool done = false;
@@ -334,7 +339,7 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
                 done = true;
             }
         }
-        if constexpr (sizeof(T) == 8) {
+        if (!done) {
             if (rows <= FINEB) {
                 trsm_rows<T, SP, Cfg64<T, SP>>(d.A(t.m, t.k).sub(r0, 0), rows, d.A(t.k, t.k), d.tm(t.k), d.inv(t.k),
                                                smem);
@@ -343,17 +348,19 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
         }
         if (!done) trsm_rows<T, SP>(d.A(t.m, t.k).sub(r0, 0), rows, d.A(t.k, t.k), d.tm(t.k), d.inv(t.k), smem);
         if constexpr (TC) {
-            // emit the split-BF16 chunks of these 128 rows for the tcgen05 updates
+            // emit the split-BF16 chunks of these rows (all or half of a
+            // 128-row chunk) for the tcgen05 updates
             const VT X = d.A(t.m, t.k).sub(r0, 0);
             const int K = d.tm(t.k);
-            uint8_t *base = split_tile(p, t.m, t.k) + (size_t)t.sub * p.split_nkc * 2 * tc05::CHUNK_BYTES;
+            uint8_t *base = split_tile(p, t.m, t.k) + (size_t)(r0 / SUBB) * p.split_nkc * 2 * tc05::CHUNK_BYTES;
+            const int cr = r0 % SUBB;   // first row in the chunk
             // one thread per (row, group of 8 columns): 16-byte stores
-            for (int idx = threadIdx.x; idx < 16 * K; idx += NT_CTA) {
-                const int r = idx % 128, c0 = (idx / 128) * 8;
+            for (int idx = threadIdx.x; idx < e / 8 * K; idx += NT_CTA) {
+                const int r = idx % e, c0 = (idx / e) * 8;
                 float v[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = (r < rows) ? (float)*X.at(r, c0 + e) : 0.f;
-                tc05::split_store8(base + (size_t)(c0 / tc05::BK) * 2 * tc05::CHUNK_BYTES, r, c0 % tc05::BK, v);
+                tc05::split_store8(base + (size_t)(c0 / tc05::BK) * 2 * tc05::CHUNK_BYTES, cr + r, c0 % tc05::BK, v);
             }
             tc05::fence_proxy_async();   // published by the executor's fence + release at task end
             cta_sync();

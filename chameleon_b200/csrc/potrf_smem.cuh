@@ -243,22 +243,23 @@ static __device__ __noinline__ int potrf(const ViewF &T, int n, float *invd, flo
         __syncthreads();
         lap(2);
     }
-    // write back the lower triangle, block column by block column: groups of
-    // four rows entirely below the diagonal as one 16-byte store when the tile
-    // allows it, the rest element by element (the upper triangle is never
-    // written)
-    for (int b = 0; b < nb; ++b) {
-        const int rows = n - BW * b, ld = blk_ld(n, b), nq = ld / 4, wb = min(BW, n - BW * b);
-        const float *Sb = sm + blk_off(n, b);
-        for (int idx = tid; idx < nq * wb; idx += NT_CTA) {
-            const int q = colmajor ? idx % nq : idx / wb, c = colmajor ? idx / nq : idx % wb, r = 4 * q;
-            if (vec && r >= c + 3 && r + 4 <= rows) {
-                *reinterpret_cast<float4 *>(T.at(BW * b + r, BW * b + c)) =
-                    *reinterpret_cast<const float4 *>(Sb + c * ld + r);
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (r + u < rows && r + u >= c) *T.at(BW * b + r + u, BW * b + c) = Sb[c * ld + r + u];
+    // write back the lower triangle, a line of the tile's contiguous direction
+    // per warp and step, so that no index needs a division (the upper triangle
+    // is never written)
+    const int warp = tid >> 5, lane = tid & 31;
+    for (int line = warp; line < n; line += NT_CTA / 32) {
+        if (colmajor) {
+            const int b = line / BW, ld = blk_ld(n, b);
+            const float *q = sm + blk_off(n, b) + (line - BW * b) * ld - BW * b;
+            float *g = T.at(0, line);
+#pragma unroll 4
+            for (int r = (line & ~31) + lane; r < n; r += 32)
+                if (r >= line) g[r] = q[r];
+        } else {
+            float *g = T.at(line, 0);
+            for (int c = lane; c <= line; c += 32) {
+                const int b = c / BW;
+                g[c] = sm[blk_off(n, b) + (c - BW * b) * blk_ld(n, b) + (line - BW * b)];
             }
         }
     }
