@@ -474,7 +474,7 @@ static int group_f64(int N, int NB, int kgroup) {
 // whose chains run side by side.  The inverses come from products over all
 // tiles at once (xinv_launch) before the chain starts, on the whole chip.
 // Order 8192, 64 right-hand sides: 6.7 ms on the factor's tiles of 512 with
-// inverted 64-blocks, 5.0 ms on tiles of 128.
+// inverted 64-blocks, 5.0 ms on tiles of 128, 2.0 ms this way.
 constexpr int SOLVE_NB = 512, SOLVE_NBB = 32;
 
 // Tile size of the substitutions, 0 when the storage allows none from 64 on.

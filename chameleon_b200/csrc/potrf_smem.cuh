@@ -78,9 +78,9 @@ static __device__ __noinline__ int leaf(float *D, int ldd, int nbk, float *sD) {
 // Ym[k * ldy + c]; 16-byte aligned columns.  Thread (r = tid % 16, q = tid /
 // 16) owns rows 4 r + 64 i .. + 3 (i < 3) and columns 4 q .. + 3, so that four
 // 16-byte loads feed 48 FMAs.  The products are small and their operands are
-// in shared memory: FMA takes 2 K cycles per 64^3 block, where the tensor-core
-// form (three TF32 products per pair, both operands split on the way) took
-// 12 K.  Rows >= M of the last 64-row group are computed from whatever follows
+// in shared memory, where the tensor-core form (three TF32 products per pair)
+// spent its time on splitting operands and rounded more: order 256 137 us with
+// it, 112 us with FMA.  Rows >= M of the last 64-row group are computed from whatever follows
 // and are not stored.
 struct Frag {
     float v[3][4][4];   // [row group][column][row]

@@ -38,8 +38,7 @@ static int handle_ws(cham_b200_handle_s *h, size_t bytes) {
 
 // C = alpha * sum_k A(i,k) B(j,k) + beta * C over one block of the tile
 // configuration CF.  One tile of a runtime (a few hundred rows) has too few
-// 128-wide blocks for the chip -- 16 at order 512, 67 us each -- so the
-// launcher takes the widest block that still gives every SM work.
+// 128-wide blocks for the chip (16 at order 512), so the launcher takes the widest block that still gives every SM work.
 template <int E>
 using CfgTile = typename std::conditional<E == 128, Cfg128<double>,
                                           typename std::conditional<E == 64, GemmCfg<double, 64, 64, 2, 4, SPLIT_BF16X3, 3>,
@@ -73,8 +72,8 @@ static void launch_gemm(View A, View B, View C, int M, int N, int K, double alph
     const dim3 grid((M + E - 1) / E, (N + E - 1) / E);
     gemm_kernel<E><<<grid, NT_CTA, CfgTile<E>::SMEM_BYTES, s>>>(A, B, C, M, N, K, alpha, beta, tri);
 }
-// Block edge: 128 from two blocks per SM on (order 2200: 296 blocks), 64 from
-// one block per SM on, 32 below.
+// Block edge: 128 from two blocks per SM on, 64 from one block per SM on, 32
+// below.
 static void gemm_tile(View A, View B, View C, int M, int N, int K, double alpha, double beta, int tri,
                       cudaStream_t s) {
     auto blocks = [&](int64_t e) {
@@ -115,8 +114,9 @@ __global__ void __launch_bounds__(NT_CTA, 1) inv_diag_kernel(View L, int n, doub
 // X <- alpha op(L)^{-1} X on strips of SW columns, one CTA each (strip_sweep).
 // A solve with a tile of order 512 has 64 strips instead of 8 64-column ones.
 // Wide right-hand sides (more than two strips per SM) read L too often this
-// way and keep the 64-column strips of trsm_kernel.  Order 512, 512 columns:
-// 215 us in 64-column strips.
+// way and keep the 64-column strips of trsm_kernel.  With the block edges of
+// gemm_kernel and the executor's dpotrf, one step on tiles of 512 (dpotrf, two
+// dtrsm, two dsyrk, dgemm) went from 1234 to 449 us.
 using rec::SW;
 using rec::strip_ld;
 constexpr int STRIP_MAXN = 3072;
