@@ -383,25 +383,40 @@ Schedule *get_schedule(const Shape &s) {
 
 ExecWs g_ws;   // workspace of the synchronous API entry points
 
-// Grow-only workspace buffers, stream-ordered (no device-wide synchronization).
-int ensure_ws(ExecWs &w, size_t ctr_bytes, size_t inv_bytes) {
+// Bytes of every buffer of a workspace.
+struct WsBytes {
+    size_t ctr = 0, inv = 0, split = 0, xinv = 0, y = 0;
+    void cover(const WsBytes &o) {
+        ctr = std::max(ctr, o.ctr);
+        inv = std::max(inv, o.inv);
+        split = std::max(split, o.split);
+        xinv = std::max(xinv, o.xinv);
+        y = std::max(y, o.y);
+    }
+};
+
+// Grow-only workspace buffers.  A buffer that grows is freed first, and the
+// pool may hand its memory out again at once, so nothing enqueued may still use
+// the workspace: a call reserves what all its launches need before the first.
+int ensure_ws(ExecWs &w, const WsBytes &need) {
     if (!w.st) {
         if (!(w.st = (ExecState *)dev_alloc(2 * sizeof(ExecState)))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
         CHB_CUDA(cudaEventCreate(&w.e0));
         CHB_CUDA(cudaEventCreate(&w.e1));
     }
-    if (ctr_bytes > w.ctr_bytes) {
-        dev_free(w.ctr);
-        w.ctr_bytes = 0;
-        if (!(w.ctr = dev_alloc(ctr_bytes))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-        w.ctr_bytes = ctr_bytes;
-    }
-    if (inv_bytes > w.inv_bytes) {
-        dev_free(w.inv);
-        w.inv_bytes = 0;
-        if (!(w.inv = dev_alloc(inv_bytes))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-        w.inv_bytes = inv_bytes;
-    }
+    auto grow = [](auto *&buf, size_t &have, size_t bytes) {
+        if (bytes <= have) return true;
+        dev_free(buf);
+        have = 0;
+        buf = static_cast<std::remove_reference_t<decltype(buf)>>(dev_alloc(bytes));
+        if (buf) have = bytes;
+        return buf != nullptr;
+    };
+    if (need.xinv > w.xinv_bytes) w.xinv_owner = nullptr;
+    if (!grow(w.ctr, w.ctr_bytes, need.ctr) || !grow(w.inv, w.inv_bytes, need.inv) ||
+        !grow(w.split, w.split_bytes, need.split) || !grow(w.xinv, w.xinv_bytes, need.xinv) ||
+        !grow(w.y, w.y_bytes, need.y))
+        return CHAMELEON_ERR_OUT_OF_RESOURCES;
     return 0;
 }
 
@@ -436,6 +451,16 @@ static thread_local const Schedule *t_given = nullptr;
 // the same addressing.
 static bool one_tile(const CHAM_desc_t *d) { return priv(d)->cm_view || d->mt == 1; }
 
+// The storage of a matrix as the tile rules see it: rows (columns) in one
+// column-major array, tile sizes, tile columns.
+struct Tiling {
+    bool rows1, cols1;
+    int mb, nb, nt;
+};
+static Tiling tiling(const CHAM_desc_t *d) {
+    return Tiling{one_tile(d), priv(d)->cm_view || d->nt == 1, d->mb, d->nb, d->nt};
+}
+
 // Tile size of the FP64 executor.  The diagonal-tile factorizations are a
 // serial chain on one CTA each, so tiles of the caller's size (512, say) leave
 // the chip waiting for them: the executor uses tiles of EXEC_NB wherever the
@@ -444,10 +469,10 @@ static bool one_tile(const CHAM_desc_t *d) { return priv(d)->cm_view || d->mt ==
 // least, below that the tasks are all overhead).  dpotrf of order 8192:
 // storage tile 512 24.9 ms, executor tile 256 12.8 ms, 128 9.8 ms, 64 14.9 ms.
 constexpr int EXEC_NB = 128;
-static int exec_tile(const CHAM_desc_t *A, const CHAM_desc_t *B) {
-    const bool free_a = one_tile(A), free_b = !B || one_tile(B);
-    if (free_a && free_b) return EXEC_NB;
-    const int nb = free_a ? B->mb : A->nb;   // A and B have the same row tile size
+static int exec_tile(const Tiling &A, const Tiling *B) {
+    const bool free_b = !B || B->rows1;
+    if (A.rows1 && free_b) return EXEC_NB;
+    const int nb = A.rows1 ? B->mb : A.nb;   // A and B have the same row tile size
     for (int d = EXEC_NB; d >= 64; d -= 64)
         if (nb % d == 0) return d;
     for (int d = std::min(EXEC_NB, nb); d >= 48; --d)
@@ -478,9 +503,9 @@ static int group_f64(int N, int NB, int kgroup) {
 constexpr int SOLVE_NB = 512, SOLVE_NBB = 32;
 
 // Tile size of the substitutions, 0 when the storage allows none from 64 on.
-static int solve_tile(const CHAM_desc_t *A, const CHAM_desc_t *B) {
-    if (one_tile(A) && one_tile(B)) return std::min(SOLVE_NB, (A->n + IB - 1) / IB * IB);
-    const int nb = one_tile(A) ? B->mb : A->nb;
+static int solve_tile(int N, const Tiling &A, const Tiling &B) {
+    if (A.rows1 && B.rows1) return std::min(SOLVE_NB, (N + IB - 1) / IB * IB);
+    const int nb = A.rows1 ? B.mb : A.nb;
     for (int d = std::min(SOLVE_NB, nb); d >= IB; --d)
         if (nb % d == 0) return d;
     return 0;
@@ -565,43 +590,53 @@ static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, cudaStr
 
 constexpr int TC_CHAIN_N = 20480;
 
-// Enqueue one launch of the executor (mode: factorization, substitutions or
-// both).  xnb > 0 (FP64 substitutions): tiles of xnb with their full inverses.
-// st: its state, initialized by the caller; after: state of an earlier launch
-// that must not have failed.  *xinv_made: the launch computes the FP32 tile
-// inverses of this factor.
-static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B, cudaStream_t s, int split,
-                       ExecWs &w, int grid_req, int flags, const CastIn *cin, int xnb, ExecState *st,
-                       const ExecState *after, bool *xinv_made, int *ntasks) {
+// One launch of the executor: its mode, tiles, task list and workspace.  Made
+// on the host alone (plan_launch).
+struct Plan {
+    int mode, N, NB, NT, nrhs, NBB, NTB, b_c, xnb, grid;
+    bool f32, tc, full_inv, xinv;
+    Shape sh;
+    int G, NIB;
+    size_t nctr, xelems;
+    WsBytes ws;
+};
+
+// mode: factorization, substitutions or both.  xnb > 0 (FP64 substitutions):
+// tiles of xnb with their full inverses.  B, b_elems: storage of B and its
+// elements (nrhs > 0).  reuse: the workspace holds the FP32 tile inverses of
+// this factor.
+static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling *B, int nrhs, size_t b_elems,
+                        int split, int grid_req, const CastIn *cin, int xnb, bool reuse) {
     Context &c = ctx();
-    const int N = A->n;
-    const bool f32 = (A->dtyp == ChamRealFloat);
-    const int NB = xnb > 0 ? xnb : (t_given || f32) ? A->nb : exec_tile(A, (mode & MODE_SOLVE) ? B : nullptr);
-    const int NT = (N + NB - 1) / NB;
-    const int nrhs = (B && (mode & MODE_SOLVE)) ? B->n : 0;
-    int NBB = B ? B->nb : NB, NTB = nrhs ? B->nt : 0, b_c = 1;
+    Plan q{};
+    if (!(mode & MODE_SOLVE)) nrhs = 0;
+    q.N = N;
+    q.f32 = f32;
+    q.xnb = xnb;
+    q.nrhs = nrhs;
+    const int NB = q.NB = xnb > 0 ? xnb : (t_given || f32) ? A.nb : exec_tile(A, (mode & MODE_SOLVE) ? B : nullptr);
+    const int NT = q.NT = (N + NB - 1) / NB;
+    q.NBB = B ? B->nb : NB;
+    q.NTB = nrhs ? B->nt : 0;
+    q.b_c = 1;
     if (xnb > 0) {
-        const bool one_col = priv(B)->cm_view || B->nt == 1;
         const int want = nrhs <= 1024 ? SOLVE_NBB : 2 * SOLVE_NBB;
-        if (one_col || B->nb % want == 0) {
-            b_c = one_col ? (nrhs + want - 1) / want : B->nb / want;
-            NBB = want;
-            NTB = (nrhs + want - 1) / want;
+        if (B->cols1 || B->nb % want == 0) {
+            q.b_c = B->cols1 ? (nrhs + want - 1) / want : B->nb / want;
+            q.NBB = want;
+            q.NTB = (nrhs + want - 1) / want;
         }
     }
-    if (cin) {
-        if (!f32 || !(mode & MODE_FACT)) return CHAMELEON_ERR_ILLEGAL_VALUE;
-        mode |= MODE_CAST;
-    }
+    const int NBB = q.NBB, NTB = q.NTB;
+    if (cin) mode |= MODE_CAST;
     // tcgen05 trailing updates: FP32 factorization with BF16x3 products and
     // 64-aligned tiles (the split chunks are 64 wide in k).
-    const bool tc = f32 && split == SPLIT_BF16X3 && (mode & MODE_FACT) && (NB % tc05::BK == 0) && NT > 1 &&
-                    c.use_tcgen05;
-    int rc = 0;
+    const bool tc = q.tc = f32 && split == SPLIT_BF16X3 && (mode & MODE_FACT) && (NB % tc05::BK == 0) && NT > 1 &&
+                           c.use_tcgen05;
     // grid_req counts SMs; FP64 places two executor CTAs on each
     const int cps = f32 ? 1 : 2;
-    const int grid = cps * ((grid_req > 0) ? std::min(grid_req, c.num_sms) : c.num_sms);
-    const bool full_inv = f32 && c.rec_tile && NB <= (64 << rec::MAX_LVL);
+    q.grid = cps * ((grid_req > 0) ? std::min(grid_req, c.num_sms) : c.num_sms);
+    const bool full_inv = q.full_inv = f32 && c.rec_tile && NB <= (64 << rec::MAX_LVL);
     if (!f32 && !t_given) mode |= MODE_FINE;
     // The tcgen05 path is bound by the chain of diagonal tiles up to about 80
     // tiles of 256 and by its updates (L2 operand traffic) beyond: the chain's
@@ -616,15 +651,14 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     // FP32 substitutions with full diagonal-tile inverses: computed off the
     // critical path in a factor+solve launch, reused by later solve-only
     // launches on the same factor and workspace (flags & EXEC_REUSE_INV).
-    const bool xinv = xnb > 0 || (f32 && !full_inv && c.xinv_solve && (mode & MODE_SOLVE) && nrhs > 0 &&
-                                  NB <= (64 << rec::MAX_LVL));
+    q.xinv = xnb > 0 || (f32 && !full_inv && c.xinv_solve && (mode & MODE_SOLVE) && nrhs > 0 &&
+                         NB <= (64 << rec::MAX_LVL));
     if (xnb > 0) mode |= MODE_XINV | MODE_NOINV;
-    else if (xinv) {
+    else if (q.xinv) {
         mode |= MODE_XINV;
-        if (!(mode & MODE_FACT) && (flags & EXEC_REUSE_INV) && w.xinv_owner == A->mat && w.xinv_nt == NT &&
-            w.xinv_nb == NB && w.xinv_n == N)
-            mode |= MODE_NOINV;
+        if (!(mode & MODE_FACT) && reuse) mode |= MODE_NOINV;
     }
+    q.mode = mode;
     // The task list depends on N only through NT and the number of SUBB-row
     // blocks of the last tile row, and on nrhs only through NTB (the kernel
     // takes the exact sizes from the parameters): key the cache on that
@@ -639,35 +673,69 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     const int canonR = nrhs ? (NTB - 1) * NBB + std::min(NBB, ((nrhs - (NTB - 1) * NBB + 15) / 16) * 16) : 0;
     // update group size: fused k steps amortize the C round trip and the
     // dispatch of an update over G panels (CHAMELEON_B200_UPD_GROUP per path)
-    const int G = t_given ? 1
-                          : prof == PROF_FP64 ? group_f64(N, NB, c.kgroup_f64)
-                                              : std::max(1, !tc ? c.kgroup_f32
-                                                                : chain_bound ? c.kgroup_tc : c.kgroup_tc + c.kgroup_tc / 2);
-    Shape sh{mode, canonN, NB, canonR, NBB, grid, prof, G, cin ? std::max(1, cin->h2d_gbs) : 0, upd_tail(prof)};
-    const Schedule *sch = t_given ? t_given : get_schedule(sh);
-    if (!sch) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-    const int NIB = (NB + IB - 1) / IB;
-    const size_t nctr = (size_t)(cin ? 3 : 2) * NT * NT + (size_t)4 * NT * std::max(NTB, 1) + NT;
+    const int G = q.G = t_given ? 1
+                                : prof == PROF_FP64 ? group_f64(N, NB, c.kgroup_f64)
+                                                    : std::max(1, !tc ? c.kgroup_f32
+                                                                      : chain_bound ? c.kgroup_tc : c.kgroup_tc + c.kgroup_tc / 2);
+    q.sh = Shape{mode, canonN, NB, canonR, NBB, q.grid, prof, G, cin ? std::max(1, cin->h2d_gbs) : 0, upd_tail(prof)};
+    q.NIB = (NB + IB - 1) / IB;
+    q.nctr = (size_t)(cin ? 3 : 2) * NT * NT + (size_t)4 * NT * std::max(NTB, 1) + NT;
     const size_t esz = f32 ? sizeof(float) : sizeof(double);
-    const size_t inv_elems = full_inv ? (size_t)NT * NB * NB : (size_t)NT * NIB * IB * IB;
-    rc = ensure_ws(w, nctr * sizeof(int), xnb > 0 ? 0 : inv_elems * esz);
-    if (rc) return rc;
-    if (!st) st = w.st;
-    int rcA = desc_upload(A);
-    if (rcA) return rcA;
-    if (nrhs) {
-        int rcB = desc_upload(B);
-        if (rcB) return rcB;
+    q.ws.ctr = q.nctr * sizeof(int);
+    if (xnb <= 0) q.ws.inv = (full_inv ? (size_t)NT * NB * NB : (size_t)NT * q.NIB * IB * IB) * esz;
+    if (q.xinv) {
+        q.xelems = (size_t)NT * NB * NB;
+        q.ws.xinv = q.xelems * (f32 ? sizeof(float) : 2 * sizeof(double));
+        q.ws.y = b_elems * esz;   // forward-substitution results, same tile layout as B
     }
+    if (tc) {
+        const size_t tile_bytes = (size_t)((NB + SUBB - 1) / SUBB) * (NB / tc05::BK) * 2 * tc05::CHUNK_BYTES;
+        q.ws.split = (size_t)NT * (NT - 1) / 2 * tile_bytes;
+    }
+    return q;
+}
+
+// The launches of one call (1 or 2); ws: what they need together.
+static int plan_call(Plan (&q)[2], WsBytes &ws, int mode, int N, bool f32, const Tiling &A, const Tiling *B, int nrhs,
+                     size_t b_elems, int split, int grid_req, const CastIn *cin, bool reuse) {
+    // FP64 substitutions above one executor tile: a launch of their own, after
+    // the factorization's (which it checks on the device).  With a
+    // factorization of a small matrix they stay in its launch, where the
+    // forward sweep runs beside it (dposv 203: 232 us in one launch, 256 in
+    // two; 2048: 1.70 and 1.73 ms; 5003: 6.16 and 5.95 ms).
+    const bool own = (mode & MODE_FACT) ? N > 3072 : N > EXEC_NB;
+    const int xnb = (!f32 && !t_given && nrhs > 0 && own) ? solve_tile(N, A, *B) : 0;
+    int n = 0;
+    if (xnb > 0) {
+        if (mode & MODE_FACT)
+            q[n++] = plan_launch(MODE_FACT, N, f32, A, nullptr, 0, 0, split, grid_req, nullptr, 0, false);
+        q[n++] = plan_launch(MODE_SOLVE, N, f32, A, B, nrhs, b_elems, split, grid_req, nullptr, xnb, false);
+    } else {
+        q[n++] = plan_launch(mode, N, f32, A, B, nrhs, b_elems, split, grid_req, cin, 0, reuse);
+    }
+    ws = WsBytes{};
+    for (int i = 0; i < n; ++i) ws.cover(q[i].ws);
+    return n;
+}
+
+// Enqueue one launch of the executor; the workspace holds what the plan needs
+// and the descriptors are uploaded.  st: its state, initialized by the caller;
+// after: state of an earlier launch that must not have failed.
+static int enqueue_dag(const Plan &q, const Schedule *sch, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
+                       cudaStream_t s, int split, ExecWs &w, const CastIn *cin, ExecState *st,
+                       const ExecState *after) {
+    Context &c = ctx();
+    const int N = q.N, NB = q.NB, NT = q.NT, nrhs = q.nrhs, NTB = q.NTB;
+    int rc = 0;
     ExecParams p{};
     p.tasks = sch->d_tasks;
     p.ntasks = (int)sch->tasks.size();
     // one CTA runs the diagonal-tile factorizations (its instruction cache stays
     // warm for their long unrolled leaves); the others skip them
-    const bool dedicate = c.potrf_cta && grid > 1 && sch->npotrf > 1;
+    const bool dedicate = c.potrf_cta && q.grid > 1 && sch->npotrf > 1;
     p.npotrf = dedicate ? sch->npotrf : 0;
     p.potrf_idx = sch->d_potrf;
-    p.mode = mode;
+    p.mode = q.mode;
     p.upper = (uplo == ChamUpper);
     p.NT = NT; p.N = N; p.NB = NB;
     p.A = A->mat;
@@ -675,13 +743,13 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     p.a_ld = priv(A)->dev.ld;
     p.a_nt = A->mt;
     p.a_r = one_tile(A) ? NT : std::max(1, A->nb / NB);
-    p.NTB = NTB; p.nrhs = nrhs; p.NBB = NBB;
+    p.NTB = NTB; p.nrhs = nrhs; p.NBB = q.NBB;
     p.B = nrhs ? B->mat : nullptr;
     p.b_off = nrhs ? priv(B)->dev.off : nullptr;
     p.b_ld = nrhs ? priv(B)->dev.ld : nullptr;
     p.b_nt = nrhs ? B->mt : 1;
     p.b_r = nrhs ? (one_tile(B) ? NT : std::max(1, B->mb / NB)) : 1;
-    p.b_c = b_c;
+    p.b_c = q.b_c;
     int *ctr = (int *)w.ctr;
     p.updA = ctr;
     p.panA = ctr + (size_t)NT * NT;
@@ -691,8 +759,8 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     p.bwdB = p.fwdDone + nb4;
     p.bwdDone = p.bwdB + nb4;
     p.invd = w.inv;
-    p.NIB = NIB;
-    p.full_inv = full_inv ? 1 : 0;
+    p.NIB = q.NIB;
+    p.full_inv = q.full_inv ? 1 : 0;
     p.xinvDone = p.bwdDone + nb4;
     if (cin) {
         p.castDone = p.xinvDone + NT;
@@ -704,28 +772,12 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
         p.covf = cin->ovf;
     }
     p.xinv = nullptr;
-    if (xinv) {
-        const size_t xelems = (size_t)NT * NB * NB, xbytes = xelems * (f32 ? sizeof(float) : 2 * sizeof(double));
-        if (xbytes > w.xinv_bytes) {
-            dev_free(w.xinv);
-            w.xinv_bytes = 0;
-            w.xinv_owner = nullptr;
-            if (!(w.xinv = dev_alloc(xbytes))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-            w.xinv_bytes = xbytes;
-        }
+    if (q.xinv) {
         p.xinv = w.xinv;
-        if (xnb > 0 || !(mode & MODE_NOINV)) w.xinv_owner = nullptr;   // rewritten by this call
-        if (xnb > 0) {
+        if (q.xnb > 0 || !(q.mode & MODE_NOINV)) w.xinv_owner = nullptr;   // rewritten by this call
+        if (q.xnb > 0) {
             const DiagTiles d{(double *)A->mat, priv(A)->dev.off, priv(A)->dev.ld, p.a_nt, p.a_r, NB, N, p.upper};
-            if ((rc = xinv_launch(d, NT, (double *)w.xinv, (double *)w.xinv + xelems, s))) return rc;
-        }
-        // forward-substitution results, same tile layout as B
-        const size_t ybytes = (size_t)(priv(B)->cm_view ? B->lda : B->lm) * B->ln * esz;
-        if (ybytes > w.y_bytes) {
-            dev_free(w.y);
-            w.y_bytes = 0;
-            if (!(w.y = dev_alloc(ybytes))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-            w.y_bytes = ybytes;
+            if ((rc = xinv_launch(d, NT, (double *)w.xinv, (double *)w.xinv + q.xelems, s))) return rc;
         }
         p.Y = w.y;
     }
@@ -733,32 +785,22 @@ static int enqueue_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *
     p.after = after;
     p.trace = (g_trace_buf && g_trace_cap >= p.ntasks) ? g_trace_buf : nullptr;
     p.wait_budget_ns = (unsigned long long)c.wait_budget_us * 1000ull;
-    p.kgroup = G;
-    p.utail = sh.tail;
-    if (tc) {
+    p.kgroup = q.G;
+    p.utail = q.sh.tail;
+    if (q.tc) {
         p.split_nrb = (NB + SUBB - 1) / SUBB;
         p.split_nkc = NB / tc05::BK;
-        const size_t tile_bytes = (size_t)p.split_nrb * p.split_nkc * 2 * tc05::CHUNK_BYTES;
-        const size_t bytes = (size_t)NT * (NT - 1) / 2 * tile_bytes;
-        if (bytes > w.split_bytes) {
-            dev_free(w.split);
-            w.split_bytes = 0;
-            if (!(w.split = (uint8_t *)dev_alloc(bytes))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-            w.split_bytes = bytes;
-        }
         p.split = w.split;
     }
-    CHB_CUDA(cudaMemsetAsync(ctr, 0, nctr * sizeof(int), s));
+    CHB_CUDA(cudaMemsetAsync(ctr, 0, q.nctr * sizeof(int), s));
     if (p.ntasks > 0) {
         CHB_LAUNCHED(1);
-        if (!f32) rc = launch_dag_f64(p, grid, s);
-        else if (split == SPLIT_TF32X3) rc = launch_dag_tf32(p, grid, s);
-        else if (tc) rc = launch_dag_f32tc(p, grid, s);
-        else rc = launch_dag_f32(p, grid, s);
+        if (!q.f32) rc = launch_dag_f64(p, q.grid, s);
+        else if (split == SPLIT_TF32X3) rc = launch_dag_tf32(p, q.grid, s);
+        else if (q.tc) rc = launch_dag_f32tc(p, q.grid, s);
+        else rc = launch_dag_f32(p, q.grid, s);
         if (rc) return rc;
     }
-    *xinv_made = f32 && xinv && !(mode & MODE_NOINV);
-    *ntasks = p.ntasks;
     return 0;
 }
 
@@ -771,32 +813,30 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     res->info = 0; res->error = 0; res->ms = 0.f;
     if (N == 0) return 0;
     if (nrhs && B->dtyp != A->dtyp) return CHAMELEON_ERR_ILLEGAL_VALUE;
-    int rc = ensure_ws(w, 0, 0);
+    if (cin && (!f32 || !(mode & MODE_FACT))) return CHAMELEON_ERR_ILLEGAL_VALUE;
+    const bool reuse = (flags & EXEC_REUSE_INV) && w.xinv_owner == A->mat && w.xinv_nt == A->nt &&
+                       w.xinv_nb == A->nb && w.xinv_n == N;
+    const Tiling tA = tiling(A), tB = B ? tiling(B) : Tiling{};
+    const size_t b_elems = nrhs ? (size_t)(priv(B)->cm_view ? B->lda : B->lm) * B->ln : 0;
+    Plan q[2];
+    WsBytes need;
+    const int nq = plan_call(q, need, mode, N, f32, tA, B ? &tB : nullptr, nrhs, b_elems, split, grid_req, cin, reuse);
+    // task lists, memory and tables of every launch before the first one
+    // starts: none of them may be replaced while a launch still uses it
+    const Schedule *sch[2] = {};
+    for (int i = 0; i < nq; ++i)
+        if (!(sch[i] = t_given ? t_given : get_schedule(q[i].sh))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+    int rc = ensure_ws(w, need);
+    if (!rc) rc = desc_upload(A);
+    if (!rc && nrhs) rc = desc_upload(B);
     if (rc) return rc;
     ExecState init[2] = {};
     init[0].info = init[1].info = INT_MAX;
     init[0].stuck_task = init[1].stuck_task = -1;
     CHB_CUDA(cudaMemcpyAsync(w.st, init, sizeof(init), cudaMemcpyHostToDevice, s));
     CHB_CUDA(cudaEventRecord(w.e0, s));
-    // FP64 substitutions above one executor tile: a launch of their own, after
-    // the factorization's (which it checks on the device).  With a
-    // factorization of a small matrix they stay in its launch, where the
-    // forward sweep runs beside it (dposv 203: 232 us in one launch, 256 in
-    // two; 2048: 1.70 and 1.73 ms; 5003: 6.16 and 5.95 ms).
-    const bool own = (mode & MODE_FACT) ? N > 3072 : N > EXEC_NB;
-    const int xnb = (!f32 && !t_given && nrhs > 0 && own) ? solve_tile(A, B) : 0;
-    bool xinv_made = false;
-    int ntasks[2] = {0, 0};
-    if (xnb > 0) {
-        if (mode & MODE_FACT)
-            rc = enqueue_dag(MODE_FACT, uplo, A, nullptr, s, split, w, grid_req, flags, nullptr, 0, w.st, nullptr,
-                             &xinv_made, &ntasks[0]);
-        if (!rc)
-            rc = enqueue_dag(MODE_SOLVE, uplo, A, B, s, split, w, grid_req, flags, nullptr, xnb, w.st + 1, w.st,
-                             &xinv_made, &ntasks[1]);
-    } else {
-        rc = enqueue_dag(mode, uplo, A, B, s, split, w, grid_req, flags, cin, 0, w.st, nullptr, &xinv_made, &ntasks[0]);
-    }
+    for (int i = 0; i < nq && !rc; ++i)
+        rc = enqueue_dag(q[i], sch[i], uplo, A, B, s, split, w, cin, w.st + i, i ? w.st : nullptr);
     if (rc) return rc;
     CHB_CUDA(cudaEventRecord(w.e1, s));
     ExecState out[2] = {};
@@ -805,17 +845,17 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     CHB_CUDA(cudaEventElapsedTime(&res->ms, w.e0, w.e1));
     res->info = (out[0].info == INT_MAX) ? 0 : out[0].info;
     res->error = out[0].error ? out[0].error : out[1].error;
-    if (xinv_made && res->info == 0 && res->error == 0) {
+    if (f32 && q[0].xinv && !(q[0].mode & MODE_NOINV) && res->info == 0 && res->error == 0) {
         w.xinv_owner = A->mat;   // the inverses now match this factor
         w.xinv_n = N;
         w.xinv_nt = A->nt;
         w.xinv_nb = A->nb;
     }
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < nq; ++i)
         if (out[i].error) {
             char msg[160];
             snprintf(msg, sizeof msg, "device wait budget exhausted at task %d (%d of %d done)", out[i].stuck_task,
-                     out[i].done, ntasks[i]);
+                     out[i].done, (int)sch[i]->tasks.size());
             warning("run_cholesky_dag", msg);
         }
     return 0;
@@ -863,7 +903,10 @@ int dag_potrf_async(cham_uplo_t uplo, int n, double *A, int lda, int *d_info, cu
     }
     const Schedule *sch = get_schedule(sh);
     if (!sch) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-    if (int rc = ensure_ws(w, ctr_bytes, inv_bytes)) return rc;
+    WsBytes need;
+    need.ctr = ctr_bytes;
+    need.inv = inv_bytes;
+    if (int rc = ensure_ws(w, need)) return rc;
     OneTile *tab = (OneTile *)w.ctr;
     int *ctr = (int *)(tab + 1);
     dag_init_kernel<<<1, 256, 0, s>>>(tab, lda, ctr, (int)nctr, w.st);
@@ -937,6 +980,30 @@ extern "C" int CHAM_B200_Schedule_Size(int mode, int N, int NB, int nrhs, int NB
     return (int)build_order(Shape{mode, N, NB, nrhs, NBB, workers, prof, std::max(1, kgroup),
                                   (mode & MODE_CAST) ? 50 : 0, upd_tail(prof)})
         .size();
+}
+
+// The launches of one FP64 call (mode MODE_FACT | MODE_SOLVE; A of order N in
+// nb x nb tiles, B in nb x nbb, or both column-major arrays) and their
+// workspace, host only: per launch {tile size, column block, bytes of counters,
+// inverted blocks, tile inverses, forward results}, and in reserved[4] the bytes
+// that the call reserves.  Returns the number of launches (at most 2).
+extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs, int nbb, int64_t *launch,
+                                   int64_t *reserved) {
+    using namespace chb;
+    auto tl = [&](int n, int t) { return Tiling{array || N <= nb, array || n <= t, nb, t, (n + t - 1) / t}; };
+    const Tiling A = tl(N, nb), B = tl(std::max(nrhs, 1), nbb);
+    Plan q[2];
+    WsBytes r;
+    const int n = plan_call(q, r, mode, N, false, A, nrhs > 0 ? &B : nullptr, nrhs, (size_t)N * std::max(nrhs, 0), 0, 0,
+                            nullptr, false);
+    for (int i = 0; i < n; ++i) {
+        const int64_t v[6] = {q[i].NB, q[i].NBB, (int64_t)q[i].ws.ctr, (int64_t)q[i].ws.inv, (int64_t)q[i].ws.xinv,
+                              (int64_t)q[i].ws.y};
+        std::copy(v, v + 6, launch + 6 * i);
+    }
+    const int64_t v[4] = {(int64_t)r.ctr, (int64_t)r.inv, (int64_t)r.xinv, (int64_t)r.y};
+    std::copy(v, v + 4, reserved);
+    return n;
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,34 @@
+"""Host-side checks of what one executor call plans before it launches anything."""
+import ctypes
+
+import numpy as np
+import pytest
+
+FACT, SOLVE = 1, 2
+CTR, INV, XINV, Y = 2, 3, 4, 5     # columns of a planned launch; 0, 1: tile size, column block
+
+
+def plan(mode, N, nb, nrhs, array=False, nbb=None):
+    import chameleon_b200 as cb
+    launch, res = np.zeros((2, 6), np.int64), np.zeros(4, np.int64)
+    p = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
+    n = cb.lib().CHAM_B200_Exec_Plan(mode, N, nb, int(array), nrhs, nbb or nb, p(launch), p(res))
+    return launch[:n], res
+
+
+@pytest.mark.parametrize("N,nb,nrhs", [(3144, 262, 64), (3200, 200, 900), (3073, 512, 1), (8192, 512, 64),
+                                       (5003, 384, 17), (2048, 320, 1)])
+@pytest.mark.parametrize("array", [False, True])
+def test_workspace_is_reserved_for_every_launch(N, nb, nrhs, array):
+    """The factorization's launch still runs when the substitutions' is
+    enqueued, so no buffer may grow between the two: what the call reserves
+    before the first launch covers both."""
+    launch, res = plan(FACT | SOLVE, N, nb, nrhs, array)
+    assert len(launch) == (2 if N > 3072 else 1)
+    assert (res >= launch[:, CTR:].max(axis=0)).all()
+
+
+def test_substitutions_may_need_more_counters_than_the_factorization():
+    launch, res = plan(FACT | SOLVE, 3144, 262, 64)
+    assert launch[1, CTR] > launch[0, CTR]
+    assert res[0] == launch[1, CTR] and res[1] == launch[0, INV]
