@@ -718,6 +718,17 @@ static int plan_call(Plan (&q)[2], WsBytes &ws, int mode, int N, bool f32, const
     return n;
 }
 
+// step(0), step(1), .. up to the first that fails, then drain() whatever
+// happened: a call never returns with its own launches still running on the
+// caller's arrays, the workspace and the descriptors' tables.
+template <class Step, class Drain>
+static int enqueue_all(int n, Step step, Drain drain) {
+    int rc = 0;
+    for (int i = 0; i < n && !rc; ++i) rc = step(i);
+    const int rd = drain();
+    return rc ? rc : rd;
+}
+
 // Enqueue one launch of the executor; the workspace holds what the plan needs
 // and the descriptors are uploaded.  st: its state, initialized by the caller;
 // after: state of an earlier launch that must not have failed.
@@ -833,15 +844,27 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
     ExecState init[2] = {};
     init[0].info = init[1].info = INT_MAX;
     init[0].stuck_task = init[1].stuck_task = -1;
-    CHB_CUDA(cudaMemcpyAsync(w.st, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    CHB_CUDA(cudaEventRecord(w.e0, s));
-    for (int i = 0; i < nq && !rc; ++i)
-        rc = enqueue_dag(q[i], sch[i], uplo, A, B, s, split, w, cin, w.st + i, i ? w.st : nullptr);
-    if (rc) return rc;
-    CHB_CUDA(cudaEventRecord(w.e1, s));
     ExecState out[2] = {};
-    CHB_CUDA(cudaMemcpyAsync(out, w.st, sizeof(out), cudaMemcpyDeviceToHost, s));
-    CHB_CUDA(cudaStreamSynchronize(s));
+    rc = enqueue_all(
+        nq + 2,
+        [&](int i) -> int {
+            if (i == 0) {
+                CHB_CUDA(cudaMemcpyAsync(w.st, init, sizeof(init), cudaMemcpyHostToDevice, s));
+                CHB_CUDA(cudaEventRecord(w.e0, s));
+                return 0;
+            }
+            if (i <= nq)
+                return enqueue_dag(q[i - 1], sch[i - 1], uplo, A, B, s, split, w, cin, w.st + i - 1,
+                                   i > 1 ? w.st : nullptr);
+            CHB_CUDA(cudaEventRecord(w.e1, s));
+            CHB_CUDA(cudaMemcpyAsync(out, w.st, sizeof(out), cudaMemcpyDeviceToHost, s));
+            return 0;
+        },
+        [&]() -> int {
+            CHB_CUDA(cudaStreamSynchronize(s));
+            return 0;
+        });
+    if (rc) return rc;
     CHB_CUDA(cudaEventElapsedTime(&res->ms, w.e0, w.e1));
     res->info = (out[0].info == INT_MAX) ? 0 : out[0].info;
     res->error = out[0].error ? out[0].error : out[1].error;
@@ -1004,6 +1027,23 @@ extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs,
     const int64_t v[4] = {(int64_t)r.ctr, (int64_t)r.inv, (int64_t)r.xinv, (int64_t)r.y};
     std::copy(v, v + 4, reserved);
     return n;
+}
+
+// enqueue_all with n steps of which step `bad` fails with rc (none: bad < 0):
+// writes the steps in the order of their calls, -1 for the drain, and returns
+// its result; *len receives the count (at most n + 1).
+extern "C" int CHAM_B200_Test_Enqueue_All(int n, int bad, int rc, int *calls, int *len) {
+    *len = 0;
+    return chb::enqueue_all(
+        n,
+        [&](int i) {
+            calls[(*len)++] = i;
+            return i == bad ? rc : 0;
+        },
+        [&] {
+            calls[(*len)++] = -1;
+            return 0;
+        });
 }
 
 // ---------------------------------------------------------------------------

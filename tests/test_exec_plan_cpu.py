@@ -32,3 +32,14 @@ def test_substitutions_may_need_more_counters_than_the_factorization():
     launch, res = plan(FACT | SOLVE, 3144, 262, 64)
     assert launch[1, CTR] > launch[0, CTR]
     assert res[0] == launch[1, CTR] and res[1] == launch[0, INV]
+
+
+@pytest.mark.parametrize("bad", [-1, 0, 1, 3])
+def test_a_failed_launch_is_not_left_behind(bad):
+    """After a step that fails nothing more is enqueued, and what was is waited for."""
+    import chameleon_b200 as cb
+    calls, n = (ctypes.c_int * 8)(), ctypes.c_int()
+    rc = cb.lib().CHAM_B200_Test_Enqueue_All(4, bad, 103, calls, ctypes.byref(n))
+    last = 3 if bad < 0 else bad
+    assert rc == (0 if bad < 0 else 103)
+    assert list(calls[:n.value]) == [*range(last + 1), -1]
