@@ -135,10 +135,12 @@ cudaStream_t meta_stream() {
 // threshold = max), so workspace churn never returns memory to the driver and
 // re-maps it -- which can stall every stream of the device.  The pool is an
 // object of this process; no device setting changes.
+static std::atomic<int> g_pool_device{-1};
 static cudaMemPool_t lib_pool() {
     static std::once_flag once;
     static cudaMemPool_t pool = nullptr;
     std::call_once(once, [] {
+        g_pool_device = ctx().device;
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -152,6 +154,12 @@ static cudaMemPool_t lib_pool() {
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     });
     return pool;
+}
+
+// (without creating the pool: the caller's stream may be under capture)
+int pool_device() {
+    const int d = g_pool_device;
+    return d >= 0 ? d : ctx().device;
 }
 
 void *dev_alloc(size_t bytes) {

@@ -907,6 +907,7 @@ int dag_potrf_async(cham_uplo_t uplo, int n, double *A, int lda, int *d_info, cu
     const int NB = EXEC_NB, NT = (n + NB - 1) / NB, mode = MODE_FACT | MODE_FINE;
     int dev = 0, sms = 0;
     CHB_CUDA(cudaGetDevice(&dev));
+    if (!dag_potrf_usable(n, dev, pool_device())) return 0;
     CHB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // as many CTAs as the first step has panel-solve and update blocks
     const int grid = std::min(2 * sms, 2 * NT * NT);
@@ -1029,6 +1030,11 @@ extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs,
     return n;
 }
 
+// Whether CUDA_dpotrf of order n takes the tile DAG on a stream of `device`
+// when the library's memory is on pool_device.
+extern "C" int CHAM_B200_Test_Potrf_On_Dag(int n, int device, int pool_device) {
+    return chb::dag_potrf_usable(n, device, pool_device);
+}
 // enqueue_all with n steps of which step `bad` fails with rc (none: bad < 0):
 // writes the steps in the order of their calls, -1 for the drain, and returns
 // its result; *len receives the count (at most n + 1).

@@ -102,6 +102,8 @@ cudaStream_t meta_stream();   // private stream of descriptor metadata uploads
 // (no device-wide synchronization, no kernel); contents undefined.
 void *dev_alloc(size_t bytes);
 void dev_free(void *p);
+// The device that dev_alloc's memory is on.
+int pool_device();
 // Map `bytes` of device memory into the library pool ahead of use.
 int pool_reserve(size_t bytes);
 // Tile-layout (CCRB) m x n descriptor on caller-owned device storage of at
@@ -218,8 +220,13 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
 
 // FP64 Cholesky of a device column-major matrix on the executor, in stream
 // order on s (no synchronization; *d_info, may be null, receives LAPACK's info
-// or an error code).  *ran = false, with nothing launched, when s is being
-// captured and the task list or the workspace w would have to be made first.
+// or an error code).  *ran = false, with nothing launched, when dag_potrf_usable
+// says no, or s is being captured and the task list or the workspace w would
+// have to be made first.
+// Above one executor tile the tile DAG runs on many CTAs (order 512: one CTA
+// 532 us).  Its task lists and workspaces are library memory, on one device: a
+// call on another one keeps to the handle's own memory and one CTA.
+constexpr bool dag_potrf_usable(int n, int device, int pool_dev) { return n > 128 && device == pool_dev; }
 int dag_potrf_async(cham_uplo_t uplo, int n, double *A, int lda, int *d_info, cudaStream_t s, ExecWs &w, bool *ran);
 
 // Tile size of the mixed solver's FP32 factorization for FP64 tile size NB (mixed.cu).

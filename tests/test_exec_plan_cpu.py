@@ -43,3 +43,14 @@ def test_a_failed_launch_is_not_left_behind(bad):
     last = 3 if bad < 0 else bad
     assert rc == (0 if bad < 0 else 103)
     assert list(calls[:n.value]) == [*range(last + 1), -1]
+
+
+@pytest.mark.parametrize("n", [1, 128, 129, 512, 4096])
+@pytest.mark.parametrize("device", [0, 1, 3])
+def test_dpotrf_of_another_device_keeps_to_its_own_memory(n, device):
+    """Task lists and executor workspaces are on the library's device: a stream
+    of another one runs the kernel that uses the handle's memory alone."""
+    import chameleon_b200 as cb
+    on = cb.lib().CHAM_B200_Test_Potrf_On_Dag
+    assert on(n, device, device) == (n > 128)
+    assert not any(on(n, device, d) for d in (-1, 0, 1, 2, 3) if d != device)
