@@ -637,7 +637,9 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     const int cps = f32 ? 1 : 2;
     q.grid = cps * ((grid_req > 0) ? std::min(grid_req, c.num_sms) : c.num_sms);
     const bool full_inv = q.full_inv = f32 && c.rec_tile && NB <= (64 << rec::MAX_LVL);
-    if (!f32 && !t_given) mode |= MODE_FINE;
+    // (a task names its block by two 8-bit indices: a storage tile too large for
+    // 64-blocks, and with no divisor to use instead, keeps 128-blocks)
+    if (!f32 && !t_given && NB <= 255 * FINEB) mode |= MODE_FINE;
     // The tcgen05 path is bound by the chain of diagonal tiles up to about 80
     // tiles of 256 and by its updates (L2 operand traffic) beyond: the chain's
     // panel solves are split in two and the update groups kept short there
@@ -1009,7 +1011,7 @@ extern "C" int CHAM_B200_Schedule_Size(int mode, int N, int NB, int nrhs, int NB
 // The launches of one FP64 call (mode MODE_FACT | MODE_SOLVE; A of order N in
 // nb x nb tiles, B in nb x nbb, or both column-major arrays) and their
 // workspace, host only: per launch {tile size, column block, bytes of counters,
-// inverted blocks, tile inverses, forward results}, and in reserved[4] the bytes
+// inverted blocks, tile inverses, forward results, mode}, and in reserved[4] the bytes
 // that the call reserves.  Returns the number of launches (at most 2).
 extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs, int nbb, int64_t *launch,
                                    int64_t *reserved) {
@@ -1021,9 +1023,9 @@ extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs,
     const int n = plan_call(q, r, mode, N, false, A, nrhs > 0 ? &B : nullptr, nrhs, (size_t)N * std::max(nrhs, 0), 0, 0,
                             nullptr, false);
     for (int i = 0; i < n; ++i) {
-        const int64_t v[6] = {q[i].NB, q[i].NBB, (int64_t)q[i].ws.ctr, (int64_t)q[i].ws.inv, (int64_t)q[i].ws.xinv,
-                              (int64_t)q[i].ws.y};
-        std::copy(v, v + 6, launch + 6 * i);
+        const int64_t v[7] = {q[i].NB, q[i].NBB, (int64_t)q[i].ws.ctr, (int64_t)q[i].ws.inv, (int64_t)q[i].ws.xinv,
+                              (int64_t)q[i].ws.y, q[i].mode};
+        std::copy(v, v + 7, launch + 7 * i);
     }
     const int64_t v[4] = {(int64_t)r.ctr, (int64_t)r.inv, (int64_t)r.xinv, (int64_t)r.y};
     std::copy(v, v + 4, reserved);

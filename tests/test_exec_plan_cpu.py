@@ -5,12 +5,13 @@ import numpy as np
 import pytest
 
 FACT, SOLVE = 1, 2
-CTR, INV, XINV, Y = 2, 3, 4, 5     # columns of a planned launch; 0, 1: tile size, column block
+# columns of a planned launch (0, 1: tile size, column block)
+CTR, INV, XINV, Y, MODE = 2, 3, 4, 5, 6
 
 
 def plan(mode, N, nb, nrhs, array=False, nbb=None):
     import chameleon_b200 as cb
-    launch, res = np.zeros((2, 6), np.int64), np.zeros(4, np.int64)
+    launch, res = np.zeros((2, 7), np.int64), np.zeros(4, np.int64)
     p = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
     n = cb.lib().CHAM_B200_Exec_Plan(mode, N, nb, int(array), nrhs, nbb or nb, p(launch), p(res))
     return launch[:n], res
@@ -25,7 +26,7 @@ def test_workspace_is_reserved_for_every_launch(N, nb, nrhs, array):
     before the first launch covers both."""
     launch, res = plan(FACT | SOLVE, N, nb, nrhs, array)
     assert len(launch) == (2 if N > 3072 else 1)
-    assert (res >= launch[:, CTR:].max(axis=0)).all()
+    assert (res >= launch[:, CTR:MODE].max(axis=0)).all()
 
 
 def test_substitutions_may_need_more_counters_than_the_factorization():
@@ -54,3 +55,27 @@ def test_dpotrf_of_another_device_keeps_to_its_own_memory(n, device):
     on = cb.lib().CHAM_B200_Test_Potrf_On_Dag
     assert on(n, device, device) == (n > 128)
     assert not any(on(n, device, d) for d in (-1, 0, 1, 2, 3) if d != device)
+
+
+@pytest.mark.parametrize("nb", [16383, 16411, 30011])
+def test_blocks_of_a_large_tile_fit_the_task(nb):
+    """Storage tiles without a usable divisor are executor tiles: their blocks'
+    indices (8 bits each) must tell all of them apart."""
+    import chameleon_b200 as cb
+    N = 2 * nb
+    launch, _ = plan(FACT, N, nb, 0)
+    NB, mode = int(launch[0, 0]), int(launch[0, MODE])
+    t = cb.schedule(mode, N, NB, 0, NB, workers=296, kgroup=1)
+    e = 64 if mode & 32 else 128
+    upd = t[t[:, 0] == 3]
+    subs = {(m, n, k): [] for m, n, k in upd[:, 2:5].tolist()}
+    for _, sub, m, n, k, _, _ in upd.tolist():
+        subs[m, n, k].append(sub & 0xffff)
+    rows = lambda m: min(NB, N - m * NB)
+    blk = lambda m: -(-rows(m) // e)
+    for (m, n, k), got in subs.items():
+        want = blk(m) * (blk(m) + 1) // 2 if m == n else blk(m) * blk(n)
+        assert len(set(got)) == len(got) == want
+        assert max(x & 255 for x in got) == blk(m) - 1
+    pan = t[t[:, 0] == 2]
+    assert (pan[:, 1] >= 0).all() and (pan[:, 1] * e < NB).all()
