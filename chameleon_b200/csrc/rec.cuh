@@ -96,8 +96,8 @@ __device__ __forceinline__ bool pivot_recip(float d, float &rc, float &rs) {
 // instead of the finished row k, which the column operations turn into column
 // k of the inverse.  The pivots run on d and its reciprocal (an LDL^T
 // recurrence on the unscaled columns); the square roots stay off the chain.
-// SAFE: any pivot; the first one that is not positive (NaN included) is
-// reported in info (1-based) and replaced by 1.  !SAFE: returns false, with
+// SAFE: any pivot, subnormal and infinite ones too; the first one that is not
+// positive (NaN included) is reported in info (1-based) and replaced by 1.  !SAFE: returns false, with
 // nothing written, when a pivot is not positive or too extreme for the
 // estimates.
 template <class T, bool SAFE>
@@ -119,7 +119,7 @@ __device__ __forceinline__ bool leaf_panel(T *S, T *X, int p, T *rd, int &info) 
         if (unit) a0[k] = (k == lane) ? T(1) : T(0);
     }
     __syncwarp();   // every lane has read the diagonal block before it is overwritten
-    T rs[PW];
+    T rs[PW], root[PW];   // root: SAFE only
     bool ok = true;
 #pragma unroll
     for (int c = 0; c < PW; ++c) {
@@ -130,19 +130,22 @@ __device__ __forceinline__ bool leaf_panel(T *S, T *X, int p, T *rd, int &info) 
                 if (info == 0) info = PW * p + c + 1;
                 dc = T(1);
             }
-            rc = T(1) / dc;
-            rs[c] = T(1) / sqrt(dc);
+            root[c] = sqrt(dc);
+            rs[c] = T(1) / root[c];
         } else {
             ok = pivot_recip(d[c][c], rc, rs[c]) && ok;
         }
-        // (w first: a product of two unscaled entries could leave the exponent range)
+        // (w first: a product of two unscaled entries could leave the exponent
+        // range; and SAFE scales by the root, since the reciprocal of a small
+        // subnormal pivot overflows)
 #pragma unroll
         for (int k = c + 1; k < PW; ++k) {
-            const T w = d[k][c] * rc;
+            const T w = d[k][c] * (SAFE ? rs[c] : rc);
+            const T f = SAFE ? rs[c] : T(1);
 #pragma unroll
-            for (int i = k; i < PW; ++i) d[i][k] -= d[i][c] * w;
-            a0[k] -= a0[c] * w;
-            a1[k] -= a1[c] * w;
+            for (int i = k; i < PW; ++i) d[i][k] -= SAFE ? d[i][c] * f * w : d[i][c] * w;
+            a0[k] -= SAFE ? a0[c] * f * w : a0[c] * w;
+            a1[k] -= SAFE ? a1[c] * f * w : a1[c] * w;
         }
     }
     if (!SAFE && !ok) return false;
@@ -152,7 +155,11 @@ __device__ __forceinline__ bool leaf_panel(T *S, T *X, int p, T *rd, int &info) 
     const int st = unit ? 1 : LDS, last0 = unit ? PW : lane - PW * p, last1 = lane + 32 - PW * p;
 #pragma unroll
     for (int c = 0; c < PW; ++c) {
-        const T v0 = a0[c] * rs[c], v1 = a1[c] * rs[c];
+        T v0 = a0[c] * rs[c], v1 = a1[c] * rs[c];
+        if (SAFE) {   // the diagonal entry: an infinite pivot has an infinite root
+            if (!unit && lane == PW * p + c) v0 = root[c];
+            if (lane + 32 == PW * p + c) v1 = root[c];
+        }
         if (c <= last0) q[c * st] = v0;
         if (c <= last1) P[lane + 32 + c * LDS] = v1;
     }

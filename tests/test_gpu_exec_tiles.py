@@ -63,8 +63,8 @@ def test_posv_and_potrs_over_tilings(cb, layout, uplo, n, nb, nrhs):
 @pytest.mark.parametrize("uplo", [UPPER, LOWER])
 def test_tile_potrf_fp64_orders_and_scales(cb, uplo, n, scale):
     """Every remainder of the 8-wide panels, and pivots beyond the range of
-    the reciprocal estimates (subnormal ones included: absolute errors of a
-    few subnormal units, relative to sqrt of them, bound the last case)."""
+    the reciprocal estimates (3e-309: the entries off the diagonal are subnormal,
+    absolute errors of a few subnormal units, relative to the scale, bound it)."""
     import torch
     L = cb.lib()
     A0 = spd(n, 3 * n, scale)
@@ -111,3 +111,44 @@ def test_first_non_positive_pivot(cb, n, bad):
     A0[bad - 1, bad - 1] = -1.0
     t = torch.from_numpy(A0.copy()).cuda()
     assert cb.dpotrf(LOWER, n, t, n) == bad
+
+
+def factor(cb, name, a):
+    """The lower factor of one tile call and its info."""
+    import torch
+    L = cb.lib()
+    t = torch.from_numpy(a.T.copy()).cuda()
+    info = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    h = ctypes.c_void_p()
+    assert L.CHAM_B200_Handle_Create(ctypes.byref(h), None) == 0
+    n = a.shape[0]
+    assert getattr(L, name)(LOWER, n, t.data_ptr(), n, None, 0, info.data_ptr(), h) == 0
+    torch.cuda.synchronize()
+    L.CHAM_B200_Handle_Destroy(h)
+    return np.tril(t.cpu().numpy().T), int(info)
+
+
+@pytest.mark.parametrize("n", [1, 5, 64])
+@pytest.mark.parametrize("name,dtype,d", [("CUDA_dpotrf", np.float64, 1e-310), ("CUDA_dpotrf", np.float64, 5e-324),
+                                          ("CUDA_spotrf", np.float32, 1e-39), ("CUDA_spotrf", np.float32, 1e-45)])
+def test_subnormal_pivots(cb, n, name, dtype, d):
+    """Diagonal matrices whose pivots' reciprocals overflow: the roots are exact
+    to one rounding, and nothing spreads to the zeros or to the padding."""
+    a = np.diag(np.full(n, d, dtype))
+    F, info = factor(cb, name, a)
+    assert info == 0
+    assert np.abs(np.diag(F) / np.sqrt(np.diag(a)) - 1).max() <= 2 * np.finfo(dtype).eps
+    assert (F[~np.eye(n, dtype=bool)] == 0).all()
+
+
+@pytest.mark.parametrize("name,dtype", [("CUDA_dpotrf", np.float64), ("CUDA_spotrf", np.float32)])
+@pytest.mark.parametrize("n,at", [(1, 0), (24, 3), (64, 63), (64, 40)])
+def test_infinite_pivot(cb, n, at, name, dtype):
+    """An infinite diagonal entry of a diagonal matrix, as LAPACK factors it."""
+    a = np.diag(np.full(n, 4.0, dtype))
+    a[at, at] = np.inf
+    F, info = factor(cb, name, a)
+    assert info == 0
+    want = np.diag(np.full(n, 2.0, dtype))
+    want[at, at] = np.inf
+    assert np.array_equal(F, want)
