@@ -498,9 +498,13 @@ static int group_f64(int N, int NB, int kgroup) {
 // 64-row block with the tile's full inverse, and on column blocks of SOLVE_NBB
 // whose chains run side by side.  The inverses come from products over all
 // tiles at once (xinv_launch) before the chain starts, on the whole chip.
+// A product with an explicit inverse has a backward error that grows with the
+// condition of what was inverted, and nothing refines it here, so a tile whose
+// norm times its inverse's is above XINV_COND is solved with its inverted 64 x
+// 64 blocks instead (solve_strips).
 // Order 8192, 64 right-hand sides: 6.7 ms on the factor's tiles of 512 with
 // inverted 64-blocks, 5.0 ms on tiles of 128, 2.0 ms this way.
-constexpr int SOLVE_NB = 512, SOLVE_NBB = 32;
+constexpr int SOLVE_NBB = 32;
 
 // Tile size of the substitutions, 0 when the storage allows none from 64 on.
 static int solve_tile(int N, const Tiling &A, const Tiling &B) {
@@ -566,8 +570,43 @@ __global__ void __launch_bounds__(NT_CTA, 2) xinv_pair_kernel(DiagTiles d, int h
     }
 }
 
-// The full inverses of all diagonal tiles into X (W: scratch of the same size).
-static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, cudaStream_t s) {
+// cond[2 k], cond[2 k + 1] = the infinity norms of diagonal tile k and of its
+// inverse (zeroed before): 64 rows of one tile per CTA, along the contiguous
+// direction.  The maxima are taken on the bits, where NaN is above Inf.
+__global__ void __launch_bounds__(NT_CTA, 4) xinv_norm_kernel(DiagTiles d, double *X, double *cond) {
+    const int k = blockIdx.y, r0 = blockIdx.x * IB, n = min(IB, d.order(k) - r0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ double s_part[4][IB];
+    const View V[2] = {d.L(k), View{X + (int64_t)k * d.NB * d.NB, 1, d.NB}};
+    for (int m = 0; m < 2; ++m) {
+        long long top = 0;
+        if (V[m].rs == 1) {
+            const int r = threadIdx.x & (IB - 1), q = threadIdx.x / IB;
+            double s = 0.0;
+            if (r < n)
+#pragma unroll 8
+                for (int c = q; c <= r0 + r; c += 4) s += fabs(*V[m].at(r0 + r, c));
+            s_part[q][r] = s;
+            __syncthreads();
+            if (q == 0) top = __double_as_longlong(fabs((s + s_part[1][r]) + (s_part[2][r] + s_part[3][r])));
+            __syncthreads();
+        } else {
+            for (int r = warp; r < n; r += NT_CTA / 32) {
+                double s = 0.0;
+#pragma unroll 4
+                for (int c = lane; c <= r0 + r; c += 32) s += fabs(*V[m].at(r0 + r, c));
+                for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                top = max(top, __double_as_longlong(fabs(s)));
+            }
+        }
+        for (int o = 16; o; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        if (lane == 0 && top) atomicMax(reinterpret_cast<long long *>(cond + 2 * k + m), top);
+    }
+}
+
+// The full inverses of all diagonal tiles into X (W: scratch of the same size),
+// and their norms into cond (zeroed).
+static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, double *cond, cudaStream_t s) {
     constexpr size_t inv_smem = sizeof(double) * 2 * IB * LEAF_LD;
     constexpr size_t pair_smem = GemmCfg<double, 64, 64, 2, 4, SPLIT_BF16X3, 3>::SMEM_BYTES;
     static bool attr = false;
@@ -584,6 +623,8 @@ static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, cudaStr
             xinv_pair_kernel<<<dim3(nb, nb, NT * pairs), NT_CTA, pair_smem, s>>>(d, h, pairs, X, W, first);
         CHB_LAUNCHED(2);
     }
+    xinv_norm_kernel<<<dim3((d.NB + IB - 1) / IB, NT), NT_CTA, 0, s>>>(d, X, cond);
+    CHB_LAUNCHED(1);
     CHB_CUDA(cudaGetLastError());
     return 0;
 }
@@ -682,6 +723,7 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     q.sh = Shape{mode, canonN, NB, canonR, NBB, q.grid, prof, G, cin ? std::max(1, cin->h2d_gbs) : 0, upd_tail(prof)};
     q.NIB = (NB + IB - 1) / IB;
     q.nctr = (size_t)(cin ? 3 : 2) * NT * NT + (size_t)4 * NT * std::max(NTB, 1) + NT;
+    if (xnb > 0) q.nctr = (q.nctr + 1) / 2 * 2 + 4 * NT;   // the tiles' norms (2 doubles each) at the end
     const size_t esz = f32 ? sizeof(float) : sizeof(double);
     q.ws.ctr = q.nctr * sizeof(int);
     if (xnb <= 0) q.ws.inv = (full_inv ? (size_t)NT * NB * NB : (size_t)NT * q.NIB * IB * IB) * esz;
@@ -764,6 +806,7 @@ static int enqueue_dag(const Plan &q, const Schedule *sch, cham_uplo_t uplo, CHA
     p.b_r = nrhs ? (one_tile(B) ? NT : std::max(1, B->mb / NB)) : 1;
     p.b_c = q.b_c;
     int *ctr = (int *)w.ctr;
+    CHB_CUDA(cudaMemsetAsync(ctr, 0, q.nctr * sizeof(int), s));
     p.updA = ctr;
     p.panA = ctr + (size_t)NT * NT;
     const size_t nb4 = (size_t)NT * std::max(NTB, 1);
@@ -790,7 +833,9 @@ static int enqueue_dag(const Plan &q, const Schedule *sch, cham_uplo_t uplo, CHA
         if (q.xnb > 0 || !(q.mode & MODE_NOINV)) w.xinv_owner = nullptr;   // rewritten by this call
         if (q.xnb > 0) {
             const DiagTiles d{(double *)A->mat, priv(A)->dev.off, priv(A)->dev.ld, p.a_nt, p.a_r, NB, N, p.upper};
-            if ((rc = xinv_launch(d, NT, (double *)w.xinv, (double *)w.xinv + q.xelems, s))) return rc;
+            double *cond = reinterpret_cast<double *>(ctr + q.nctr - 4 * NT);
+            p.cond = cond;
+            if ((rc = xinv_launch(d, NT, (double *)w.xinv, (double *)w.xinv + q.xelems, cond, s))) return rc;
         }
         p.Y = w.y;
     }
@@ -805,7 +850,6 @@ static int enqueue_dag(const Plan &q, const Schedule *sch, cham_uplo_t uplo, CHA
         p.split_nkc = NB / tc05::BK;
         p.split = w.split;
     }
-    CHB_CUDA(cudaMemsetAsync(ctr, 0, q.nctr * sizeof(int), s));
     if (p.ntasks > 0) {
         CHB_LAUNCHED(1);
         if (!q.f32) rc = launch_dag_f64(p, q.grid, s);

@@ -95,6 +95,14 @@ constexpr int SUBB = 128;      // sub-block edge of trailing updates / row block
 // diagonal-tile inverses (MODE_XINV): the forward and backward solves are a
 // chain of 2 NT dependent steps, and 64-row tasks halve each step's latency.
 constexpr int SOLB = 64;
+// FP64 substitutions: largest tile with a full inverse, and the bound on the
+// product of the infinity norms of the tile and of its inverse up to which the
+// inverse is used.  Backward errors restated on the host over kernel, Wishart,
+// Laplacian and scaled matrices of orders 512 to 2048 (|b - A x| / |A| |x|):
+// below 8 they agree with those of inverted 64 x 64 blocks, around 30 they are
+// twice as large, at 3e3 up to 20 times, at 1e6 1e4 times.
+constexpr int SOLVE_NB = 512;
+constexpr double XINV_COND = 8.0;
 // Row block of the substitution tasks of a launch mode.
 __host__ __device__ constexpr int solve_rows(int mode) { return (mode & (4 | 32) /*XINV, FINE*/) ? SOLB : SUBB; }
 // Edge of the blocks that the counters count, and of an update task's block
@@ -164,6 +172,7 @@ struct ExecParams {
     void *Y;                // MODE_XINV: forward results (layout of B): the substitutions
                             // read B and write Y (forward), read Y and write B (backward)
     int *xinvDone;          // MODE_XINV: TK_XINV(k) done
+    const double *cond;     // FP64 MODE_XINV: infinity norms of diagonal tile k and of its inverse at 2 k, 2 k + 1
     ExecState *st;
     const ExecState *after;     // state of an earlier launch: do nothing when that one failed (or null)
     TraceRec *trace;        // optional per-task trace (nullptr: off)

@@ -97,6 +97,9 @@ struct Dims {
     __device__ ViewT<T> XI(int k) const {
         return ViewT<T>{static_cast<T *>(p.xinv) + (int64_t)k * p.NB * p.NB, 1, p.NB};
     }
+    // Whether the full inverse of diagonal tile k is too inaccurate to solve with
+    // (FP64 MODE_XINV; NaN norms count).
+    __device__ bool ill(int k) const { return !(p.cond[2 * k] * p.cond[2 * k + 1] <= XINV_COND); }
 };
 
 // The counters a task waits on and the values they must reach (up to three;
@@ -299,6 +302,30 @@ __device__ __forceinline__ void solve_cols(int w, F &&f) {
     f(acc);
 }
 
+// Solve with diagonal tile t.k by its inverted 64 x 64 diagonal blocks (those
+// of its full inverse), from src into dst: strips of 8 columns, dealt out over
+// the tile's row-block tasks, which otherwise have a row block of the product
+// with the full inverse.
+__device__ __noinline__ void solve_strips(const Task &t, const Dims<double> &d, const View &src, const View &dst, int w,
+                                          double *smem) {
+    const int n = d.tm(t.k), ld = rec::strip_ld(n), np = ld - 4;
+    double *sR = smem + rec::SW * ld;
+    const View X = d.XI(t.k);
+    for (int c0 = t.sub * rec::SW; c0 < w; c0 += d.nsolve(t.k) * rec::SW) {
+        const int wc = min(rec::SW, w - c0);
+        for (int idx = threadIdx.x; idx < rec::SW * np; idx += NT_CTA) {
+            const int r = idx % np, c = idx / np;
+            smem[r + c * ld] = (r < n && c < wc) ? __ldcg(src.at(r, c0 + c)) : 0.0;
+        }
+        rec::strip_sweep<double, true>(d.A(t.k, t.k), n, X.p, smem, ld, sR, t.kind == TK_BWD_TRSM, (int)X.cs);
+        for (int idx = threadIdx.x; idx < rec::SW * np; idx += NT_CTA) {
+            const int r = idx % np, c = idx / np;
+            if (r < n && c < wc) *dst.at(r, c0 + c) = smem[r + c * ld];
+        }
+        __syncthreads();
+    }
+}
+
 template <class T, int SP, bool TC>
 __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T *smem, tc05::Smem *tsm,
                          uint8_t *stage, unsigned *ph, Ahead *ah) {
@@ -477,13 +504,23 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
             const int mr = min(SOLB, n - r0);
             const VT Xk = d.XI(t.k);
             const VT Yk = d.Yt(t.k, t.bn);
+            if constexpr (sizeof(T) == 8) {
+                if (d.ill(t.k)) {
+                    solve_strips(t, d, t.kind == TK_FWD_TRSM ? X : Yk, t.kind == TK_FWD_TRSM ? Yk : X, w, smem);
+                    break;
+                }
+            }
             auto apply = [&](auto &acc, int c0, int wc) {
                 acc.zero();
                 if (t.kind == TK_FWD_TRSM) {
                     cta_gemm(acc, Xk.sub(r0, 0), X.sub(0, c0).t(), mr, wc, r0 + mr, smem);
                     acc.store_to(Yk.sub(r0, c0), mr, wc);
                 } else {
-                    cta_gemm(acc, Xk.sub(r0, r0).t(), Yk.sub(r0, c0).t(), mr, wc, n - r0, smem);
+                    // (the diagonal block last: it holds the largest terms, and
+                    // every later addition would round at their size)
+                    const int r1 = r0 + mr;
+                    cta_gemm(acc, Xk.sub(r1, r0).t(), Yk.sub(r1, c0).t(), mr, wc, n - r1, smem);
+                    cta_gemm(acc, Xk.sub(r0, r0).t(), Yk.sub(r0, c0).t(), mr, wc, mr, smem);
                     acc.store_to(X.sub(r0, c0), mr, wc);
                 }
             };
@@ -652,6 +689,7 @@ template <class T, int SP, bool TC>
 constexpr size_t dag_smem_bytes() {
     // FP64: two CTAs per SM, each task within a 128 x 64 DMMA tile's stages
     if (sizeof(T) == 8 && !TC) {
+        static_assert(sizeof(T) == 4 || rec::strip_smem_elems(SOLVE_NB) <= Cfg12864<T, SP>::SMEM_ELEMS, "strips");
         static_assert(sizeof(T) == 4 || (size_t)rec::fused_smem_elems() <= Cfg12864<T, SP>::SMEM_ELEMS, "diagonal tile");
         return Cfg12864<T, SP>::SMEM_BYTES + 1024;
     }

@@ -593,14 +593,17 @@ static __device__ int tile_potrf_fused(const View &Tv, int n, double *invd, doub
 // the lower L.  The rows of L are used once per strip, so its MMA fragments
 // come straight from L2 into registers, the next ones in flight during the
 // products, and a 64-row step is two products and two barriers without a
-// global round trip of X.  FP32 operands are multiplied in FP64.  sR: SW x
-// LEAF_LD doubles.  All threads; starts and ends with a barrier.
+// global round trip of X.  FP32 operands are multiplied in FP64.
+// WITHIN: the blocks are those of a larger inverse with leading dimension ldi,
+// whose entries outside the matrix are not read (a variant of its own: the
+// guards on every call cost the batch 3%).  sR: SW x LEAF_LD doubles.  All
+// threads; starts and ends with a barrier.
 constexpr int SW = 8;
 __host__ __device__ constexpr int strip_ld(int n) { return (n + IB - 1) / IB * IB + 4; }   // 4 mod 16: no conflicts
 __host__ __device__ constexpr size_t strip_smem_elems(int n) { return (size_t)SW * (strip_ld(n) + LEAF_LD); }
-template <class T>
+template <class T, bool WITHIN = false>
 __device__ __noinline__ void strip_sweep(const ViewT<T> &L, int n, const T *invd, double *sX, int ld, double *sR,
-                                         bool trans) {
+                                         bool trans, int ldi = IB) {
     sX = in_shared(sX);
     sR = in_shared(sR);
     const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
@@ -611,10 +614,13 @@ __device__ __noinline__ void strip_sweep(const ViewT<T> &L, int n, const T *invd
         const int b = trans ? nblk - 1 - s : s, jb = b * IB;
         const bool live = jb + row < n;
         // fragments of the inverted diagonal block: independent of the sum below
-        const T *inv = invd + (int64_t)b * IB * IB;
+        const T *inv = invd + (WITHIN ? (int64_t)jb * (ldi + 1) : (int64_t)b * IB * IB);
         T iv[IB / 4];
 #pragma unroll
-        for (int q = 0; q < IB / 4; ++q) iv[q] = trans ? inv[4 * q + t + row * IB] : inv[row + (4 * q + t) * IB];
+        for (int q = 0; q < IB / 4; ++q) {
+            const int k = 4 * q + t, l = WITHIN ? ldi : IB;
+            iv[q] = (!WITHIN || (live && jb + k < n)) ? (trans ? inv[k + row * l] : inv[row + k * l]) : T(0);
+        }
         // rows jb .. of the sum over the columns solved so far
         const int k0 = trans ? jb + IB : 0, k1 = trans ? n : jb;
         const ViewT<T> Lr = trans ? L.sub(0, jb).t() : L.sub(jb, 0);   // (row, k)

@@ -5,9 +5,11 @@ import sys
 
 import numpy as np
 import pytest
+import scipy.linalg as sla
 
 pytestmark = pytest.mark.gpu
 EPS = np.finfo(np.float64).eps
+UPPER, LOWER = 121, 122
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 FRESH = """
@@ -31,3 +33,81 @@ def test_first_call_of_a_process(n, nb, nrhs):
     """The substitutions need more counters than the factorization, and no
     earlier call has grown the workspace."""
     subprocess.run([sys.executable, "-c", FRESH % (n, nb, nrhs)], cwd=ROOT, check=True, timeout=300)
+
+
+def kernel_matrix(n, length, nugget, seed):
+    """Covariance of a Gaussian kernel on sorted points: ill-conditioned diagonal tiles."""
+    x = np.sort(np.random.default_rng(seed).uniform(0, 1, n))
+    return np.exp(-0.5 * ((x[:, None] - x) / length) ** 2) + nugget * np.eye(n)
+
+
+def block_inverse(L, w=8):
+    """L^-1 by block rows of w, as the 64 x 64 leaf makes it."""
+    X = np.zeros_like(L)
+    for p in range(0, len(L), w):
+        q = slice(p, min(p + w, len(L)))
+        X[q, q] = sla.solve_triangular(L[q, q], np.eye(q.stop - p), lower=True)
+        X[q, :p] = -X[q, q] @ (L[q, :p] @ X[:p, :p])
+    return X
+
+
+def solve_by_blocks(L, B, h=64):
+    """L L^T X = B with explicit inverses of the h x h diagonal blocks alone."""
+    Y, n = B.copy(), len(L)
+    inv = [block_inverse(L[j:j + h, j:j + h]) for j in range(0, n, h)]
+    for j in range(0, n, h):
+        Y[j:j + h] = inv[j // h] @ (Y[j:j + h] - L[j:j + h, :j] @ Y[:j])
+    for j in reversed(range(0, n, h)):
+        Y[j:j + h] = inv[j // h].T @ (Y[j:j + h] - L[j + h:, j:j + h].T @ Y[j + h:])
+    return Y
+
+
+def backward_error(A, X, B):
+    return np.abs(B - A @ X).max() / (np.abs(A).sum(1).max() * np.abs(X).max())
+
+
+@pytest.mark.parametrize("n,nb,nrhs,uplo", [(512, 512, 3, LOWER), (700, 350, 40, UPPER), (1000, 384, 9, LOWER),
+                                            (3073, 512, 5, UPPER), (2048, 200, 70, LOWER)])
+@pytest.mark.parametrize("length,nugget", [(0.02, 1e-10), (0.1, 1e-8), (0.02, 1e-4)])
+def test_backward_error_of_ill_conditioned_potrs(cb, n, nb, nrhs, uplo, length, nugget):
+    """No further from backward stability than inverted 64 x 64 blocks are
+    (within 4 x: another order of the same sums), whatever the condition."""
+    A = kernel_matrix(n, length, nugget, n)
+    L = np.linalg.cholesky(A)
+    A = L @ L.T
+    B = A @ np.random.default_rng(nb).standard_normal((n, nrhs))
+    F = np.where(np.tri(n, dtype=bool), L, np.nan)
+    F = F if uplo == LOWER else F.T
+    dA, dB = cb.Desc.create(n, n, nb), cb.Desc.create(n, nrhs, nb)
+    dA.from_numpy(F)
+    dB.from_numpy(B)
+    assert cb.dpotrs_Tile(uplo, dA, dB) == 0
+    got, ref = backward_error(A, dB.to_numpy(), B), backward_error(A, solve_by_blocks(L, B), B)
+    assert got <= 4 * ref + 4 * EPS, (got, ref)
+
+
+@pytest.mark.parametrize("n", [2000, 3100, 4096])
+def test_backward_error_of_ill_conditioned_posv(cb, n):
+    A = kernel_matrix(n, 0.02, 1e-8, n)
+    B = A @ np.random.default_rng(n).standard_normal((n, 4))
+    dA, dB = cb.Desc.create(n, n, 512), cb.Desc.create(n, 4, 512)
+    dA.from_numpy(A)
+    dB.from_numpy(B)
+    assert cb.dposv_Tile(LOWER, dA, dB) == 0
+    got = backward_error(A, dB.to_numpy(), B)
+    ref = backward_error(A, solve_by_blocks(np.linalg.cholesky(A), B), B)
+    assert got <= 4 * ref + 4 * EPS, (got, ref)
+
+
+@pytest.mark.parametrize("uplo", [LOWER, UPPER])
+def test_nan_in_a_factor_reaches_the_solution_it_belongs_to(cb, uplo):
+    """A NaN in the last diagonal tile of the factor spoils that tile's rows and,
+    through the backward sweep, those above: no stale or partial result."""
+    n, nb = 1024, 256
+    L = np.linalg.cholesky(kernel_matrix(n, 0.02, 1e-2, 5))
+    L[n - 1, n - 1] = np.nan
+    dA, dB = cb.Desc.create(n, n, nb), cb.Desc.create(n, 2, nb)
+    dA.from_numpy(L if uplo == LOWER else L.T.copy())
+    dB.from_numpy(np.ones((n, 2)))
+    assert cb.dpotrs_Tile(uplo, dA, dB) == 0
+    assert np.isnan(dB.to_numpy()[n - 1]).all()
