@@ -571,37 +571,11 @@ __global__ void __launch_bounds__(NT_CTA, 2) xinv_pair_kernel(DiagTiles d, int h
 }
 
 // cond[2 k], cond[2 k + 1] = the infinity norms of diagonal tile k and of its
-// inverse (zeroed before): 64 rows of one tile per CTA, along the contiguous
-// direction.  The maxima are taken on the bits, where NaN is above Inf.
+// inverse (zeroed before): 64 rows of one tile per CTA.
 __global__ void __launch_bounds__(NT_CTA, 4) xinv_norm_kernel(DiagTiles d, double *X, double *cond) {
-    const int k = blockIdx.y, r0 = blockIdx.x * IB, n = min(IB, d.order(k) - r0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __shared__ double s_part[4][IB];
-    const View V[2] = {d.L(k), View{X + (int64_t)k * d.NB * d.NB, 1, d.NB}};
-    for (int m = 0; m < 2; ++m) {
-        long long top = 0;
-        if (V[m].rs == 1) {
-            const int r = threadIdx.x & (IB - 1), q = threadIdx.x / IB;
-            double s = 0.0;
-            if (r < n)
-#pragma unroll 8
-                for (int c = q; c <= r0 + r; c += 4) s += fabs(*V[m].at(r0 + r, c));
-            s_part[q][r] = s;
-            __syncthreads();
-            if (q == 0) top = __double_as_longlong(fabs((s + s_part[1][r]) + (s_part[2][r] + s_part[3][r])));
-            __syncthreads();
-        } else {
-            for (int r = warp; r < n; r += NT_CTA / 32) {
-                double s = 0.0;
-#pragma unroll 4
-                for (int c = lane; c <= r0 + r; c += 32) s += fabs(*V[m].at(r0 + r, c));
-                for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                top = max(top, __double_as_longlong(fabs(s)));
-            }
-        }
-        for (int o = 16; o; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-        if (lane == 0 && top) atomicMax(reinterpret_cast<long long *>(cond + 2 * k + m), top);
-    }
+    const int k = blockIdx.y, r0 = blockIdx.x * IB;
+    rec::lower_norms<IB>(d.L(k), View{X + (int64_t)k * d.NB * d.NB, 1, d.NB}, r0, min(IB, d.order(k) - r0), false,
+                         cond + 2 * k);
 }
 
 // The full inverses of all diagonal tiles into X (W: scratch of the same size),

@@ -9,7 +9,10 @@
 // of triangular operands, so that each does its n^3 / 3 operations:
 //   dtrtri: the inverted 64 x 64 diagonal blocks in one launch, then doubling:
 //           at block size h = 64, 128, ... every pair of neighbouring h-blocks
-//           gets X21 = -X22 (L21 X11), two launches for all pairs together;
+//           gets X21 = -X22 (L21 X11), two launches for all pairs together; a
+//           factor too ill-conditioned for that (INV_COND) by substitution,
+//           whose residual does not grow with the condition (order 2500: 0.59
+//           and 2.4 ms);
 //   dlauum: A(i,j) = sum_{k >= i} L(k,i) L(k,j), one launch;
 //   dpotri: dtrtri then dlauum, as LAPACK and the reference; the inverse of
 //           the factor stays in the workspace between the two (order 2500:
@@ -37,18 +40,59 @@ namespace chb {
 constexpr int HB = 64;
 using CfgInv = Cfg64<double>;
 constexpr int INV_CTAS_PER_SM = 3;
+constexpr size_t LEAF_BYTES = 2 * IB * LEAF_LD * sizeof(double);
 
-// X (column-major, ld ldx) gets the inverted HB x HB diagonal blocks of the
-// lower L (n x n), one CTA each; unit: with an implied unit diagonal.
-__global__ void __launch_bounds__(NT_CTA, 1) diag_inv_kernel(View L, int n, int unit, double *X, int64_t ldx) {
+// What is known of a triangular matrix and its inverse: its first zero diagonal
+// entry (1-based; INT_MAX: none) and the infinity norms of the two.
+//
+// Doubling keeps the residual X L - I of LAPACK's dtrtri, but L X - I grows with
+// the condition: restated on the host (kernel, Wishart, Laplacian matrices,
+// orders 512 and 1024), it is within 1.5 times a substitution's while the product
+// of the norms is below 64, 4 times at 5e2, 1e2 times at 4e4, 1e4 times at 1e6.
+// Beyond INV_COND (NaN included) the inverse is made by substitution instead.
+constexpr double INV_COND = 64.0;
+struct InvState {
+    int first;
+    double norm[2];
+    __host__ __device__ bool ill() const { return !(norm[0] * norm[1] <= INV_COND); }
+    __host__ __device__ bool usable() const { return first == INT_MAX && !ill(); }
+};
+constexpr int NORM_ROWS = 16;   // rows per CTA of the norms: 157 CTAs at order 2500
+
+// The inverted HB x HB diagonal blocks of the lower L (n x n), one CTA each, at
+// X + q step (column-major, ld ldx); unit: with an implied unit diagonal.
+__global__ void __launch_bounds__(NT_CTA, 1) diag_inv_kernel(View L, int n, int unit, double *X, int64_t ldx,
+                                                             int64_t step) {
     extern __shared__ __align__(128) double smem[];
     const int j0 = blockIdx.x * HB, nb = min(HB, n - j0);
     rec::leaf64_load(L.sub(j0, j0), nb, smem);
     double *sX = smem + 64 * rec::LDS;
     rec::leaf64_core<double, false>(smem, sX, nb, unit != 0);
-    double *D = X + j0 + (int64_t)j0 * ldx;
+    double *D = X + blockIdx.x * step;
     for (int idx = threadIdx.x; idx < nb * nb; idx += NT_CTA)
         D[idx % nb + (int64_t)(idx / nb) * ldx] = sX[idx % nb + (idx / nb) * rec::LDS];
+}
+
+// X (column-major, ld ldx) <- L^-1 (trans: L^-T) for the lower L by substitution
+// with its inverted diagonal blocks (HB x HB each, one after the other): strips
+// of SUBST_W columns, one CTA each, the longest first; only the rows in which a
+// strip of the result is not zero.  A strip is a chain of n / 64 products on one
+// SM, so it is narrow, with two CTAs per SM and a deep pipeline.
+constexpr int SUBST_W = 32;
+using CfgSubst = GemmCfg<double, 64, SUBST_W, 4, 2, SPLIT_BF16X3, 4>;
+__global__ void __launch_bounds__(NT_CTA, 2)
+    inv_subst_kernel(View L, int n, const double *invd, double *X, int64_t ldx, int trans) {
+    extern __shared__ __align__(128) double smem[];
+    const int c0 = (trans ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * SUBST_W, w = min(SUBST_W, n - c0);
+    const int b = c0 / HB, r0 = trans ? 0 : b * HB, m = trans ? min(n, (b + 1) * HB) : n - r0;
+    const View S = View{X, 1, ldx}.sub(0, c0);
+    for (int idx = threadIdx.x; idx < w * n; idx += NT_CTA) {
+        const int i = idx % n, j = idx / n;
+        *S.at(i, j) = i == c0 + j ? 1.0 : 0.0;
+    }
+    cta_sync_global();
+    trsm_left<double, SPLIT_BF16X3, CfgSubst>(S.sub(r0, 0), w, L.sub(r0, r0), m, invd + (int64_t)(r0 / HB) * HB * HB,
+                                              trans != 0, smem);
 }
 
 // One half of a doubling step on the pairs of h-blocks (rows [r, r + h2) below
@@ -81,11 +125,11 @@ __global__ void __launch_bounds__(NT_CTA, INV_CTAS_PER_SM)
 // C (lower triangle, n x n view) = X^T X for the lower X (column-major, ld
 // ldx): blocks of the lower triangle in row order, so that the longest sums
 // (k from the block's first row to n) start first.  Nothing is written when
-// *skip is a valid index (a singular factor).
+// st is given and its inverse is not to be used.
 __global__ void __launch_bounds__(NT_CTA, INV_CTAS_PER_SM)
-    lauum_kernel(View X, int n, View C, const int *skip) {
+    lauum_kernel(View X, int n, View C, const InvState *st) {
     extern __shared__ __align__(128) double smem[];
-    if (skip && *skip != INT_MAX) return;
+    if (st && !st->usable()) return;
     int bi = (int)((sqrtf(8.f * (float)blockIdx.x + 1.f) - 1.f) * 0.5f);
     while ((bi + 1) * (bi + 2) / 2 <= (int)blockIdx.x) ++bi;
     while (bi * (bi + 1) / 2 > (int)blockIdx.x) --bi;
@@ -101,11 +145,11 @@ __global__ void __launch_bounds__(NT_CTA, INV_CTAS_PER_SM)
 }
 
 // D <- the lower triangle of S (views of order n), zeros above it when
-// zero_upper; the diagonal is left out when skip_diag; nothing when *skip is a
-// valid index.  Block (x, y): 64 rows of 4 columns per step, along the
+// zero_upper; the diagonal is left out when skip_diag; nothing when st is given
+// and its inverse is not to be used.  Block (x, y): 64 rows of 4 columns per step, along the
 // destination's contiguous direction.
-__global__ void tri_copy_kernel(View S, View D, int n, int zero_upper, int skip_diag, const int *skip) {
-    if (skip && *skip != INT_MAX) return;
+__global__ void tri_copy_kernel(View S, View D, int n, int zero_upper, int skip_diag, const InvState *st) {
+    if (st && !st->usable()) return;
     const bool cm = D.rs == 1;
     for (int y = blockIdx.y; y < n; y += gridDim.y)
         for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
@@ -115,13 +159,16 @@ __global__ void tri_copy_kernel(View S, View D, int n, int zero_upper, int skip_
         }
 }
 
-// *first = min over i of (i + 1) with A(i,i) == 0 (INT_MAX: none).
-__global__ void flag_kernel(int *first) {
-    if (threadIdx.x == 0) *first = INT_MAX;
-}
-__global__ void zero_diag_kernel(View A, int N, int *first) {
+__global__ void inv_state_kernel(InvState *st) { *st = InvState{INT_MAX, {0.0, 0.0}}; }
+// st->first = min over i of (i + 1) with A(i,i) == 0.
+__global__ void zero_diag_kernel(View A, int N, InvState *st) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
-        if (*A.at(i, i) == 0.0) atomicMin(first, i + 1);
+        if (*A.at(i, i) == 0.0) atomicMin(&st->first, i + 1);
+}
+// st->norm = the infinity norms of L and of its inverse X.
+__global__ void __launch_bounds__(NT_CTA, 4) inv_norm_kernel(View L, View X, int n, int unit, InvState *st) {
+    const int r0 = (gridDim.x - 1 - blockIdx.x) * NORM_ROWS;   // the longest rows first
+    rec::lower_norms<NORM_ROWS>(L, X, r0, min(NORM_ROWS, n - r0), unit != 0, st->norm);
 }
 
 namespace {
@@ -134,9 +181,9 @@ cublasHandle_t lib_handle() {
     return h;
 }
 
-double *g_w1 = nullptr, *g_w2 = nullptr, *g_w3 = nullptr, *g_w4 = nullptr;
-size_t g_w1_bytes = 0, g_w2_bytes = 0, g_w3_bytes = 0, g_w4_bytes = 0;
-int *g_flag = nullptr;
+double *g_w1 = nullptr, *g_w2 = nullptr, *g_w3 = nullptr, *g_w4 = nullptr, *g_w5 = nullptr;
+size_t g_w1_bytes = 0, g_w2_bytes = 0, g_w3_bytes = 0, g_w4_bytes = 0, g_w5_bytes = 0;
+InvState *g_state = nullptr;
 
 double *work(double **buf, size_t *cap, size_t bytes) {
     if (bytes > *cap) {
@@ -160,15 +207,16 @@ static int inv_attrs() {
     if (done) return 0;
     CHB_CUDA(cudaFuncSetAttribute(trtri_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgInv::SMEM_BYTES));
     CHB_CUDA(cudaFuncSetAttribute(lauum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgInv::SMEM_BYTES));
+    CHB_CUDA(cudaFuncSetAttribute(inv_subst_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CfgSubst::SMEM_BYTES));
     CHB_CUDA(cudaFuncSetAttribute(diag_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * IB * LEAF_LD * sizeof(double))));
+                                  (int)LEAF_BYTES));
     done = true;
     return 0;
 }
 
-static void tri_copy(View S, View D, int N, int zero_upper, int skip_diag, const int *skip, cudaStream_t s) {
+static void tri_copy(View S, View D, int N, int zero_upper, int skip_diag, const InvState *st, cudaStream_t s) {
     const dim3 grid((N + 255) / 256, std::min(N, 2048));
-    tri_copy_kernel<<<grid, 256, 0, s>>>(S, D, N, zero_upper, skip_diag, skip);
+    tri_copy_kernel<<<grid, 256, 0, s>>>(S, D, N, zero_upper, skip_diag, st);
     CHB_LAUNCHED(1);
 }
 
@@ -176,24 +224,24 @@ static void tri_copy(View S, View D, int N, int zero_upper, int skip_diag, const
 // and not a multiple of a power of two for the common orders.
 static int64_t work_ld(int N) { return (N + 1) / 2 * 2 + 2; }
 
-// The inverse of the lower L (view of order N) into the first workspace
-// (column-major, ld work_ld(N), zeros above the diagonal of every HB-block);
-// g_flag = the first zero diagonal entry (INT_MAX: none, or unit).  Stream
-// operations only; returns the workspace.
+// The inverse of the lower L (view of order N) by doubling into the first
+// workspace (column-major, ld work_ld(N), zeros above the diagonal of every
+// HB-block), and g_state.  Stream operations only; returns the workspace.
 static int trtri_work(View L, cham_diag_t diag, int N, cudaStream_t s, double **Xp) {
     if (int rc = inv_attrs()) return rc;
-    if (!g_flag && !(g_flag = (int *)dev_alloc(sizeof(int)))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+    if (!g_state && !(g_state = (InvState *)dev_alloc(sizeof(InvState)))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
     const int64_t ld = work_ld(N);
+    const bool unit = diag == ChamUnit;
     double *X = work(&g_w1, &g_w1_bytes, (size_t)ld * N * sizeof(double));
     double *T = N > HB ? work(&g_w2, &g_w2_bytes, (size_t)ld * N * sizeof(double)) : X;
     if (!X || !T) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-    flag_kernel<<<1, 32, 0, s>>>(g_flag);
+    inv_state_kernel<<<1, 1, 0, s>>>(g_state);
     CHB_LAUNCHED(1);
-    if (diag == ChamNonUnit) {
-        zero_diag_kernel<<<grid_for(N), 256, 0, s>>>(L, N, g_flag);
+    if (!unit) {
+        zero_diag_kernel<<<grid_for(N), 256, 0, s>>>(L, N, g_state);
         CHB_LAUNCHED(1);
     }
-    diag_inv_kernel<<<(N + HB - 1) / HB, NT_CTA, 2 * IB * LEAF_LD * sizeof(double), s>>>(L, N, diag == ChamUnit, X, ld);
+    diag_inv_kernel<<<(N + HB - 1) / HB, NT_CTA, LEAF_BYTES, s>>>(L, N, unit, X, ld, HB * (ld + 1));
     CHB_LAUNCHED(1);
     for (int64_t h = HB; h < N; h *= 2) {
         // pairs with any rows in their second block
@@ -202,28 +250,72 @@ static int trtri_work(View L, cham_diag_t diag, int N, cudaStream_t s, double **
             trtri_pair_kernel<<<dim3(nb, nb, pairs), NT_CTA, CfgInv::SMEM_BYTES, s>>>(L, N, (int)h, X, T, ld, first);
         CHB_LAUNCHED(2);
     }
+    inv_norm_kernel<<<(N + NORM_ROWS - 1) / NORM_ROWS, NT_CTA, 0, s>>>(L, View{X, 1, ld}, N, unit, g_state);
+    CHB_LAUNCHED(1);
     CHB_CUDA(cudaGetLastError());
     *Xp = X;
     return 0;
 }
 
-static int read_flag(int *first, cudaStream_t s) {
-    CHB_CUDA(cudaMemcpyAsync(first, g_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+// The same inverse by substitution, as a lower view on the first workspace.
+// For an upper matrix U = L^T it is U X = I that is solved, as for a lower one.
+static int trtri_subst(cham_uplo_t uplo, View L, cham_diag_t diag, int N, cudaStream_t s, View *Xv) {
+    if (int rc = inv_attrs()) return rc;
+    const int64_t ld = work_ld(N);
+    const int nb = (N + HB - 1) / HB, upper = uplo == ChamUpper;
+    double *X = work(&g_w1, &g_w1_bytes, (size_t)ld * N * sizeof(double));
+    double *invd = work(&g_w5, &g_w5_bytes, (size_t)nb * HB * HB * sizeof(double));
+    if (!X || !invd) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+    diag_inv_kernel<<<nb, NT_CTA, LEAF_BYTES, s>>>(L, N, diag == ChamUnit, invd, HB, HB * HB);
+    inv_subst_kernel<<<(N + SUBST_W - 1) / SUBST_W, NT_CTA, CfgSubst::SMEM_BYTES, s>>>(L, N, invd, X, ld, upper);
+    CHB_LAUNCHED(2);
+    CHB_CUDA(cudaGetLastError());
+    *Xv = upper ? View{X, ld, 1} : View{X, 1, ld};
+    return 0;
+}
+
+static int read_state(InvState *st, cudaStream_t s) {
+    CHB_CUDA(cudaMemcpyAsync(st, g_state, sizeof(InvState), cudaMemcpyDeviceToHost, s));
     CHB_CUDA(cudaStreamSynchronize(s));
     return 0;
 }
 
+static void lauum_launch(View X, int N, View C, const InvState *st, cudaStream_t s) {
+    const int nb = (N + HB - 1) / HB;
+    lauum_kernel<<<nb * (nb + 1) / 2, NT_CTA, CfgInv::SMEM_BYTES, s>>>(X, N, C, st);
+    CHB_LAUNCHED(1);
+}
+
 // The three operations on a device column-major A (ld lda), on the library
 // stream; synchronous.  Return LAPACK's info (> 0) or a CHAMELEON_ERR_* code.
+//
+// dtrtri (potri: then dlauum): finish(X, st) writes the result from the lower
+// inverse X, unless st says that it is not to be used.  The inverse by doubling
+// is finished at once; what the host reads at the end decides whether that has
+// happened, or A is singular (not modified), or the substitution has to run.
+template <class Finish>
+static int invert(cham_uplo_t uplo, cham_diag_t diag, int N, double *A, int lda, Finish finish) {
+    cudaStream_t s = ctx().stream;
+    double *X = nullptr;
+    if (int rc = trtri_work(lower_view(uplo, A, lda), diag, N, s, &X)) return rc;
+    finish(View{X, 1, work_ld(N)}, g_state);
+    InvState st;
+    if (int rc = read_state(&st, s)) return rc;
+    if (st.first != INT_MAX) return st.first;
+    if (!st.ill()) return 0;
+    View Xv;
+    if (int rc = trtri_subst(uplo, lower_view(uplo, A, lda), diag, N, s, &Xv)) return rc;
+    finish(Xv, nullptr);
+    CHB_CUDA(cudaGetLastError());
+    CHB_CUDA(cudaStreamSynchronize(s));
+    return 0;
+}
+
 int trtri_dev(cham_uplo_t uplo, cham_diag_t diag, int N, double *A, int lda) {
     cudaStream_t s = ctx().stream;
-    const View L = lower_view(uplo, A, lda);
-    double *X = nullptr;
-    if (int rc = trtri_work(L, diag, N, s, &X)) return rc;
-    tri_copy(View{X, 1, work_ld(N)}, L, N, 0, diag == ChamUnit, g_flag, s);
-    int first = INT_MAX;
-    if (int rc = read_flag(&first, s)) return rc;
-    return first != INT_MAX ? first : 0;   // singular: A is not modified
+    return invert(uplo, diag, N, A, lda, [&](View X, const InvState *st) {
+        tri_copy(X, lower_view(uplo, A, lda), N, 0, diag == ChamUnit, st, s);
+    });
 }
 
 int lauum_dev(cham_uplo_t uplo, int N, double *A, int lda) {
@@ -234,9 +326,7 @@ int lauum_dev(cham_uplo_t uplo, int N, double *A, int lda) {
     double *T = work(&g_w1, &g_w1_bytes, (size_t)ld * N * sizeof(double));
     if (!T) return CHAMELEON_ERR_OUT_OF_RESOURCES;
     tri_copy(L, View{T, 1, ld}, N, 1, 0, nullptr, s);
-    const int nb = (N + HB - 1) / HB;
-    lauum_kernel<<<nb * (nb + 1) / 2, NT_CTA, CfgInv::SMEM_BYTES, s>>>(View{T, 1, ld}, N, L, nullptr);
-    CHB_LAUNCHED(1);
+    lauum_launch(View{T, 1, ld}, N, L, nullptr, s);
     CHB_CUDA(cudaGetLastError());
     CHB_CUDA(cudaStreamSynchronize(s));
     return 0;
@@ -244,16 +334,9 @@ int lauum_dev(cham_uplo_t uplo, int N, double *A, int lda) {
 
 int potri_dev(cham_uplo_t uplo, int N, double *A, int lda) {
     cudaStream_t s = ctx().stream;
-    const View L = lower_view(uplo, A, lda);
-    double *X = nullptr;
-    if (int rc = trtri_work(L, ChamNonUnit, N, s, &X)) return rc;
-    const int nb = (N + HB - 1) / HB;
-    lauum_kernel<<<nb * (nb + 1) / 2, NT_CTA, CfgInv::SMEM_BYTES, s>>>(View{X, 1, work_ld(N)}, N, L, g_flag);
-    CHB_LAUNCHED(1);
-    CHB_CUDA(cudaGetLastError());
-    int first = INT_MAX;
-    if (int rc = read_flag(&first, s)) return rc;
-    return first != INT_MAX ? first : 0;   // singular: A is not modified
+    return invert(uplo, ChamNonUnit, N, A, lda, [&](View X, const InvState *st) {
+        lauum_launch(X, N, lower_view(uplo, A, lda), st, s);
+    });
 }
 
 // S (N x N, ld N) <- the symmetric matrix whose uplo triangle is in A.

@@ -657,6 +657,55 @@ __device__ __noinline__ void strip_sweep(const ViewT<T> &L, int n, const T *invd
     }
 }
 
+// The largest sum of absolute values of rows r0 .. r0 + n - 1 (n <= R) of the
+// lower V (unit: with an implied unit diagonal), along the contiguous
+// direction, as the bits of a double: maxima are taken on the bits, where NaN is
+// above Inf.  The whole CTA; valid in every warp's lane 0 for what that warp
+// has seen.
+template <int R>
+__device__ inline long long lower_row_norm(const View &V, int r0, int n, bool unit) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int Q = NT_CTA / R;
+    __shared__ double s_part[Q][R];
+    long long top = 0;
+    const int skip = unit ? 1 : 0;
+    if (V.rs == 1) {
+        const int r = threadIdx.x % R, q = threadIdx.x / R;
+        double s = (unit && q == 0) ? 1.0 : 0.0;
+        if (r < n)
+#pragma unroll 8
+            for (int c = q; c <= r0 + r - skip; c += Q) s += fabs(*V.at(r0 + r, c));
+        s_part[q][r] = s;
+        __syncthreads();
+        if (q == 0 && r < n) {
+#pragma unroll
+            for (int i = 1; i < Q; ++i) s += s_part[i][r];
+            top = __double_as_longlong(fabs(s));
+        }
+        __syncthreads();
+    } else {
+        for (int r = warp; r < n; r += NT_CTA / 32) {
+            double s = (unit && lane == 0) ? 1.0 : 0.0;
+#pragma unroll 8
+            for (int c = lane; c <= r0 + r - skip; c += 32) s += fabs(*V.at(r0 + r, c));
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            top = max(top, __double_as_longlong(fabs(s)));
+        }
+    }
+    for (int o = 16; o; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    return top;
+}
+// norm[0], norm[1] = the infinity norms of the lower L and of its inverse X
+// (zeroed before), R rows per CTA.
+template <int R>
+__device__ inline void lower_norms(const View &L, const View &X, int r0, int n, bool unit, double *norm) {
+#pragma unroll 1
+    for (int m = 0; m < 2; ++m) {
+        const long long top = lower_row_norm<R>(m ? X : L, r0, n, unit && m == 0);
+        if ((threadIdx.x & 31) == 0 && top) atomicMax(reinterpret_cast<long long *>(norm + m), top);
+    }
+}
+
 // Inverted 64 x 64 diagonal blocks of an existing lower factor (n x n), for
 // the solve-only executor mode.
 template <class T>

@@ -12,6 +12,7 @@ import ctypes
 
 import numpy as np
 import pytest
+import scipy.linalg as sla
 
 pytestmark = pytest.mark.gpu
 
@@ -253,3 +254,47 @@ def test_dpotrimm_lapack_and_tile(cb, orc, uplo, N):
         Ab = np.asfortranarray(A.copy())
         Ab[N // 2, N // 2] = -1.0
         assert L.CHAMELEON_dpotrimm(uplo, N, cb._addr(Ab), N, cb._addr(Bw), N, cb._addr(C), N) == N // 2 + 1
+
+
+def kernel_factor(n, length, nugget):
+    x = np.sort(np.random.default_rng(n).uniform(0, 1, n))
+    return np.linalg.cholesky(np.exp(-0.5 * ((x[:, None] - x) / length) ** 2) + nugget * np.eye(n))
+
+
+def substitution(T, upper, h=64, w=8):
+    """T X = I by substitution with inverted h x h diagonal blocks (made by block rows of w)."""
+    n = len(T)
+    X = np.eye(n)
+    for j in (reversed(range(0, n, h)) if upper else range(0, n, h)):
+        b = slice(j, min(j + h, n))
+        D = T[b, b].T.copy() if upper else T[b, b].copy()
+        I = np.zeros_like(D)
+        for p in range(0, len(D), w):
+            q = slice(p, min(p + w, len(D)))
+            I[q, q] = sla.solve_triangular(D[q, q], np.eye(q.stop - p), lower=True)
+            I[q, :p] = -I[q, q] @ (D[q, :p] @ I[:p, :p])
+        rest = slice(b.stop, n) if upper else slice(0, j)
+        X[b] = (I.T if upper else I) @ (X[b] - T[b, rest] @ X[rest])
+    return np.triu(X) if upper else np.tril(X)
+
+
+@pytest.mark.parametrize("uplo", [UPPER, LOWER])
+@pytest.mark.parametrize("N", [200, 512, 1000, 2500])
+@pytest.mark.parametrize("length,nugget", [(0.02, 1e-10), (0.1, 1e-8), (0.02, 1e-4)])
+def test_inverses_of_ill_conditioned_factors(cb, uplo, N, length, nugget):
+    """Residuals no larger than a substitution's (within 4 x: another order of
+    the same sums), whatever the condition: T X - I of dtrtri, and A A^-1 - I
+    of dpotri."""
+    L = kernel_factor(N, length, nugget)
+    T = L if uplo == LOWER else np.ascontiguousarray(L.T)
+    A = L @ L.T
+    size = lambda R: np.abs(R).sum(1).max()
+    ref = substitution(T, uplo == UPPER)
+    W = np.asfortranarray(T.copy())
+    assert cb.dtrtri(uplo, NONUNIT, N, W, N) == 0
+    assert size(T @ tri(uplo)(W) - np.eye(N)) <= 4 * size(T @ ref - np.eye(N)) + 4 * N * EPS
+    W = np.asfortranarray(T.copy())
+    assert cb.dpotri(uplo, N, W, N) == 0
+    full = lambda X: X + (np.tril(X, -1).T if uplo == LOWER else np.triu(X, 1).T)
+    P, R = full(tri(uplo)(W)), full(tri(uplo)(ref.T @ ref if uplo == LOWER else ref @ ref.T))
+    assert size(A @ P - np.eye(N)) <= 4 * size(A @ R - np.eye(N)) + 4 * N * EPS
