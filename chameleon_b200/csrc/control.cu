@@ -162,10 +162,21 @@ int pool_device() {
     return d >= 0 ? d : ctx().device;
 }
 
+// Upper bound of the pool's memory in use (CHAM_B200_Workspace_Limit).
+static std::atomic<uint64_t> g_ws_limit{~0ull};
+static uint64_t pool_used(cudaMemPool_t pool) {
+    uint64_t used = 0;
+    cudaStreamSynchronize(meta_stream());   // releases on it count once they are done
+    if (pool) cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    return used;
+}
+
 void *dev_alloc(size_t bytes) {
     void *p = nullptr;
     cudaStream_t ms = meta_stream();
     cudaMemPool_t pool = lib_pool();
+    const uint64_t limit = g_ws_limit;
+    if (limit != ~0ull && pool_used(pool) + bytes > limit) return nullptr;
     const cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 16), pool, ms)
                                : cudaMallocAsync(&p, std::max<size_t>(bytes, 16), ms);
     if (e != cudaSuccess) {
@@ -1020,6 +1031,13 @@ int CHAM_B200_dposv_timed(cham_uplo_t uplo, int N, int NRHS, double *A, int LDA,
     int rc = ensure_init();
     if (rc) return rc;
     return lapack_call(MODE_FACT | MODE_SOLVE, uplo, N, NRHS, A, LDA, B, LDB, device_ms);
+}
+
+// Workspaces may grow by at most `extra` bytes from what they use now (negative:
+// no limit); a request beyond it fails as an exhausted device's would.
+int CHAM_B200_Workspace_Limit(long long extra) {
+    g_ws_limit = extra < 0 ? ~0ull : pool_used(lib_pool()) + (uint64_t)extra;
+    return 0;
 }
 
 // ---- measurement hooks (benchmark) ------------------------------------------

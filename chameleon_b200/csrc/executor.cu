@@ -635,6 +635,11 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     q.NTB = nrhs ? B->nt : 0;
     q.b_c = 1;
     if (xnb > 0) {
+        // column blocks twice as wide read the factor half as often, from about
+        // 1024 columns on, where the blocks alone fill the chip (us at order 3000
+        // and 8192, 32 or 64 wide: 512 columns 934 or 1194, 4244 or 3764; 1024
+        // columns 1342 or 1353, 8005 or 6447; 4096 columns 4508 or 3517, 31066
+        // or 23950)
         const int want = nrhs <= 1024 ? SOLVE_NBB : 2 * SOLVE_NBB;
         if (B->cols1 || B->nb % want == 0) {
             q.b_c = B->cols1 ? (nrhs + want - 1) / want : B->nb / want;
@@ -713,16 +718,17 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     return q;
 }
 
-// The launches of one call (1 or 2); ws: what they need together.
+// The launches of one call (1 or 2); ws: what they need together.  small: the
+// form with the least workspace (no array of B's size, no tile inverses in FP64).
 static int plan_call(Plan (&q)[2], WsBytes &ws, int mode, int N, bool f32, const Tiling &A, const Tiling *B, int nrhs,
-                     size_t b_elems, int split, int grid_req, const CastIn *cin, bool reuse) {
+                     size_t b_elems, int split, int grid_req, const CastIn *cin, bool reuse, bool small) {
     // FP64 substitutions above one executor tile: a launch of their own, after
     // the factorization's (which it checks on the device).  With a
     // factorization of a small matrix they stay in its launch, where the
     // forward sweep runs beside it (dposv 203: 232 us in one launch, 256 in
     // two; 2048: 1.70 and 1.73 ms; 5003: 6.16 and 5.95 ms).
     const bool own = (mode & MODE_FACT) ? N > 3072 : N > EXEC_NB;
-    const int xnb = (!f32 && !t_given && nrhs > 0 && own) ? solve_tile(N, A, *B) : 0;
+    const int xnb = (!f32 && !t_given && nrhs > 0 && own && !small) ? solve_tile(N, A, *B) : 0;
     int n = 0;
     if (xnb > 0) {
         if (mode & MODE_FACT)
@@ -849,15 +855,28 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
                        w.xinv_nb == A->nb && w.xinv_n == N;
     const Tiling tA = tiling(A), tB = B ? tiling(B) : Tiling{};
     const size_t b_elems = nrhs ? (size_t)(priv(B)->cm_view ? B->lda : B->lm) * B->ln : 0;
-    Plan q[2];
-    WsBytes need;
-    const int nq = plan_call(q, need, mode, N, f32, tA, B ? &tB : nullptr, nrhs, b_elems, split, grid_req, cin, reuse);
     // task lists, memory and tables of every launch before the first one
     // starts: none of them may be replaced while a launch still uses it
+    Plan q[2];
     const Schedule *sch[2] = {};
-    for (int i = 0; i < nq; ++i)
-        if (!(sch[i] = t_given ? t_given : get_schedule(q[i].sh))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
-    int rc = ensure_ws(w, need);
+    int nq = 0;
+    auto prepare = [&](bool small) -> int {
+        WsBytes need;
+        nq = plan_call(q, need, mode, N, f32, tA, B ? &tB : nullptr, nrhs, b_elems, split, grid_req, cin, reuse, small);
+        for (int i = 0; i < nq; ++i)
+            if (!(sch[i] = t_given ? t_given : get_schedule(q[i].sh))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
+        return ensure_ws(w, need);
+    };
+    int rc = prepare(false);
+    if (rc == CHAMELEON_ERR_OUT_OF_RESOURCES && q[nq - 1].xnb > 0) {
+        // without the workspace of the FP64 tile inverses, and with its memory
+        dev_free(w.xinv);
+        dev_free(w.y);
+        w.xinv = w.y = nullptr;
+        w.xinv_bytes = w.y_bytes = 0;
+        w.xinv_owner = nullptr;
+        rc = prepare(true);
+    }
     if (!rc) rc = desc_upload(A);
     if (!rc && nrhs) rc = desc_upload(B);
     if (rc) return rc;
@@ -1039,7 +1058,7 @@ extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs,
     Plan q[2];
     WsBytes r;
     const int n = plan_call(q, r, mode, N, false, A, nrhs > 0 ? &B : nullptr, nrhs, (size_t)N * std::max(nrhs, 0), 0, 0,
-                            nullptr, false);
+                            nullptr, false, false);
     for (int i = 0; i < n; ++i) {
         const int64_t v[7] = {q[i].NB, q[i].NBB, (int64_t)q[i].ws.ctr, (int64_t)q[i].ws.inv, (int64_t)q[i].ws.xinv,
                               (int64_t)q[i].ws.y, q[i].mode};

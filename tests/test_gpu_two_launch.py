@@ -28,11 +28,48 @@ assert r <= 8 * n * np.finfo(float).eps, r
 """
 
 
+def run_fresh(code):
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True, timeout=300)
+
+
 @pytest.mark.parametrize("n,nb,nrhs", [(3144, 262, 64), (3200, 200, 900)])
 def test_first_call_of_a_process(n, nb, nrhs):
     """The substitutions need more counters than the factorization, and no
     earlier call has grown the workspace."""
-    subprocess.run([sys.executable, "-c", FRESH % (n, nb, nrhs)], cwd=ROOT, check=True, timeout=300)
+    run_fresh(FRESH % (n, nb, nrhs))
+
+
+SCARCE = """
+import numpy as np, chameleon_b200 as cb
+n, nb, nrhs, mib, potrs, want = %r
+cb.init()
+g = np.random.default_rng(n)
+A0 = g.uniform(-0.5, 0.5, (n, n)); A0 = A0 + A0.T + n * np.eye(n)
+B0 = g.uniform(-0.5, 0.5, (n, nrhs))
+dA, dB = cb.Desc.create(n, n, nb), cb.Desc.create(n, nrhs, nb)
+dA.from_numpy(A0); dB.from_numpy(B0)
+if potrs:
+    assert cb.dpotrf_Tile(cb.ChamLower, dA) == 0
+L = cb.lib()
+L.CHAM_B200_Workspace_Limit(int(mib * 2**20))
+rc = (cb.dpotrs_Tile if potrs else cb.dposv_Tile)(cb.ChamLower, dA, dB)
+assert rc == want, rc
+L.CHAM_B200_Workspace_Limit(-1)
+if want:   # nothing was started
+    assert np.array_equal(dB.to_numpy(), B0) and (potrs or np.array_equal(dA.to_numpy(), A0))
+    assert (cb.dpotrs_Tile if potrs else cb.dposv_Tile)(cb.ChamLower, dA, dB) == 0
+X = dB.to_numpy()
+r = np.linalg.norm(B0 - A0 @ X) / (np.linalg.norm(A0) * np.linalg.norm(X))
+assert r <= 8 * n * np.finfo(float).eps, r
+"""
+
+
+@pytest.mark.parametrize("potrs", [False, True])
+@pytest.mark.parametrize("mib,want", [(8, 0), (0.01, -106)])
+def test_little_memory(mib, want, potrs):
+    """Tile inverses and forward results take 35 MiB here: without them the call
+    runs as one launch, and without room for that it leaves A and B alone."""
+    run_fresh(SCARCE % ((3200, 200, 1000, mib, potrs, want),))
 
 
 def kernel_matrix(n, length, nugget, seed):
