@@ -226,21 +226,23 @@ static int64_t work_ld(int N) { return (N + 1) / 2 * 2 + 2; }
 
 // The inverse of the lower L (view of order N) by doubling into the first
 // workspace (column-major, ld work_ld(N), zeros above the diagonal of every
-// HB-block), and g_state.  Stream operations only; returns the workspace.
+// HB-block), and g_state.  Returns the workspace, null when there is no memory
+// for the two that doubling needs (g_state then has the first zero alone).
 static int trtri_work(View L, cham_diag_t diag, int N, cudaStream_t s, double **Xp) {
     if (int rc = inv_attrs()) return rc;
     if (!g_state && !(g_state = (InvState *)dev_alloc(sizeof(InvState)))) return CHAMELEON_ERR_OUT_OF_RESOURCES;
     const int64_t ld = work_ld(N);
     const bool unit = diag == ChamUnit;
-    double *X = work(&g_w1, &g_w1_bytes, (size_t)ld * N * sizeof(double));
-    double *T = N > HB ? work(&g_w2, &g_w2_bytes, (size_t)ld * N * sizeof(double)) : X;
-    if (!X || !T) return CHAMELEON_ERR_OUT_OF_RESOURCES;
     inv_state_kernel<<<1, 1, 0, s>>>(g_state);
     CHB_LAUNCHED(1);
     if (!unit) {
         zero_diag_kernel<<<grid_for(N), 256, 0, s>>>(L, N, g_state);
         CHB_LAUNCHED(1);
     }
+    double *X = work(&g_w1, &g_w1_bytes, (size_t)ld * N * sizeof(double));
+    double *T = N > HB ? work(&g_w2, &g_w2_bytes, (size_t)ld * N * sizeof(double)) : X;
+    *Xp = nullptr;
+    if (!X || !T) return 0;
     diag_inv_kernel<<<(N + HB - 1) / HB, NT_CTA, LEAF_BYTES, s>>>(L, N, unit, X, ld, HB * (ld + 1));
     CHB_LAUNCHED(1);
     for (int64_t h = HB; h < N; h *= 2) {
@@ -292,17 +294,18 @@ static void lauum_launch(View X, int N, View C, const InvState *st, cudaStream_t
 // dtrtri (potri: then dlauum): finish(X, st) writes the result from the lower
 // inverse X, unless st says that it is not to be used.  The inverse by doubling
 // is finished at once; what the host reads at the end decides whether that has
-// happened, or A is singular (not modified), or the substitution has to run.
+// happened, or A is singular (not modified), or the substitution has to run,
+// which also serves when there is memory for one workspace only.
 template <class Finish>
 static int invert(cham_uplo_t uplo, cham_diag_t diag, int N, double *A, int lda, Finish finish) {
     cudaStream_t s = ctx().stream;
     double *X = nullptr;
     if (int rc = trtri_work(lower_view(uplo, A, lda), diag, N, s, &X)) return rc;
-    finish(View{X, 1, work_ld(N)}, g_state);
+    if (X) finish(View{X, 1, work_ld(N)}, g_state);
     InvState st;
     if (int rc = read_state(&st, s)) return rc;
     if (st.first != INT_MAX) return st.first;
-    if (!st.ill()) return 0;
+    if (X && !st.ill()) return 0;
     View Xv;
     if (int rc = trtri_subst(uplo, lower_view(uplo, A, lda), diag, N, s, &Xv)) return rc;
     finish(Xv, nullptr);

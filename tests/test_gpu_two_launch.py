@@ -72,6 +72,37 @@ def test_little_memory(mib, want, potrs):
     run_fresh(SCARCE % ((3200, 200, 1000, mib, potrs, want),))
 
 
+SCARCE_INVERSE = """
+import numpy as np, torch, chameleon_b200 as cb
+n = 1500
+cb.init()
+T = np.tril(np.random.default_rng(n).uniform(-0.5, 0.5, (n, n)) / n) + np.eye(n)
+for uplo, F in ((cb.ChamLower, T), (cb.ChamUpper, T.T)):
+    R = np.linalg.inv(F)
+    W = np.asfortranarray(F.copy())
+    cb.dlauum(uplo, 8, np.eye(8, order="F"), 8)      # the context's first allocations
+    V = np.asfortranarray(F.copy())
+    S = np.asfortranarray(F.copy()); S[700, 700] = 0.0
+    dev = [torch.from_numpy(a.T.copy()).cuda() for a in (W, V, S)]
+    cb.lib().CHAM_B200_Workspace_Limit(24 << 20)     # one N x N workspace (18 MiB), not two
+    assert cb.dtrtri(uplo, cb.ChamNonUnit, n, dev[0], n) == 0
+    assert cb.dpotri(uplo, n, dev[1], n) == 0
+    assert cb.dtrtri(uplo, cb.ChamNonUnit, n, dev[2], n) == 701
+    cb.lib().CHAM_B200_Workspace_Limit(-1)
+    W, V, Z = (d.cpu().numpy().T for d in dev)
+    tri = np.tril if uplo == cb.ChamLower else np.triu
+    bound = 8 * n * np.finfo(float).eps
+    assert np.abs(W - F + tri(F) - tri(R)).max() <= bound
+    P = R.T @ R if uplo == cb.ChamLower else R @ R.T
+    assert np.abs(tri(V) - tri(P)).max() <= bound * 4
+    assert np.array_equal(Z, S)
+"""
+
+
+def test_inverses_with_one_workspace():
+    run_fresh(SCARCE_INVERSE)
+
+
 def kernel_matrix(n, length, nugget, seed):
     """Covariance of a Gaussian kernel on sorted points: ill-conditioned diagonal tiles."""
     x = np.sort(np.random.default_rng(seed).uniform(0, 1, n))
