@@ -306,8 +306,8 @@ __device__ __forceinline__ void solve_cols(int w, F &&f) {
 // of its full inverse), from src into dst: strips of 8 columns, dealt out over
 // the tile's row-block tasks, which otherwise have a row block of the product
 // with the full inverse.
-__device__ __noinline__ void solve_strips(const Task &t, const Dims<double> &d, const View &src, const View &dst, int w,
-                                          double *smem) {
+static __device__ __noinline__ void solve_strips(const Task &t, const Dims<double> &d, const View &src, const View &dst,
+                                                 int w, double *smem) {
     const int n = d.tm(t.k), ld = rec::strip_ld(n), np = ld - 4;
     double *sR = smem + rec::SW * ld;
     const View X = d.XI(t.k);
