@@ -417,19 +417,20 @@ __device__ __forceinline__ void mma_stage(Acc<C> &acc, const typename C::T *sA, 
     }
 }
 
-template <class C, bool AK, bool BK>
+template <class C, bool AK, bool BK, bool REV>
 __device__ void cta_gemm_impl(Acc<C> &acc, const ViewT<typename C::T> &A, const ViewT<typename C::T> &B, int M,
                               int N, int K, typename C::T *smem, bool alA, bool alB) {
     using T = typename C::T;
     constexpr int ST = C::ST;
     T *sA = smem, *sB = smem + ST * C::SA;
     const int nk = (K + KC - 1) / KC;
+    auto k_of = [&](int c) { return (REV ? nk - 1 - c : c) * KC; };
     // prologue: stages 0 .. ST-2 in flight (one commit group each, possibly empty)
 #pragma unroll
     for (int st = 0; st < ST - 1; ++st) {
         if (st < nk) {
-            load_stage<T, C::BM, AK>(sA + st * C::SA, A, M, K, st * KC, alA);
-            load_stage<T, C::BN, BK>(sB + st * C::SB, B, N, K, st * KC, alB);
+            load_stage<T, C::BM, AK>(sA + st * C::SA, A, M, K, k_of(st), alA);
+            load_stage<T, C::BN, BK>(sB + st * C::SB, B, N, K, k_of(st), alB);
         }
         cp_async_commit();
     }
@@ -437,8 +438,8 @@ __device__ void cta_gemm_impl(Acc<C> &acc, const ViewT<typename C::T> &A, const 
         const int nxt = c + ST - 1;
         if (nxt < nk) {
             const int slot = nxt % ST;
-            load_stage<T, C::BM, AK>(sA + slot * C::SA, A, M, K, nxt * KC, alA);
-            load_stage<T, C::BN, BK>(sB + slot * C::SB, B, N, K, nxt * KC, alB);
+            load_stage<T, C::BM, AK>(sA + slot * C::SA, A, M, K, k_of(nxt), alA);
+            load_stage<T, C::BN, BK>(sB + slot * C::SB, B, N, K, k_of(nxt), alB);
         }
         cp_async_commit();
         cp_async_wait<ST - 1>();   // stage c has landed
@@ -458,17 +459,18 @@ __device__ __forceinline__ bool view_aligned(const ViewT<T> &V) {
 
 // acc(i,j) += sum_{k<K} A(i,k) B(j,k), i < M <= BM, j < N <= BN.  All threads
 // of the CTA call it; shared memory `smem` holds C::SMEM_BYTES.  Ends with a
-// barrier, so `smem` may be reused right after.
-template <class C>
+// barrier, so `smem` may be reused right after.  REV: sums from the end of K, KC
+// at a time.
+template <class C, bool REV = false>
 __device__ void cta_gemm(Acc<C> &acc, const ViewT<typename C::T> &A, const ViewT<typename C::T> &B, int M, int N,
                          int K, typename C::T *smem) {
     if (K <= 0 || M <= 0 || N <= 0) return;
     const bool ak = (A.rs != 1), bk = (B.rs != 1);
     const bool alA = view_aligned(A), alB = view_aligned(B);
-    if (!ak && !bk) cta_gemm_impl<C, false, false>(acc, A, B, M, N, K, smem, alA, alB);
-    else if (!ak && bk) cta_gemm_impl<C, false, true>(acc, A, B, M, N, K, smem, alA, alB);
-    else if (ak && !bk) cta_gemm_impl<C, true, false>(acc, A, B, M, N, K, smem, alA, alB);
-    else cta_gemm_impl<C, true, true>(acc, A, B, M, N, K, smem, alA, alB);
+    if (!ak && !bk) cta_gemm_impl<C, false, false, REV>(acc, A, B, M, N, K, smem, alA, alB);
+    else if (!ak && bk) cta_gemm_impl<C, false, true, REV>(acc, A, B, M, N, K, smem, alA, alB);
+    else if (ak && !bk) cta_gemm_impl<C, true, false, REV>(acc, A, B, M, N, K, smem, alA, alB);
+    else cta_gemm_impl<C, true, true, REV>(acc, A, B, M, N, K, smem, alA, alB);
 }
 
 // ---------------------------------------------------------------------------

@@ -571,11 +571,13 @@ __global__ void __launch_bounds__(NT_CTA, 2) xinv_pair_kernel(DiagTiles d, int h
 }
 
 // cond[2 k], cond[2 k + 1] = the infinity norms of diagonal tile k and of its
-// inverse (zeroed before): 64 rows of one tile per CTA.
+// inverse (zeroed before): 16 rows of one tile per CTA, 16 threads each, since a
+// row is a chain of loads (64 rows and 4 threads: 30 us at order 512).
+constexpr int NORM_ROWS = 16;
 __global__ void __launch_bounds__(NT_CTA, 4) xinv_norm_kernel(DiagTiles d, double *X, double *cond) {
-    const int k = blockIdx.y, r0 = blockIdx.x * IB;
-    rec::lower_norms<IB>(d.L(k), View{X + (int64_t)k * d.NB * d.NB, 1, d.NB}, r0, min(IB, d.order(k) - r0), false,
-                         cond + 2 * k);
+    const int k = blockIdx.y, r0 = blockIdx.x * NORM_ROWS;
+    rec::lower_norms<NORM_ROWS>(d.L(k), View{X + (int64_t)k * d.NB * d.NB, 1, d.NB}, r0,
+                                min(NORM_ROWS, d.order(k) - r0), false, cond + 2 * k);
 }
 
 // The full inverses of all diagonal tiles into X (W: scratch of the same size),
@@ -597,7 +599,7 @@ static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, double 
             xinv_pair_kernel<<<dim3(nb, nb, NT * pairs), NT_CTA, pair_smem, s>>>(d, h, pairs, X, W, first);
         CHB_LAUNCHED(2);
     }
-    xinv_norm_kernel<<<dim3((d.NB + IB - 1) / IB, NT), NT_CTA, 0, s>>>(d, X, cond);
+    xinv_norm_kernel<<<dim3((d.NB + NORM_ROWS - 1) / NORM_ROWS, NT), NT_CTA, 0, s>>>(d, X, cond);
     CHB_LAUNCHED(1);
     CHB_CUDA(cudaGetLastError());
     return 0;

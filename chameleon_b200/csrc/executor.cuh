@@ -103,6 +103,7 @@ constexpr int SOLB = 64;
 // twice as large, at 3e3 up to 20 times, at 1e6 1e4 times.
 constexpr int SOLVE_NB = 512;
 constexpr double XINV_COND = 8.0;
+constexpr int ILL_TILES = 1024;
 // Row block of the substitution tasks of a launch mode.
 __host__ __device__ constexpr int solve_rows(int mode) { return (mode & (4 | 32) /*XINV, FINE*/) ? SOLB : SUBB; }
 // Edge of the blocks that the counters count, and of an update task's block

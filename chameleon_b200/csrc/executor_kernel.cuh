@@ -30,6 +30,7 @@ constexpr int dag_ctas_per_sm() {
 template <class T>
 struct Dims {
     const ExecParams &p;
+    const unsigned *ill_bits;   // FP64 MODE_XINV: one bit per diagonal tile (mark_ill)
     __device__ int tm(int m) const { return (m == p.NT - 1) ? p.N - m * p.NB : p.NB; }
     // Row blocks of tile m that the counters count.
     __device__ int nbi(int m) const {
@@ -99,7 +100,17 @@ struct Dims {
     }
     // Whether the full inverse of diagonal tile k is too inaccurate to solve with
     // (FP64 MODE_XINV; NaN norms count).
-    __device__ bool ill(int k) const { return !(p.cond[2 * k] * p.cond[2 * k + 1] <= XINV_COND); }
+    __device__ bool ill_norms(int k) const { return !(p.cond[2 * k] * p.cond[2 * k + 1] <= XINV_COND); }
+    // ... for the first ILL_TILES tiles from the bits in shared memory: a step of
+    // the chain does not wait for two loads of its own
+    __device__ bool ill(int k) const { return k < ILL_TILES ? (ill_bits[k / 32] >> (k % 32)) & 1 : ill_norms(k); }
+    __device__ void mark_ill(unsigned *bits) const {
+        for (int k = threadIdx.x; k < ILL_TILES && k / 32 * 32 < p.NT; k += NT_CTA) {
+            const unsigned b = __ballot_sync(0xffffffffu, k < p.NT && ill_norms(k));
+            if (threadIdx.x % 32 == 0) bits[k / 32] = b;
+        }
+        __syncthreads();
+    }
 };
 
 // The counters a task waits on and the values they must reach (up to three;
@@ -516,11 +527,10 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
                     cta_gemm(acc, Xk.sub(r0, 0), X.sub(0, c0).t(), mr, wc, r0 + mr, smem);
                     acc.store_to(Yk.sub(r0, c0), mr, wc);
                 } else {
-                    // (the diagonal block last: it holds the largest terms, and
-                    // every later addition would round at their size)
-                    const int r1 = r0 + mr;
-                    cta_gemm(acc, Xk.sub(r1, r0).t(), Yk.sub(r1, c0).t(), mr, wc, n - r1, smem);
-                    cta_gemm(acc, Xk.sub(r0, r0).t(), Yk.sub(r0, c0).t(), mr, wc, mr, smem);
+                    // FP64: from the end, so that the diagonal terms, the largest,
+                    // come last: every later addition would round at their size
+                    cta_gemm<typename std::remove_reference_t<decltype(acc)>::C, sizeof(T) == 8>(
+                        acc, Xk.sub(r0, r0).t(), Yk.sub(r0, c0).t(), mr, wc, n - r0, smem);
                     acc.store_to(X.sub(r0, c0), mr, wc);
                 }
             };
@@ -616,7 +626,11 @@ __global__ void __launch_bounds__(NT_CTA, dag_ctas_per_sm<T, TC>()) cholesky_dag
     __shared__ int s_ok;
     __shared__ tc05::Smem tsm;
     __shared__ unsigned s_ph[3];   // phase cycles of the current task (tracing only)
-    const Dims<T> d{p};
+    __shared__ unsigned s_ill[ILL_TILES / 32];
+    const Dims<T> d{p, s_ill};
+    if constexpr (sizeof(T) == 8) {
+        if (p.mode & MODE_XINV) d.mark_ill(s_ill);
+    }
     if (p.after && (p.after->abort || p.after->error)) return;
     if constexpr (TC) tc05::init(&tsm);
     __shared__ Task s_desc;
