@@ -515,6 +515,19 @@ static int solve_tile(int N, const Tiling &A, const Tiling &B) {
     return 0;
 }
 
+// Right-hand sides so many that 128-row tasks fill the chip are solved with
+// them, on the storage's tiles (384 in a column-major array) with inverted 64 x
+// 64 blocks: they read the factor half as often as 64-row ones and need no array
+// for the forward results.  The line lies at 2e5 elements of B per row of a tile
+// (ms with tile inverses / this way: column-major order 8192 with 6000 columns
+// 35.1 / 48.8, 10000 58.4 / 57.9, 16384 95.1 / 85.1; 4096 with 12000 17.9 / 24.4,
+// 30000 44.3 / 40.3; tiles of 512, 8192 with 10000 58.3 / 75.7, 16384 94.9 / 89.2;
+// tiles of 250, 8192 with 3000 21.0 / 29.0, 6000 40.2 / 39.7).
+constexpr size_t WIDE_ELEMS = 200000;
+static int wide_tile(const Tiling &A, const Tiling &B) {
+    return A.rows1 && B.rows1 ? 384 : A.rows1 ? B.mb : A.nb;
+}
+
 // The diagonal tiles (order <= NB, NT of them) of a factor, as lower views.
 struct DiagTiles {
     double *A;
@@ -606,6 +619,7 @@ static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, double 
 }
 
 constexpr int TC_CHAIN_N = 20480;
+constexpr size_t OWN_ELEMS = (size_t)1 << 25;
 
 // One launch of the executor: its mode, tiles, task list and workspace.  Made
 // on the host alone (plan_launch).
@@ -619,7 +633,8 @@ struct Plan {
 };
 
 // mode: factorization, substitutions or both.  xnb > 0 (FP64 substitutions):
-// tiles of xnb with their full inverses.  B, b_elems: storage of B and its
+// tiles of xnb with their full inverses; xnb < 0: tiles of -xnb with 128-row
+// tasks.  B, b_elems: storage of B and its
 // elements (nrhs > 0).  reuse: the workspace holds the FP32 tile inverses of
 // this factor.
 static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling *B, int nrhs, size_t b_elems,
@@ -631,7 +646,8 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     q.f32 = f32;
     q.xnb = xnb;
     q.nrhs = nrhs;
-    const int NB = q.NB = xnb > 0 ? xnb : (t_given || f32) ? A.nb : exec_tile(A, (mode & MODE_SOLVE) ? B : nullptr);
+    const int NB = q.NB = xnb ? std::abs(xnb)
+                              : (t_given || f32) ? A.nb : exec_tile(A, (mode & MODE_SOLVE) ? B : nullptr);
     const int NT = q.NT = (N + NB - 1) / NB;
     q.NBB = B ? B->nb : NB;
     q.NTB = nrhs ? B->nt : 0;
@@ -661,7 +677,7 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     const bool full_inv = q.full_inv = f32 && c.rec_tile && NB <= (64 << rec::MAX_LVL);
     // (a task names its block by two 8-bit indices: a storage tile too large for
     // 64-blocks, and with no divisor to use instead, keeps 128-blocks)
-    if (!f32 && !t_given && NB <= 255 * FINEB) mode |= MODE_FINE;
+    if (!f32 && !t_given && xnb >= 0 && NB <= 255 * FINEB) mode |= MODE_FINE;
     // The tcgen05 path is bound by the chain of diagonal tiles up to about 80
     // tiles of 256 and by its updates (L2 operand traffic) beyond: the chain's
     // panel solves are split in two and the update groups kept short there
@@ -727,12 +743,18 @@ static int plan_call(Plan (&q)[2], WsBytes &ws, int mode, int N, bool f32, const
     // FP64 substitutions above one executor tile: a launch of their own, after
     // the factorization's (which it checks on the device).  With a
     // factorization of a small matrix they stay in its launch, where the
-    // forward sweep runs beside it (dposv 203: 232 us in one launch, 256 in
-    // two; 2048: 1.70 and 1.73 ms; 5003: 6.16 and 5.95 ms).
-    const bool own = (mode & MODE_FACT) ? N > 3072 : N > EXEC_NB;
-    const int xnb = (!f32 && !t_given && nrhs > 0 && own && !small) ? solve_tile(N, A, *B) : 0;
-    int n = 0;
+    // forward sweep runs beside it (1 to 17 right-hand sides, dposv 203: 232 us in
+    // one launch, 256 in two; 2048: 1.70 and 1.73 ms; 5003: 6.16 and 5.95 ms),
+    // unless B outweighs the factorization (2048 with 16384 columns 9.4 and 8.0
+    // ms; the line could lie lower: 3000 with 512 takes 8.4 in one, 3200 3.2 in two).
+    const bool own = (mode & MODE_FACT) ? N > 3072 || b_elems > OWN_ELEMS : N > EXEC_NB;
+    int xnb = (!f32 && !t_given && nrhs > 0 && own && !small) ? solve_tile(N, A, *B) : 0;
     if (xnb > 0) {
+        const int wide = wide_tile(A, *B);
+        if (b_elems / WIDE_ELEMS > (size_t)std::min(wide, 512)) xnb = -wide;
+    }
+    int n = 0;
+    if (xnb != 0) {
         if (mode & MODE_FACT)
             q[n++] = plan_launch(MODE_FACT, N, f32, A, nullptr, 0, 0, split, grid_req, nullptr, 0, false);
         q[n++] = plan_launch(MODE_SOLVE, N, f32, A, B, nrhs, b_elems, split, grid_req, nullptr, xnb, false);

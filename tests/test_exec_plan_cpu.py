@@ -79,3 +79,18 @@ def test_blocks_of_a_large_tile_fit_the_task(nb):
         assert max(x & 255 for x in got) == blk(m) - 1
     pan = t[t[:, 0] == 2]
     assert (pan[:, 1] >= 0).all() and (pan[:, 1] * e < NB).all()
+
+
+@pytest.mark.parametrize("n,nb,array,few,many", [(4096, 384, True, 12000, 30000), (8192, 512, False, 8192, 16384),
+                                                 (8192, 250, False, 3000, 7000), (2048, 384, True, 300, 45000)])
+def test_wide_right_hand_sides_take_no_second_array(n, nb, array, few, many):
+    """Past the width where 128-row tasks are faster the substitutions run on the
+    storage's tiles, without tile inverses and without an array of B's size."""
+    FINE, XINV_MODE = 32, 4
+    for mode in (SOLVE, FACT | SOLVE):
+        a, _ = plan(mode, n, nb, few, array)
+        b, _ = plan(mode, n, nb, many, array)
+        assert a[-1, MODE] & FINE and (mode == SOLVE) <= (a[-1, Y] == 8 * n * few)
+        assert not b[-1, MODE] & (FINE | XINV_MODE) and b[-1, Y] == b[-1, XINV] == 0
+        assert b[-1, 0] == (384 if array else nb)
+        assert len(b) == (1 if mode == SOLVE else 2)

@@ -1,4 +1,5 @@
 """dposv above the order where the substitutions get a launch of their own."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -179,3 +180,26 @@ def test_nan_in_a_factor_reaches_the_solution_it_belongs_to(cb, uplo):
     dB.from_numpy(np.ones((n, 2)))
     assert cb.dpotrs_Tile(uplo, dA, dB) == 0
     assert np.isnan(dB.to_numpy()[n - 1]).all()
+
+
+@pytest.mark.parametrize("n,nb,nrhs,array,uplo", [(2048, 512, 40001, True, LOWER), (1000, 200, 50003, False, UPPER),
+                                                  (700, 250, 75001, False, LOWER)])
+@pytest.mark.parametrize("posv", [False, True])
+def test_wide_right_hand_sides(cb, n, nb, nrhs, array, uplo, posv):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    S = torch.rand((n, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    S = S + S.T + n * torch.eye(n, dtype=torch.float64, device="cuda")
+    F = torch.linalg.cholesky(S)                     # lower; torch rows are our columns
+    a = (S if posv else F.T if uplo == LOWER else F).clone(memory_format=torch.contiguous_format)
+    b0 = torch.rand((nrhs, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    b, ptr = b0.clone(), lambda t: ctypes.c_void_p(t.data_ptr())
+    if array:
+        assert (cb.dposv if posv else cb.dpotrs)(uplo, n, nrhs, a, n, b, n) == 0
+    else:
+        L, dA, dB = cb.lib(), cb.Desc.create(n, n, nb), cb.Desc.create(n, nrhs, nb)
+        assert L.CHAMELEON_Lap2Desc(123, ptr(a), n, dA.ptr) == 0 and L.CHAMELEON_Lap2Desc(123, ptr(b), n, dB.ptr) == 0
+        assert (cb.dposv_Tile if posv else cb.dpotrs_Tile)(uplo, dA, dB) == 0
+        assert L.CHAMELEON_Desc2Lap(123, dB.ptr, ptr(b), n) == 0
+    r = float(torch.linalg.norm(b @ S - b0) / (torch.linalg.norm(S) * torch.linalg.norm(b)))
+    assert r <= 8 * n * EPS
