@@ -52,12 +52,26 @@ constexpr size_t lean_smem_bytes() {
            64;
 }
 
+// Right-hand-side columns of one system that are solved in strips of 8.  A strip
+// costs the same each, a block of up to 64 columns little more than one of 9
+// (2000 systems of order 200, ms, strips / block: FP64 with 8 columns 1.67 / 1.65,
+// 16 2.01 / 2.14, 24 2.27 / 2.15, 64 3.56 / 2.25; FP32 8 1.34 / 1.25, 32 2.13 /
+// 1.59; order 512, FP64 16 8.9 / 9.8, 24 10.0 / 9.8; FP32 8 5.0 / 5.3, 32 7.6 /
+// 6.5).  The FP32 line lies higher than its time, for precision: strips multiply
+// in FP64 (error of the solutions 1.8e-7 on dominant diagonals), the blocks two
+// bf16 parts (5e-6; two tf32 parts, 5e-7, took registers from the whole kernel:
+// 1500 systems of up to 300 0.77 -> 1.03 ms).
+template <class T>
+constexpr int strip_cols() {
+    return sizeof(T) == 8 ? 16 : 32;
+}
+
 // Generic bin: factor (+ forward and backward solve) of one system per task.
 // LEAN: 64-row panels and the leaf blocks aliased onto the GEMM staging area
 // (rec::lean_smem_elems), MINB CTAs per SM, so that the latency-bound leaf of
 // one system overlaps the GEMMs and leaves of the systems beside it.  Right-
-// hand sides are solved in strips of 8 columns in shared memory where the
-// order allows it.
+// hand sides are solved in blocks of 64 columns, the last few in strips of 8 in
+// shared memory where the order allows it.
 template <class T, bool LEAN = false, int MINB = 1>
 __global__ void __launch_bounds__(NT_CTA, MINB) posv_batch_kernel(const BatchItem *items, int count, T *A, T *B,
                                                                   int upper, int *info, int *cursor, T *scratch,
@@ -83,7 +97,21 @@ __global__ void __launch_bounds__(NT_CTA, MINB) posv_batch_kernel(const BatchIte
             const ViewT<T> X{B + it.b_off, 1, it.ldb};
             constexpr size_t smem_bytes = LEAN ? lean_smem_bytes<T, MINB>() : tile_smem_bytes<T>();
             const bool strips = rec::strip_smem_elems(it.n) * sizeof(double) <= smem_bytes;
-            for (int c0 = 0; strips && c0 < it.nrhs; c0 += rec::SW) {
+            // blocks of 64 columns, and what is left in strips where they are faster
+            int c0 = 0;
+            for (; c0 < it.nrhs && !(strips && it.nrhs - c0 <= strip_cols<T>()); c0 += IB) {
+                const int w = min(IB, it.nrhs - c0);
+                // a narrow last block (few right-hand sides, the common case)
+                // runs on the narrow tile instead of padding it to 64 columns
+                if (w <= Cfg64N<T>::BN) {
+                    trsm_left<T, SPLIT_BF16X3, Cfg64N<T>>(X.sub(0, c0), w, Lv, it.n, invd, false, smem);
+                    trsm_left<T, SPLIT_BF16X3, Cfg64N<T>>(X.sub(0, c0), w, Lv, it.n, invd, true, smem);
+                } else {
+                    trsm_left<T, SPLIT_BF16X3>(X.sub(0, c0), w, Lv, it.n, invd, false, smem);
+                    trsm_left<T, SPLIT_BF16X3>(X.sub(0, c0), w, Lv, it.n, invd, true, smem);
+                }
+            }
+            for (; c0 < it.nrhs; c0 += rec::SW) {
                 const int w = min(rec::SW, it.nrhs - c0), ld = rec::strip_ld(it.n), np = ld - 4;
                 double *sX = reinterpret_cast<double *>(smem_raw), *sR = sX + rec::SW * ld;
                 for (int idx = threadIdx.x; idx < rec::SW * np; idx += NT_CTA) {
@@ -97,18 +125,6 @@ __global__ void __launch_bounds__(NT_CTA, MINB) posv_batch_kernel(const BatchIte
                     *X.at(rr, c0 + cc) = (T)sX[rr + cc * ld];
                 }
                 __syncthreads();
-            }
-            for (int c0 = strips ? it.nrhs : 0; c0 < it.nrhs; c0 += IB) {
-                const int w = min(IB, it.nrhs - c0);
-                // a narrow last block (few right-hand sides, the common case)
-                // runs on the narrow tile instead of padding it to 64 columns
-                if (w <= Cfg64N<T>::BN) {
-                    trsm_left<T, SPLIT_BF16X3, Cfg64N<T>>(X.sub(0, c0), w, Lv, it.n, invd, false, smem);
-                    trsm_left<T, SPLIT_BF16X3, Cfg64N<T>>(X.sub(0, c0), w, Lv, it.n, invd, true, smem);
-                } else {
-                    trsm_left<T, SPLIT_BF16X3>(X.sub(0, c0), w, Lv, it.n, invd, false, smem);
-                    trsm_left<T, SPLIT_BF16X3>(X.sub(0, c0), w, Lv, it.n, invd, true, smem);
-                }
             }
         }
         cta_sync_global();

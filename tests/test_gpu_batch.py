@@ -208,3 +208,32 @@ def test_every_batch_shape_is_correct(cb, orc, r, lo, hi):
         assert ran >= 2
     finally:
         L.CHAM_B200_Batch_SetShape(cb.ChamRealDouble, r, -1)
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("n", [65, 200, 513])
+@pytest.mark.parametrize("nrhs", [1, 16, 17, 32, 33, 64, 65, 72, 80, 97, 130])
+def test_column_blocks_and_strips(cb, fp32, n, nrhs):
+    """Every split of the right-hand sides into 64-column blocks and strips of 8.
+    FP64: the bound of a backward stable solve; FP32: the products' 2^-16 (two
+    bf16 parts, their rounding and the part left out) in each of the two sweeps,
+    on a matrix of condition about 1."""
+    import ctypes
+
+    import torch
+    dt = torch.float32 if fp32 else torch.float64
+    g = torch.Generator().manual_seed(n + nrhs)
+    A = torch.rand((3, n, n), dtype=torch.float64, generator=g).sub_(0.5)
+    A = (A + A.transpose(1, 2) + n * torch.eye(n, dtype=torch.float64)).to(dt)
+    B = torch.rand((3, nrhs, n), dtype=torch.float64, generator=g).sub_(0.5).to(dt)
+    a, b = A.cuda(), B.cuda()
+    full = lambda v: torch.full((3,), v, dtype=torch.int32, device="cuda")
+    nn, kk, info = full(n), full(nrhs), full(-1)
+    ao, bo = (torch.arange(3, device="cuda") * s for s in (n * n, n * nrhs))
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    f = cb.lib().CHAM_B200_sposv_batch if fp32 else cb.lib().CHAM_B200_dposv_batch
+    assert f(122, 3, p(nn), p(kk), p(a), p(ao), p(b), p(bo), p(info), None) == 0
+    assert info.tolist() == [0, 0, 0]
+    X = torch.linalg.solve(A.double(), B.double().transpose(1, 2)).transpose(1, 2)
+    err = float((b.cpu().double() - X).norm() / X.norm())
+    assert err <= (4 * 2.0 ** -16 if fp32 else 64 * 2.0 ** -53)
