@@ -232,7 +232,7 @@ EXTRAS = {
     "CHAM_B200_Init": (_i, []),
     "CHAM_B200_Schedule_Size": (_i, [_i, _i, _i, _i, _i, _i, _i, _i]),
     "CHAM_B200_Schedule_Build": (_i, [_i, _i, _i, _i, _i, _i, _i, _i, ctypes.POINTER(Task), _i]),
-    "CHAM_B200_Exec_Plan": (_i, [_i, _i, _i, _i, _i, _i, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]),
+    "CHAM_B200_Exec_Plan": (_i, [_i, _i, _i, _i, _i, _i, _i, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]),
     "CHAM_B200_Test_Potrf_On_Dag": (_i, [_i, _i, _i]),
     "CHAM_B200_Workspace_Limit": (_i, [ctypes.c_longlong]),
     "CHAM_B200_Test_Enqueue_All": (_i, [_i, _i, _i, ctypes.POINTER(_i), ctypes.POINTER(_i)]),

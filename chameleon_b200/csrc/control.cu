@@ -517,6 +517,7 @@ int CHAMELEON_Set(int param, int value) {
         (param == CHAMELEON_B200_UPD_GROUP_F64 ? c.kgroup_f64
                                                : param == CHAMELEON_B200_UPD_GROUP_F32 ? c.kgroup_f32 : c.kgroup_tc) =
             value;
+        if (param == CHAMELEON_B200_UPD_GROUP_TC) c.kgroup_tc_set = true;
         return 0;
     case CHAMELEON_B200_UPD_TAIL_F64:
         if (value < 0 || value > 8) return CHAMELEON_ERR_ILLEGAL_VALUE;

@@ -618,7 +618,7 @@ static int xinv_launch(const DiagTiles &d, int NT, double *X, double *W, double 
     return 0;
 }
 
-constexpr int TC_CHAIN_N = 20480;
+constexpr int TC_DEEP_GROUP = 12;   // panels per update beyond the chain-bound orders, unless the caller set a number
 constexpr size_t OWN_ELEMS = (size_t)1 << 25;
 
 // One launch of the executor: its mode, tiles, task list and workspace.  Made
@@ -678,14 +678,16 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     // (a task names its block by two 8-bit indices: a storage tile too large for
     // 64-blocks, and with no divisor to use instead, keeps 128-blocks)
     if (!f32 && !t_given && xnb >= 0 && NB <= 255 * FINEB) mode |= MODE_FINE;
-    // The tcgen05 path is bound by the chain of diagonal tiles up to about 80
-    // tiles of 256 and by its updates (L2 operand traffic) beyond: the chain's
-    // panel solves are split in two and the update groups kept short there
-    // (order 16384: 16.9 -> 15.4 ms, 4096: 3.5 -> 3.05), while a chain that
-    // runs further ahead only costs the updates locality at larger orders
-    // (32768: 61 -> 65 ms), where deeper groups save C round trips instead
-    // (8 panels 61.0 ms, 12 panels 59.3).
-    const bool chain_bound = N <= TC_CHAIN_N;
+    // The tcgen05 path is bound by the chain of diagonal tiles at smaller orders
+    // and by its updates (L2 operand traffic) at larger ones: there the chain's
+    // panel solves are split in two and the update groups kept short (tiles of
+    // 256, order 16384: 16.9 -> 15.4 ms, 4096: 3.5 -> 3.05), while a chain that
+    // runs further ahead only costs the updates locality beyond (32768: 61 -> 65
+    // ms), where deeper groups save C round trips instead (8 panels 61.0 ms, 12
+    // panels 59.3).  The line moves with the tile size (short / deep, ms): 128
+    // 14000 12.6 / 13.1, 20480 24.9 / 23.8; 384 26880 36.5 / 36.7, 32768 58.1 /
+    // 55.9; 512 30000 45.4 / 46.4, 32768 55.2 / 54.2.
+    const bool chain_bound = N <= 20480;
     if (tc && !full_inv && chain_bound) mode |= MODE_HALF;
     const int prof = !f32 ? PROF_FP64 : (tc ? PROF_F32_TC05 : PROF_F32_MMA);
     // FP32 substitutions with full diagonal-tile inverses: computed off the
@@ -715,8 +717,8 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     // dispatch of an update over G panels (CHAMELEON_B200_UPD_GROUP per path)
     const int G = q.G = t_given ? 1
                                 : prof == PROF_FP64 ? group_f64(N, NB, c.kgroup_f64)
-                                                    : std::max(1, !tc ? c.kgroup_f32
-                                                                      : chain_bound ? c.kgroup_tc : c.kgroup_tc + c.kgroup_tc / 2);
+                                                    : !tc ? c.kgroup_f32
+                                                          : chain_bound || c.kgroup_tc_set ? c.kgroup_tc : TC_DEEP_GROUP;
     q.sh = Shape{mode, canonN, NB, canonR, NBB, q.grid, prof, G, cin ? std::max(1, cin->h2d_gbs) : 0, upd_tail(prof)};
     q.NIB = (NB + IB - 1) / IB;
     q.nctr = (size_t)(cin ? 3 : 2) * NT * NT + (size_t)4 * NT * std::max(NTB, 1) + NT;
@@ -1069,24 +1071,25 @@ extern "C" int CHAM_B200_Schedule_Size(int mode, int N, int NB, int nrhs, int NB
         .size();
 }
 
-// The launches of one FP64 call (mode MODE_FACT | MODE_SOLVE; A of order N in
-// nb x nb tiles, B in nb x nbb, or both column-major arrays) and their
-// workspace, host only: per launch {tile size, column block, bytes of counters,
-// inverted blocks, tile inverses, forward results, mode}, and in reserved[4] the bytes
+// The launches of one call (mode MODE_FACT | MODE_SOLVE; A of order N in nb x nb
+// tiles, B in nb x nbb, or both column-major arrays; fp32: the BF16x3 path) and
+// their workspace, host only: per launch {tile size, column block, bytes of
+// counters, inverted blocks, tile inverses, forward results, mode, update
+// group}, and in reserved[4] the bytes
 // that the call reserves.  Returns the number of launches (at most 2).
-extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs, int nbb, int64_t *launch,
+extern "C" int CHAM_B200_Exec_Plan(int mode, int N, int nb, int array, int nrhs, int nbb, int fp32, int64_t *launch,
                                    int64_t *reserved) {
     using namespace chb;
     auto tl = [&](int n, int t) { return Tiling{array || N <= nb, array || n <= t, nb, t, (n + t - 1) / t}; };
     const Tiling A = tl(N, nb), B = tl(std::max(nrhs, 1), nbb);
     Plan q[2];
     WsBytes r;
-    const int n = plan_call(q, r, mode, N, false, A, nrhs > 0 ? &B : nullptr, nrhs, (size_t)N * std::max(nrhs, 0), 0, 0,
-                            nullptr, false, false);
+    const int n = plan_call(q, r, mode, N, fp32 != 0, A, nrhs > 0 ? &B : nullptr, nrhs, (size_t)N * std::max(nrhs, 0),
+                            SPLIT_BF16X3, 0, nullptr, false, false);
     for (int i = 0; i < n; ++i) {
-        const int64_t v[7] = {q[i].NB, q[i].NBB, (int64_t)q[i].ws.ctr, (int64_t)q[i].ws.inv, (int64_t)q[i].ws.xinv,
-                              (int64_t)q[i].ws.y, q[i].mode};
-        std::copy(v, v + 7, launch + 7 * i);
+        const int64_t v[8] = {q[i].NB, q[i].NBB, (int64_t)q[i].ws.ctr, (int64_t)q[i].ws.inv, (int64_t)q[i].ws.xinv,
+                              (int64_t)q[i].ws.y, q[i].mode, q[i].G};
+        std::copy(v, v + 8, launch + 8 * i);
     }
     const int64_t v[4] = {(int64_t)r.ctr, (int64_t)r.inv, (int64_t)r.xinv, (int64_t)r.y};
     std::copy(v, v + 4, reserved);

@@ -6,14 +6,14 @@ import pytest
 
 FACT, SOLVE = 1, 2
 # columns of a planned launch (0, 1: tile size, column block)
-CTR, INV, XINV, Y, MODE = 2, 3, 4, 5, 6
+CTR, INV, XINV, Y, MODE, GROUP = 2, 3, 4, 5, 6, 7
 
 
-def plan(mode, N, nb, nrhs, array=False, nbb=None):
+def plan(mode, N, nb, nrhs, array=False, nbb=None, fp32=False):
     import chameleon_b200 as cb
-    launch, res = np.zeros((2, 7), np.int64), np.zeros(4, np.int64)
+    launch, res = np.zeros((2, 8), np.int64), np.zeros(4, np.int64)
     p = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
-    n = cb.lib().CHAM_B200_Exec_Plan(mode, N, nb, int(array), nrhs, nbb or nb, p(launch), p(res))
+    n = cb.lib().CHAM_B200_Exec_Plan(mode, N, nb, int(array), nrhs, nbb or nb, int(fp32), p(launch), p(res))
     return launch[:n], res
 
 
@@ -94,3 +94,11 @@ def test_wide_right_hand_sides_take_no_second_array(n, nb, array, few, many):
         assert not b[-1, MODE] & (FINE | XINV_MODE) and b[-1, Y] == b[-1, XINV] == 0
         assert b[-1, 0] == (384 if array else nb)
         assert len(b) == (1 if mode == SOLVE else 2)
+
+
+@pytest.mark.parametrize("nb,line", [(128, 20480), (256, 20480), (384, 20480), (512, 20480)])
+def test_update_groups_of_the_tensor_core_path(nb, line):
+    HALF = 64
+    for n, half, group in ((line, True, 8), (line + nb, False, 12)):
+        a, _ = plan(FACT, n, nb, 0, fp32=True)
+        assert bool(a[0, MODE] & HALF) == half and a[0, GROUP] == group

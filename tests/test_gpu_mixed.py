@@ -253,3 +253,25 @@ def test_dsposv_host_matrix_streams_while_factoring(cb, orc, uplo, N, NB, nrhs):
         assert np.array_equal(Ah.numpy(), A.T, equal_nan=True)   # the host matrix is not written
     finally:
         cb.set_param(cb.CHAMELEON_TILE_SIZE, 384)
+
+
+def test_update_group_that_the_caller_sets_is_used(cb):
+    """A caller's number of panels per update holds at every order."""
+    import subprocess
+    import sys
+    code = """
+import ctypes, numpy as np, chameleon_b200 as cb
+cb.init()
+L = cb.lib()
+launch, res = (ctypes.c_int64 * 16)(), (ctypes.c_int64 * 4)()
+def group(n):
+    assert L.CHAM_B200_Exec_Plan(1, n, 256, 0, 0, 256, 1, launch, res) == 1
+    return launch[7]
+assert (group(8192), group(32768)) == (8, 12)
+for g in (8, 3, 20):
+    assert L.CHAMELEON_Set(cb.CHAMELEON_B200_UPD_GROUP_TC, g) == 0
+    assert (group(8192), group(32768)) == (g, g)
+"""
+    import os
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], cwd=root, check=True, timeout=300)
