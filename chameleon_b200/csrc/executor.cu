@@ -687,7 +687,7 @@ static Plan plan_launch(int mode, int N, bool f32, const Tiling &A, const Tiling
     // panels 59.3).  The line moves with the tile size (short / deep, ms): 128
     // 14000 12.6 / 13.1, 20480 24.9 / 23.8; 384 26880 36.5 / 36.7, 32768 58.1 /
     // 55.9; 512 30000 45.4 / 46.4, 32768 55.2 / 54.2.
-    const bool chain_bound = N <= 20480;
+    const bool chain_bound = N <= (NB < 384 ? 20480 : 30720);
     if (tc && !full_inv && chain_bound) mode |= MODE_HALF;
     const int prof = !f32 ? PROF_FP64 : (tc ? PROF_F32_TC05 : PROF_F32_MMA);
     // FP32 substitutions with full diagonal-tile inverses: computed off the

@@ -96,7 +96,7 @@ def test_wide_right_hand_sides_take_no_second_array(n, nb, array, few, many):
         assert len(b) == (1 if mode == SOLVE else 2)
 
 
-@pytest.mark.parametrize("nb,line", [(128, 20480), (256, 20480), (384, 20480), (512, 20480)])
+@pytest.mark.parametrize("nb,line", [(128, 20480), (256, 20480), (384, 30720), (512, 30720)])
 def test_update_groups_of_the_tensor_core_path(nb, line):
     HALF = 64
     for n, half, group in ((line, True, 8), (line + nb, False, 12)):
