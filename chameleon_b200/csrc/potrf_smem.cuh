@@ -80,13 +80,16 @@ static __device__ __noinline__ int leaf(float *D, int ldd, int nbk, float *sD) {
 // 16-byte loads feed 48 FMAs.  The products are small and their operands are
 // in shared memory, where the tensor-core form (three TF32 products per pair)
 // spent its time on splitting operands and rounded more: order 256 137 us with
-// it, 112 us with FMA.  Rows >= M of the last 64-row group are computed from whatever follows
-// and are not stored.
+// it, 112 us with FMA.  Threads whose rows are all >= M, or columns >= N, sum
+// those of row or column 0 instead (what follows may be written meanwhile);
+// neither is stored.
 struct Frag {
     float v[3][4][4];   // [row group][column][row]
 };
-static __device__ __forceinline__ void gemm64(Frag &acc, const float *Xm, int ldx, int M, const float *Ym, int ldy) {
-    const float *x = Xm + 4 * (threadIdx.x & 15), *y = Ym + 4 * (threadIdx.x >> 4);
+static __device__ __forceinline__ void gemm64(Frag &acc, const float *Xm, int ldx, int M, const float *Ym, int ldy,
+                                              int N) {
+    const int r0 = 4 * (threadIdx.x & 15), c0 = 4 * (threadIdx.x >> 4);
+    const float *x = Xm + r0, *y = Ym + (c0 < N ? c0 : 0);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -94,6 +97,7 @@ static __device__ __forceinline__ void gemm64(Frag &acc, const float *Xm, int ld
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc.v[i][j][e] = 0.f;
     const int ng = (M + 63) / 64;   // row groups (uniform across the CTA)
+    const float *xl = Xm + (r0 + 64 * (ng - 1) < M ? r0 + 64 * (ng - 1) : 0);   // the last one
     auto sweep = [&](auto groups) {
         constexpr int G = decltype(groups)::value;
 #pragma unroll 4
@@ -101,7 +105,7 @@ static __device__ __forceinline__ void gemm64(Frag &acc, const float *Xm, int ld
             const float4 b = *reinterpret_cast<const float4 *>(y + k * ldy);
 #pragma unroll
             for (int i = 0; i < G; ++i) {
-                const float4 a = *reinterpret_cast<const float4 *>(x + 64 * i + k * ldx);
+                const float4 a = *reinterpret_cast<const float4 *>((i == G - 1 ? xl : x + 64 * i) + k * ldx);
                 const float bb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -225,7 +229,7 @@ static __device__ __noinline__ int potrf(const ViewF &T, int n, float *invd, flo
         // panel: L_ib = A_ib X_b^T, computed in registers, then stored in place
         {
             Frag acc;
-            gemm64(acc, Sb + BW, ldb, M, Xs, LDI);   // X_b(c, k) at Xs[k * LDI + c]
+            gemm64(acc, Sb + BW, ldb, M, Xs, LDI, BW);   // X_b(c, k) at Xs[k * LDI + c]
             __syncthreads();
             frag_store<false>(acc, Sb + BW, ldb, M, nbk, false);
             __syncthreads();
@@ -237,7 +241,7 @@ static __device__ __noinline__ int potrf(const ViewF &T, int n, float *invd, flo
             const int ldc = blk_ld(n, cb), Mc = n - BW * cb, wc = min(BW, n - BW * cb);
             Frag acc;
             // rows i >= 64 cb of panel b, against its rows 64 cb .. 64 cb + 63
-            gemm64(acc, Sb + BW * (cb - b), ldb, Mc, Sb + BW * (cb - b), ldb);
+            gemm64(acc, Sb + BW * (cb - b), ldb, Mc, Sb + BW * (cb - b), ldb, wc);
             frag_store<true>(acc, Sc, ldc, Mc, wc, true);
         }
         __syncthreads();
