@@ -235,6 +235,7 @@ EXTRAS = {
     "CHAM_B200_Exec_Plan": (_i, [_i, _i, _i, _i, _i, _i, _i, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]),
     "CHAM_B200_Test_Potrf_On_Dag": (_i, [_i, _i, _i]),
     "CHAM_B200_Workspace_Limit": (_i, [ctypes.c_longlong]),
+    "CHAM_B200_Test_Pivot_Recip": (_i, [_i, _i, _vp, _vp, _vp, _vp]),
     "CHAM_B200_Test_Enqueue_All": (_i, [_i, _i, _i, ctypes.POINTER(_i), ctypes.POINTER(_i)]),
     "CHAM_B200_dposv_timed": (_i, [_i, _i, _i, _vp, _i, _vp, _i, ctypes.POINTER(ctypes.c_float)]),
     "CHAM_B200_Event_Record": (_i, [_i]),

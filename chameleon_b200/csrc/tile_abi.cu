@@ -256,6 +256,14 @@ static dim3 cast_grid(int m, int n) {
     return dim3(gx, gy);
 }
 
+// The leaf's pivot estimates over arrays (its accuracy test); ok: 1 where they
+// can be used.
+template <class T>
+__global__ void pivot_recip_kernel(const T *d, T *rc, T *rs, int *ok, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        ok[i] = rec::pivot_recip(d[i], rc[i], rs[i]);
+}
+
 static int ew_grid(int64_t total) {
     const int64_t b = (total + 255) / 256;
     return (int)std::min<int64_t>(std::max<int64_t>(b, 1), 148 * 32);
@@ -391,6 +399,15 @@ int CUDA_dtrsm(cham_side_t side, cham_uplo_t uplo, cham_trans_t transa, cham_dia
         CHB_LAUNCHED(3);
     }
     return cudaGetLastError() == cudaSuccess ? CHAMELEON_SUCCESS : CHAMELEON_ERR_UNEXPECTED;
+}
+
+int CHAM_B200_Test_Pivot_Recip(int fp32, int n, const void *d, void *rc, void *rs, int *ok) {
+    if (n <= 0) return 0;
+    if (fp32) pivot_recip_kernel<<<ew_grid(n), 256>>>((const float *)d, (float *)rc, (float *)rs, ok, n);
+    else pivot_recip_kernel<<<ew_grid(n), 256>>>((const double *)d, (double *)rc, (double *)rs, ok, n);
+    CHB_CUDA(cudaGetLastError());
+    CHB_CUDA(cudaDeviceSynchronize());
+    return 0;
 }
 
 int CUDA_dpotrf(cham_uplo_t uplo, int n, double *A, int lda, double *WORK, int lwork, int *d_info,

@@ -166,3 +166,28 @@ def test_fp32_leaf_rounds_an_entry_about_once(cb):
         R = np.linalg.cholesky(a.astype(np.float64))
         errs.append(np.linalg.norm(F - R) / np.linalg.norm(R))
     assert np.mean(errs) <= 2.0 ** -24
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+def test_pivot_estimates(cb, fp32):
+    """1 / d and d^(-1/2) over the accepted exponents: one rounding and what the
+    series leaves out, and for the root half a rounding of d q (rec.cuh)."""
+    import torch
+    dt, u, lo, hi = (np.float32, 2.0 ** -24, 1e-30, 1e30) if fp32 else (np.float64, 2.0 ** -53, 1e-280, 1e280)
+    g = np.random.default_rng(3)
+    n = 1 << 18
+    d = np.concatenate([np.exp(g.uniform(np.log(lo), np.log(hi), n)), g.uniform(1, 4, n), 1 + g.uniform(0, 1e-6, n),
+                        4 - g.uniform(0, 1e-6, n), 2.0 ** g.integers(-90, 90, n)]).astype(dt)
+    bad = np.array([0.0, -1.0, np.nan, np.inf, -np.inf, lo / 2, hi * 2], dt)
+    x = torch.from_numpy(np.concatenate([d, bad])).cuda()
+    rc, rs, ok = torch.empty_like(x), torch.empty_like(x), torch.empty(x.numel(), dtype=torch.int32, device="cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    torch.cuda.synchronize()
+    assert cb.lib().CHAM_B200_Test_Pivot_Recip(int(fp32), x.numel(), p(x), p(rc), p(rs), p(ok)) == 0
+    used = ok.cpu().numpy().astype(bool)
+    assert used[:len(d)][(d > lo) & (d < hi)].all() and not used[len(d):].any()
+    t = d.astype(np.longdouble)
+    use = used[:len(d)]
+    erc = np.abs(rc.cpu().numpy()[:len(d)].astype(np.longdouble) * t - 1)[use].max()
+    ers = np.abs(rs.cpu().numpy()[:len(d)].astype(np.longdouble) * np.sqrt(t) - 1)[use].max()
+    assert erc <= 1.01 * u and ers <= 1.6 * u, (erc / u, ers / u)
