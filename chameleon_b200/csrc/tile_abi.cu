@@ -72,6 +72,18 @@ static void launch_gemm(View A, View B, View C, int M, int N, int K, double alph
     const dim3 grid((M + E - 1) / E, (N + E - 1) / E);
     gemm_kernel<E><<<grid, NT_CTA, CfgTile<E>::SMEM_BYTES, s>>>(A, B, C, M, N, K, alpha, beta, tri);
 }
+// SMs of the current device.
+static int sm_count() {
+    static std::atomic<int> n[64];
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if ((v = n[dev]) == 0) {
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;
+        n[dev] = v;
+    }
+    return v;
+}
+
 // Block edge: 128 from two blocks per SM on, 64 from one block per SM on, 32
 // below.
 static void gemm_tile(View A, View B, View C, int M, int N, int K, double alpha, double beta, int tri,
@@ -80,8 +92,9 @@ static void gemm_tile(View A, View B, View C, int M, int N, int K, double alpha,
         const int64_t a = (M + e - 1) / e, b = (N + e - 1) / e;
         return tri ? a * (a + 1) / 2 : a * b;
     };
-    if (blocks(128) >= 2 * 148) launch_gemm<128>(A, B, C, M, N, K, alpha, beta, tri, s);
-    else if (blocks(64) >= 148) launch_gemm<64>(A, B, C, M, N, K, alpha, beta, tri, s);
+    const int sms = sm_count();
+    if (blocks(128) >= 2 * sms) launch_gemm<128>(A, B, C, M, N, K, alpha, beta, tri, s);
+    else if (blocks(64) >= sms) launch_gemm<64>(A, B, C, M, N, K, alpha, beta, tri, s);
     else launch_gemm<32>(A, B, C, M, N, K, alpha, beta, tri, s);
 }
 
@@ -387,7 +400,7 @@ int CUDA_dtrsm(cham_side_t side, cham_uplo_t uplo, cham_trans_t transa, cham_dia
     const int nblk = (ns + IB - 1) / IB;
     if (int rc = handle_ws(handle, (size_t)nblk * IB * IB * sizeof(double))) return rc;
     inv_diag_kernel<<<nblk, NT_CTA, INV_SMEM_BYTES, handle->stream>>>(L, ns, handle->ws, diag == ChamUnit);
-    if (ns <= STRIP_MAXN && w <= 2 * 148 * SW) {
+    if (ns <= STRIP_MAXN && w <= 2 * sm_count() * SW) {
         trsm_strip_kernel<<<(w + SW - 1) / SW, NT_CTA, strip_smem(ns), handle->stream>>>(L, ns, handle->ws, X, w,
                                                                                        trans_eff, *alpha);
         CHB_LAUNCHED(2);
