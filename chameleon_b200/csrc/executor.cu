@@ -106,8 +106,11 @@ std::vector<Task> build_order(const Shape &s) {
     auto wB = [&](int bn) { return (bn == NTB - 1) ? s.nrhs - bn * s.NBB : s.NBB; };
     const bool fact = s.mode & MODE_FACT, solve = s.mode & MODE_SOLVE;
 
+    // the updates are all but all of a factorization's tasks
+    size_t count = (size_t)2 * NT * NT + (size_t)NTB * NT * (NT + 1);
+    for (int n = 0; fact && n < NT; ++n) count += (size_t)upd_ngroups(n, s.G, s.tail) * (NT - n);
     std::vector<Coarse> ct;
-    ct.reserve(fact ? (size_t)NT * NT * NT / 6 + 4 * NT * NT : 4 * NT * NT + 8);
+    ct.reserve(count);
     auto add = [&](int kind, int m, int n, int k, int bn, int nsub, double dur) {
         Coarse c;
         c.kind = kind; c.m = m; c.n = n; c.k = k; c.bn = bn; c.grp = 0; c.nsub = nsub; c.dur = dur;

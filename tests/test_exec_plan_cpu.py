@@ -102,3 +102,20 @@ def test_update_groups_of_the_tensor_core_path(nb, line):
     for n, half, group in ((line, True, 8), (line + nb, False, 12)):
         a, _ = plan(FACT, n, nb, 0, fp32=True)
         assert bool(a[0, MODE] & HALF) == half and a[0, GROUP] == group
+
+
+def test_task_list_of_a_large_order_fits_a_small_process():
+    """The host's task graph has a task per update group, not per update: order
+    65536 in 1 GB of address space beyond the process's own."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import resource, chameleon_b200 as cb
+L = cb.lib()
+have = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (have + (1 << 30),) * 2)
+assert L.CHAM_B200_Schedule_Size(1 | 32, 65536, 128, 0, 128, 296, 0, 32) > 0
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], cwd=root, check=True, timeout=300)
