@@ -436,13 +436,15 @@ int CUDA_dpotrf(cham_uplo_t uplo, int n, double *A, int lda, double *WORK, int l
         return 0;
     }
     if (int rc = set_smem_attrs()) return rc;
+    // (also when the tile DAG runs: a later call of another order on a stream under
+    // capture may need it, and cannot allocate)
+    const int nblk = (n + IB - 1) / IB;
+    if (int rc = handle_ws(handle, (size_t)nblk * IB * IB * sizeof(double))) return rc;
     // the tile DAG where it can be used; a stream under capture takes it only
     // when nothing has to be allocated or uploaded for it
     bool ran = false;
     if (int rc = dag_potrf_async(uplo, n, A, lda, d_info, handle->stream, handle->ews, &ran)) return rc;
     if (ran) return CHAMELEON_SUCCESS;
-    const int nblk = (n + IB - 1) / IB;
-    if (int rc = handle_ws(handle, (size_t)nblk * IB * IB * sizeof(double))) return rc;
     const View T = (uplo == ChamLower) ? View{A, 1, lda} : View{A, lda, 1};
     potrf_kernel<<<1, NT_CTA, POTRF_SMEM_BYTES, handle->stream>>>(T, n, handle->ws, d_info);
     CHB_LAUNCHED(1);

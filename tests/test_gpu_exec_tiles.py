@@ -191,3 +191,68 @@ def test_pivot_estimates(cb, fp32):
     erc = np.abs(rc.cpu().numpy()[:len(d)].astype(np.longdouble) * t - 1)[use].max()
     ers = np.abs(rs.cpu().numpy()[:len(d)].astype(np.longdouble) * np.sqrt(t) - 1)[use].max()
     assert erc <= 1.01 * u and ers <= 1.6 * u, (erc / u, ers / u)
+
+
+@pytest.mark.parametrize("n", [512, 300, 129, 100])
+def test_potrf_under_stream_capture(cb, n):
+    """A handle that has factored order 512 is captured at that order and at
+    smaller ones it has not seen; the graph factors what its replays find."""
+    import torch
+    L, h, s = cb.lib(), ctypes.c_void_p(), torch.cuda.Stream()
+    assert L.CHAM_B200_Handle_Create(ctypes.byref(h), ctypes.c_void_p(s.cuda_stream)) == 0
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    info = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    warm = torch.from_numpy(spd(512, 1).T.copy()).cuda()
+    torch.cuda.synchronize()
+    assert L.CUDA_dpotrf(LOWER, 512, p(warm), 512, None, 0, p(info), h) == 0
+    t = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        assert L.CUDA_dpotrf(LOWER, n, p(t), n, None, 0, p(info), h) == 0
+    for seed in (5, 6):
+        A0 = spd(n, seed)
+        t.copy_(torch.from_numpy(A0.T.copy()))
+        info.fill_(-7)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        F = np.tril(t.cpu().numpy().T)
+        assert int(info) == 0
+        assert np.linalg.norm(A0 - F @ F.T) <= 8 * n * EPS * np.linalg.norm(A0)
+    del graph
+    torch.cuda.synchronize()
+    L.CHAM_B200_Handle_Destroy(h)
+
+
+@pytest.mark.parametrize("n,w", [(1, 1), (64, 3), (65, 9), (513, 130), (200, 2369), (3072, 5), (3073, 2), (1000, 2500)])
+@pytest.mark.parametrize("side", [141, 142])
+@pytest.mark.parametrize("uplo,trans,diag,alpha", [(LOWER, 111, 131, 1.0), (LOWER, 112, 132, -0.5), (UPPER, 111, 132, 2.0),
+                                                   (UPPER, 112, 131, 0.0)])
+def test_trsm_routes(cb, n, w, side, uplo, trans, diag, alpha):
+    """Strips, and the 64-column route beyond their order and width."""
+    import torch
+    g = np.random.default_rng(n + w)
+    T = g.uniform(-0.5, 0.5, (n, n)) / n
+    T[np.diag_indices(n)] = g.uniform(1, 2, n)
+    tri = np.tril if uplo == LOWER else np.triu
+    full = tri(T).copy()
+    if diag == 132:
+        full[np.diag_indices(n)] = 1.0
+        T[np.diag_indices(n)] = np.nan                     # not referenced
+    A = np.where(tri(np.ones((n, n), bool)), T, np.nan)
+    rows, cols = (n, w) if side == 141 else (w, n)
+    B = g.uniform(-0.5, 0.5, (rows, cols))
+    op = full if trans == 111 else full.T
+    want = alpha * (np.linalg.solve(op, B) if side == 141 else np.linalg.solve(op.T, B.T).T)
+    a, b = torch.from_numpy(A.T.copy()).cuda(), torch.from_numpy(B.T.copy()).cuda()
+    L, h = cb.lib(), ctypes.c_void_p()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert L.CHAM_B200_Handle_Create(ctypes.byref(h), None) == 0
+    torch.cuda.synchronize()
+    assert L.CUDA_dtrsm(side, uplo, trans, diag, rows, cols, ctypes.byref(ctypes.c_double(alpha)), p(a), n, p(b), rows,
+                        h) == 0
+    torch.cuda.synchronize()
+    L.CHAM_B200_Handle_Destroy(h)
+    # row sums of |T^-1| |T| are below 4: a few eps each, whatever n
+    assert np.abs(b.cpu().numpy().T - want).max() <= 64 * EPS * np.abs(want).max()
