@@ -203,3 +203,55 @@ def test_wide_right_hand_sides(cb, n, nb, nrhs, array, uplo, posv):
         assert L.CHAMELEON_Desc2Lap(123, dB.ptr, ptr(b), n) == 0
     r = float(torch.linalg.norm(b @ S - b0) / (torch.linalg.norm(S) * torch.linalg.norm(b)))
     assert r <= 8 * n * EPS
+
+
+@pytest.mark.parametrize("bad", [1, 40, 3050])
+@pytest.mark.parametrize("uplo", [LOWER, UPPER])
+def test_failed_factorization_leaves_the_right_hand_sides(cb, uplo, bad):
+    """The substitutions' launch sees that the factorization's has failed."""
+    n, nb = 3100, 512
+    A = np.random.default_rng(1).uniform(-0.5, 0.5, (n, n)) + n * np.eye(n)
+    A[bad - 1, bad - 1] = -1.0
+    B = np.random.default_rng(2).uniform(-0.5, 0.5, (n, 7))
+    dA, dB = cb.Desc.create(n, n, nb), cb.Desc.create(n, 7, nb)
+    dA.from_numpy(A)
+    dB.from_numpy(B)
+    assert cb.dposv_Tile(uplo, dA, dB) == bad
+    assert np.array_equal(dB.to_numpy(), B)
+    dA.from_numpy(n * np.eye(n))               # and the next call is not affected
+    assert cb.dposv_Tile(uplo, dA, dB) == 0
+    assert np.abs(dB.to_numpy() * n - B).max() <= 4 * EPS
+
+
+@pytest.mark.parametrize("n,nb,nrhs", [(3073, 512, 1), (3200, 200, 17), (3144, 262, 64), (3100, 509, 33)])
+@pytest.mark.parametrize("uplo", [LOWER, UPPER])
+@pytest.mark.parametrize("layout", ["tiles", "array"])
+def test_two_launches_over_tilings(cb, layout, uplo, n, nb, nrhs):
+    """Remainders, tiles with and without usable divisors, odd leading dimension."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ld = n + 3
+    S = torch.rand((n, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    S = S + S.T + n * torch.eye(n, dtype=torch.float64, device="cuda")
+    B = torch.rand((nrhs, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    part = S.triu() if uplo == LOWER else S.tril()     # rows are columns
+    a = torch.full((n, ld), float("nan"), dtype=torch.float64, device="cuda")
+    a[:, :n] = torch.where(part != 0, part, a[:, :n])
+    b = torch.full((nrhs, ld), float("nan"), dtype=torch.float64, device="cuda")
+    b[:, :n] = B
+    p, L = lambda t: ctypes.c_void_p(t.data_ptr()), cb.lib()
+    if layout == "tiles":
+        dA, dB = cb.Desc.create(n, n, nb), cb.Desc.create(n, nrhs, nb)
+    for step in ("posv", "potrs"):
+        b[:, :n] = B
+        if layout == "array":
+            assert (cb.dposv if step == "posv" else cb.dpotrs)(uplo, n, nrhs, a, ld, b, ld) == 0
+        else:
+            if step == "posv":
+                assert L.CHAMELEON_Lap2Desc(123, p(a), ld, dA.ptr) == 0
+            assert L.CHAMELEON_Lap2Desc(123, p(b), ld, dB.ptr) == 0
+            assert (cb.dposv_Tile if step == "posv" else cb.dpotrs_Tile)(uplo, dA, dB) == 0
+            assert L.CHAMELEON_Desc2Lap(123, dB.ptr, p(b), ld) == 0
+        X = b[:, :n]
+        r = float(torch.linalg.norm(X @ S - B) / (torch.linalg.norm(S) * torch.linalg.norm(X)))
+        assert r <= 8 * n * EPS, (step, r)
