@@ -337,10 +337,19 @@ static __device__ __noinline__ void solve_strips(const Task &t, const Dims<doubl
     }
 }
 
-template <class T, int SP, bool TC>
+// What a kernel variant runs.  FP64 substitutions with full tile inverses are
+// launches of their own, with a kernel of their own: in one kernel the two share
+// registers and code (dpotrf of order 8192 10.02 ms in one kernel, 9.79 apart;
+// dposv of order 2048 1.74 and 1.69).
+enum Part : int { PART_ALL = 0, PART_NO_XINV = 1, PART_XINV = 2 };
+
+template <class T, int SP, bool TC, int PART>
 __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T *smem, tc05::Smem *tsm,
                          uint8_t *stage, unsigned *ph, Ahead *ah) {
     using VT = ViewT<T>;
+    if constexpr (PART == PART_XINV) {   // the other cases are not compiled
+        if (t.kind != TK_FWD_TRSM && t.kind != TK_FWD_UPD && t.kind != TK_BWD_TRSM && t.kind != TK_BWD_UPD) return;
+    }
     switch (t.kind) {
     case TK_POTRF: {
         int info;
@@ -508,7 +517,7 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
     case TK_BWD_TRSM: {
         const VT X = d.Bt(t.k, t.bn);
         const int w = d.wB(t.bn);
-        if (p.mode & MODE_XINV) {
+        if (PART != PART_NO_XINV && (PART == PART_XINV || (p.mode & MODE_XINV))) {
             // row block t.sub (SOLB rows) of the tile: forward Y_k = X_k B_k,
             // backward B_k = X_k^T Y_k
             const int r0 = t.sub * SOLB, n = d.tm(t.k);
@@ -560,7 +569,7 @@ __device__ void run_task(const Task &t, const ExecParams &p, const Dims<T> &d, T
     case TK_BWD_UPD: {
         // MODE_XINV: forward updates read Y_k into B_m, backward ones read B_k
         // into Y_m, in SOLB-row blocks
-        const bool y = p.mode & MODE_XINV;
+        const bool y = PART != PART_NO_XINV && (PART == PART_XINV || (p.mode & MODE_XINV));
         const int rb = solve_rows(p.mode);
         const int r0 = t.sub * rb;
         const int rows = min(rb, d.tm(t.m) - r0);
@@ -613,7 +622,7 @@ __device__ inline int *task_counter(const Task &t, const ExecParams &p) {
     return nullptr;
 }
 
-template <class T, int SP, bool TC>
+template <class T, int SP, bool TC, int PART>
 __global__ void __launch_bounds__(NT_CTA, dag_ctas_per_sm<T, TC>()) cholesky_dag_kernel(ExecParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte aligned base: the tcgen05 stages need it; other tasks share it
@@ -628,9 +637,7 @@ __global__ void __launch_bounds__(NT_CTA, dag_ctas_per_sm<T, TC>()) cholesky_dag
     __shared__ unsigned s_ph[3];   // phase cycles of the current task (tracing only)
     __shared__ unsigned s_ill[ILL_TILES / 32];
     const Dims<T> d{p, s_ill};
-    if constexpr (sizeof(T) == 8) {
-        if (p.mode & MODE_XINV) d.mark_ill(s_ill);
-    }
+    if constexpr (PART == PART_XINV) d.mark_ill(s_ill);
     if (p.after && (p.after->abort || p.after->error)) return;
     if constexpr (TC) tc05::init(&tsm);
     __shared__ Task s_desc;
@@ -678,7 +685,7 @@ __global__ void __launch_bounds__(NT_CTA, dag_ctas_per_sm<T, TC>()) cholesky_dag
         const Task t = s_desc;
         uint64_t t0 = 0;
         if (p.trace && threadIdx.x == 0) t0 = globaltimer();
-        run_task<T, SP, TC>(t, p, d, smem, &tsm, stage, p.trace ? s_ph : nullptr, &ah);
+        run_task<T, SP, TC, PART>(t, p, d, smem, &tsm, stage, p.trace ? s_ph : nullptr, &ah);
         // Every thread's writes of the task precede thread 0's release through
         // the barrier (the release is cumulative), so no per-thread fence.
         __syncthreads();
@@ -717,15 +724,15 @@ constexpr size_t dag_smem_bytes() {
 
 // Launch one persistent executor kernel of a variant (its shared-memory size
 // attribute is set on first use).
-template <class T, int SP, bool TC>
+template <class T, int SP, bool TC, int PART = PART_ALL>
 int launch_dag(const ExecParams &p, int grid, cudaStream_t s) {
     static bool attr = false;
     if (!attr) {
-        CHB_CUDA(cudaFuncSetAttribute(cholesky_dag_kernel<T, SP, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CHB_CUDA(cudaFuncSetAttribute(cholesky_dag_kernel<T, SP, TC, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)dag_smem_bytes<T, SP, TC>()));
         attr = true;
     }
-    cholesky_dag_kernel<T, SP, TC><<<grid, NT_CTA, dag_smem_bytes<T, SP, TC>(), s>>>(p);
+    cholesky_dag_kernel<T, SP, TC, PART><<<grid, NT_CTA, dag_smem_bytes<T, SP, TC>(), s>>>(p);
     CHB_CUDA(cudaGetLastError());
     return 0;
 }
