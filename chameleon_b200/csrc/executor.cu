@@ -77,9 +77,36 @@ struct Coarse {
     bool virt = false;           // model-only task: runs on the copy engine, not on a CTA
     int nsub;
     double dur;               // duration of one sub-task (model units)
-    std::vector<int> succ;
+    int head = -1, tail = -1; // successors: first and last entry of Graph::e
     int npred = 0;
     double blevel = 0;
+};
+
+// A coarse DAG.  The successor lists are chains in one array: a vector in every
+// task made building the list of an order of 32768 half as long again.
+struct Graph {
+    std::vector<Coarse> t;
+    std::vector<std::pair<int, int>> e;   // successor, next entry
+    size_t size() const { return t.size(); }
+    Coarse &operator[](int i) { return t[i]; }
+    int add(int kind, int m, int n, int k, int bn, int nsub, double dur) {
+        Coarse c;
+        c.kind = kind; c.m = m; c.n = n; c.k = k; c.bn = bn; c.grp = 0; c.nsub = nsub; c.dur = dur;
+        t.push_back(c);
+        return (int)t.size() - 1;
+    }
+    void edge(int a, int b) {
+        if (a < 0 || b < 0 || a == b) return;
+        const int i = (int)e.size();
+        e.push_back({b, -1});
+        (t[a].tail < 0 ? t[a].head : e[t[a].tail].second) = i;
+        t[a].tail = i;
+        t[b].npred++;
+    }
+    template <class F>
+    void succ(int i, F &&f) const {
+        for (int j = t[i].head; j >= 0; j = e[j].second) f(e[j].first);
+    }
 };
 
 struct Schedule {
@@ -90,7 +117,7 @@ struct Schedule {
 };
 
 template <class NBU>
-std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBU nbu);
+std::vector<Task> list_schedule(Graph &ct, int P, NBU nbu);
 
 std::vector<Task> build_order(const Shape &s) {
     const int NT = (s.N + s.NB - 1) / s.NB;
@@ -109,19 +136,13 @@ std::vector<Task> build_order(const Shape &s) {
     // the updates are all but all of a factorization's tasks
     size_t count = (size_t)2 * NT * NT + (size_t)NTB * NT * (NT + 1);
     for (int n = 0; fact && n < NT; ++n) count += (size_t)upd_ngroups(n, s.G, s.tail) * (NT - n);
-    std::vector<Coarse> ct;
-    ct.reserve(count);
+    Graph ct;
+    ct.t.reserve(count);
+    ct.e.reserve(4 * count);
     auto add = [&](int kind, int m, int n, int k, int bn, int nsub, double dur) {
-        Coarse c;
-        c.kind = kind; c.m = m; c.n = n; c.k = k; c.bn = bn; c.grp = 0; c.nsub = nsub; c.dur = dur;
-        ct.push_back(c);
-        return (int)ct.size() - 1;
+        return ct.add(kind, m, n, k, bn, nsub, dur);
     };
-    auto edge = [&](int a, int b) {
-        if (a < 0 || b < 0) return;
-        ct[a].succ.push_back(b);
-        ct[b].npred++;
-    };
+    auto edge = [&](int a, int b) { ct.edge(a, b); };
     // ids: potrf[k], trsm[m,k], upd[m,n,k] (last update of tile (m,n) so far)
     std::vector<int> P(NT, -1), XI(NT, -1), Tr((size_t)NT * NT, -1), lastU((size_t)NT * NT, -1);
     std::vector<int> Cst((size_t)NT * NT, -1);   // MODE_CAST: cast task of tile (m, n)
@@ -271,11 +292,11 @@ std::vector<Task> build_order(const Shape &s) {
 // workers with critical-path priorities; emits the sub-tasks in start order.
 // nbu(m, cnt): row blocks of tile m in an update of cnt panels.
 template <class NBU>
-std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBU nbu) {
+std::vector<Task> list_schedule(Graph &ct, int P, NBU nbu) {
     // bottom levels (generation order is topological)
     for (int i = (int)ct.size() - 1; i >= 0; --i) {
         double b = 0;
-        for (int sidx : ct[i].succ) b = std::max(b, ct[sidx].blevel);
+        ct.succ(i, [&](int j) { b = std::max(b, ct[j].blevel); });
         ct[i].blevel = b + ct[i].dur;
     }
     // list scheduling on s.P workers
@@ -300,7 +321,7 @@ std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBU nbu) {
         if (ct[i].npred == 0) make_ready(i);
     std::vector<Task> out;
     size_t total = 0;
-    for (auto &c : ct)
+    for (auto &c : ct.t)
         if (!c.virt) total += c.nsub;
     out.reserve(total);
     int free_w = P;
@@ -340,10 +361,10 @@ std::vector<Task> list_schedule(std::vector<Coarse> &ct, int P, NBU nbu) {
         running.pop();
         now = f.t;
         if (!ct[f.id].virt) ++free_w;
-        if (++finished[f.id] == ct[f.id].nsub) {
-            for (int sidx : ct[f.id].succ)
-                if (--ct[sidx].npred == 0) make_ready(sidx);
-        }
+        if (++finished[f.id] == ct[f.id].nsub)
+            ct.succ(f.id, [&](int j) {
+                if (--ct[j].npred == 0) make_ready(j);
+            });
     }
     return out;
 }
@@ -1221,22 +1242,15 @@ static int dag_to_tasks(const cham_b200_dag_s &dag, int N, int NB, int nrhs, int
     auto nbi = [&](int m) { return (tm(m) + SUBB - 1) / SUBB; };
     int mode = 0;
     for (auto &r : dag.rec) mode |= (r[0] <= TK_UPD) ? MODE_FACT : MODE_SOLVE;
-    std::vector<Coarse> ct;
+    Graph ct;
     // tile ids: A (m, n) -> m + NT n; B (m, bn) -> NT NT + m + NT bn
     const size_t ntile = (size_t)NT * NT + (size_t)NT * std::max(NTB, 1);
     std::vector<int> last_w(ntile, -1);
     std::vector<std::vector<int>> readers(ntile);
     auto add = [&](int kind, int m, int n, int k, int bn, int nsub, double dur) {
-        Coarse c;
-        c.kind = kind; c.m = m; c.n = n; c.k = k; c.bn = bn; c.grp = 0; c.nsub = nsub; c.dur = dur;
-        ct.push_back(c);
-        return (int)ct.size() - 1;
+        return ct.add(kind, m, n, k, bn, nsub, dur);
     };
-    auto edge = [&](int a, int b) {
-        if (a < 0 || b < 0 || a == b) return;
-        ct[a].succ.push_back(b);
-        ct[b].npred++;
-    };
+    auto edge = [&](int a, int b) { ct.edge(a, b); };
     auto rd = [&](size_t tile, int id) {
         edge(last_w[tile], id);
         readers[tile].push_back(id);
