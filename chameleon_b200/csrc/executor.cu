@@ -504,15 +504,16 @@ static int exec_tile(const Tiling &A, const Tiling *B) {
     return nb;
 }
 
-// Panels per trailing update of the FP64 executor: a depth of n / 16, at least
-// 512 and at most the configured group (given in tiles of 512).  A deeper
-// group amortizes the C round trip, but a tile's last group only becomes ready
-// a few steps before the tile is factored, and a 128 x 128 x 4096 update takes
-// 0.8 ms on a CTA: order 8192 with depth 4096 21.0 ms, 1024 10.0, 512 9.8,
-// 256 10.4.
+// Panels per trailing update of the FP64 executor: a depth of n / 16 (n / 8 from
+// order 20480 on), at least 512 and at most the configured group (given in tiles
+// of 512).  A deeper group amortizes the C round trip, but a tile's last group only
+// becomes ready a few steps before the tile is factored, and a 128 x 128 x 4096
+// update takes 0.8 ms on a CTA: order 8192 with depth 4096 21.0 ms, 1024 10.0, 512
+// 9.8, 256 10.4; order 24576 with 1536 178.3, 3072 176.1; 32768 with 2048 410.2,
+// 4096 406.2.
 constexpr int GROUP_NB = 512;
 static int group_f64(int N, int NB, int kgroup) {
-    const int depth = std::min(kgroup * GROUP_NB, std::max(512, N / 16));
+    const int depth = std::min(kgroup * GROUP_NB, std::max(512, N / (N < 20480 ? 16 : 8)));
     return std::max(1, depth / NB);
 }
 
