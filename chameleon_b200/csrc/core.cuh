@@ -233,9 +233,9 @@ struct GemmCfg {
     static_assert(WM * WN * 32 == NT_CTA, "8 warps");
     static_assert(FM >= 1 && FN >= 1, "warp tile too small");
     static constexpr int SA = stage_elems_max<T_, BM>(), SB = stage_elems_max<T_, BN>();
-    // cp.async pipeline depth (2 in the executor kernel: deeper pipelines
-    // measured slower there, and FP64 tiles would not fit more; standalone
-    // long-K kernels such as the residual use 3)
+    // cp.async pipeline depth: 2 for the executor's updates and panel solves (more
+    // measured slower there, and FP64 tiles would not fit it), 3 to 5 for its short
+    // substitution products, 3 or 4 in kernels of 64- and 32-wide blocks
     static constexpr int ST = ST_;
     static constexpr int SMEM_ELEMS = ST * (SA + SB);
     static constexpr size_t SMEM_BYTES = sizeof(T_) * SMEM_ELEMS;

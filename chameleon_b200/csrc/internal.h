@@ -126,7 +126,7 @@ int stage_out(double *host, int ld, const double *dev, int rows, int cols, cudaS
 struct ExecWs {
     uint8_t *split = nullptr;
     size_t split_bytes = 0;
-    void *xinv = nullptr;               // full inverses of the diagonal tiles (FP32 solves)
+    void *xinv = nullptr;               // full inverses of the diagonal tiles (FP64: and scratch)
     size_t xinv_bytes = 0;
     const void *xinv_owner = nullptr;   // factor storage the inverses belong to (nullptr: none)
     int xinv_n = 0, xinv_nt = 0, xinv_nb = 0;

@@ -21,7 +21,9 @@
 //
 // Using the explicit inverse of a whole tile trades the backward stability of
 // a substitution for fewer dependent steps; the mixed-precision solver runs it
-// in FP32 and its FP64 refinement restores the FP64 backward error.
+// in FP32 and its FP64 refinement restores the FP64 backward error.  The FP64
+// substitutions, which nothing refines, use full inverses of well-conditioned
+// tiles only (XINV_COND, executor.cuh).
 #pragma once
 #include "core.cuh"
 

@@ -332,7 +332,9 @@ int CUDA_spotrf(cham_uplo_t uplo, int n, float *A, int lda, float *WORK, int lwo
  * memory, so n <= 1024 (larger n returns CHAMELEON_ERR_INTERNAL_LIMIT); all
  * calls on a device share that array, so calls that could overlap on the GPU
  * must not be issued.  The first call on a device does a one-time set-up and
- * should come before any stream capture.  Same result and `info` as CUDA_dpotrf. */
+ * should come before any stream capture.  Same `info` as CUDA_dpotrf and the same
+ * factor up to rounding (above order 128 CUDA_dpotrf sums in another order, on many
+ * CTAs). */
 int CUDA_dpotrf_noalloc(cham_uplo_t uplo, int n, double *A, int lda, int *d_info, void *cuda_stream);
 int CUDA_dplgsy(const double *bump, int m, int n, double *A, int lda, int bigM, int m0, int n0,
                 unsigned long long int seed, cublasHandle_t handle);
