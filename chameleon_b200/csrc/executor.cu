@@ -776,8 +776,9 @@ static int plan_call(Plan (&q)[2], WsBytes &ws, int mode, int N, bool f32, const
     // forward sweep runs beside it (1 to 17 right-hand sides, dposv 203: 232 us in
     // one launch, 256 in two; 2048: 1.70 and 1.73 ms; 5003: 6.16 and 5.95 ms),
     // unless B outweighs the factorization (2048 with 16384 columns 9.4 and 8.0
-    // ms; the line could lie lower: 3000 with 512 takes 8.4 in one, 3200 3.2 in two).
-    const bool own = (mode & MODE_FACT) ? N > 3072 || b_elems > OWN_ELEMS : N > EXEC_NB;
+    // ms; the line could lie lower: 3000 with 512 takes 8.4 in one, 3200 3.2 in two)
+    // and there are more than two tiles (100 with 4e5 columns 1.20 and 1.47 ms).
+    const bool own = (mode & MODE_FACT) ? N > 3072 || (N > 2 * EXEC_NB && b_elems > OWN_ELEMS) : N > EXEC_NB;
     int xnb = (!f32 && !t_given && nrhs > 0 && own && !small) ? solve_tile(N, A, *B) : 0;
     if (xnb > 0) {
         const int wide = wide_tile(A, *B);

@@ -119,3 +119,10 @@ assert L.CHAM_B200_Schedule_Size(1 | 32, 65536, 128, 0, 128, 296, 0, 32) > 0
 """
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     subprocess.run([sys.executable, "-c", code], cwd=root, check=True, timeout=300)
+
+
+@pytest.mark.parametrize("n,nrhs,launches", [(100, 400001, 1), (256, 150000, 1), (500, 70000, 2), (2048, 16385, 2),
+                                             (2048, 64, 1), (3073, 1, 2)])
+def test_launches_of_a_solve(n, nrhs, launches):
+    """Two where B outweighs the factorization of more than two tiles, or above 3072."""
+    assert len(plan(FACT | SOLVE, n, 384, nrhs, array=True)[0]) == launches
