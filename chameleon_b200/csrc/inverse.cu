@@ -57,7 +57,7 @@ struct InvState {
     __host__ __device__ bool ill() const { return !(norm[0] * norm[1] <= INV_COND); }
     __host__ __device__ bool usable() const { return first == INT_MAX && !ill(); }
 };
-constexpr int NORM_ROWS = 16;   // rows per CTA of the norms: 157 CTAs at order 2500
+constexpr int NORM_ROWS = 4;   // rows per CTA of the norms (a row is a chain of loads: 64 threads each)
 
 // The inverted HB x HB diagonal blocks of the lower L (n x n), one CTA each, at
 // X + q step (column-major, ld ldx); unit: with an implied unit diagonal.
