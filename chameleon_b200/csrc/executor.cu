@@ -810,10 +810,11 @@ static int enqueue_all(int n, Step step, Drain drain) {
 
 // Enqueue one launch of the executor; the workspace holds what the plan needs
 // and the descriptors are uploaded.  st: its state, initialized by the caller;
-// after: state of an earlier launch that must not have failed.
+// after: state of an earlier launch that must not have failed; trace_at: where its
+// trace records start, after those of an earlier launch.
 static int enqueue_dag(const Plan &q, const Schedule *sch, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
                        cudaStream_t s, int split, ExecWs &w, const CastIn *cin, ExecState *st,
-                       const ExecState *after) {
+                       const ExecState *after, int trace_at) {
     Context &c = ctx();
     const int N = q.N, NB = q.NB, NT = q.NT, nrhs = q.nrhs, NTB = q.NTB;
     int rc = 0;
@@ -876,7 +877,7 @@ static int enqueue_dag(const Plan &q, const Schedule *sch, cham_uplo_t uplo, CHA
     }
     p.st = st;
     p.after = after;
-    p.trace = (g_trace_buf && g_trace_cap >= p.ntasks) ? g_trace_buf : nullptr;
+    p.trace = (g_trace_buf && g_trace_cap - trace_at >= p.ntasks) ? g_trace_buf + trace_at : nullptr;
     p.wait_budget_ns = (unsigned long long)c.wait_budget_us * 1000ull;
     p.kgroup = q.G;
     p.utail = q.sh.tail;
@@ -949,7 +950,7 @@ int run_cholesky_dag(int mode, cham_uplo_t uplo, CHAM_desc_t *A, CHAM_desc_t *B,
             }
             if (i <= nq)
                 return enqueue_dag(q[i - 1], sch[i - 1], uplo, A, B, s, split, w, cin, w.st + i - 1,
-                                   i > 1 ? w.st : nullptr);
+                                   i > 1 ? w.st : nullptr, i > 1 ? (int)sch[0]->tasks.size() : 0);
             CHB_CUDA(cudaEventRecord(w.e1, s));
             CHB_CUDA(cudaMemcpyAsync(out, w.st, sizeof(out), cudaMemcpyDeviceToHost, s));
             return 0;

@@ -255,3 +255,25 @@ def test_two_launches_over_tilings(cb, layout, uplo, n, nb, nrhs):
         X = b[:, :n]
         r = float(torch.linalg.norm(X @ S - B) / (torch.linalg.norm(S) * torch.linalg.norm(X)))
         assert r <= 8 * n * EPS, (step, r)
+
+
+def test_trace_holds_both_launches(cb):
+    """The substitutions' records follow the factorization's."""
+    rec = np.dtype([("task", "<i4"), ("smid", "<i4"), ("t0", "<u8"), ("t1", "<u8"), ("wait", "<u4"), ("ph", "<u4", 3)])
+    n, cap, L = 3100, 40000, cb.lib()
+    dA, dB = cb.Desc.create(n, n, 512), cb.Desc.create(n, 5, 512)
+    dA.from_numpy(n * np.eye(n))
+    dB.from_numpy(np.ones((n, 5)))
+    assert L.CHAM_B200_Trace_Enable(cap) == 0
+    try:
+        assert cb.dposv_Tile(LOWER, dA, dB) == 0
+        out = np.zeros(cap, rec)
+        assert L.CHAM_B200_Trace_Read(out.ctypes.data_as(ctypes.c_void_p), cap) == 0
+    finally:
+        L.CHAM_B200_Trace_Enable(0)
+    used = int((out["t1"] > 0).sum())
+    starts = np.flatnonzero(out["task"][:used] == 0)
+    assert (out["t1"][:used] > 0).all() and len(starts) == 2, used
+    k = int(starts[1])
+    assert np.array_equal(out["task"][:k], np.arange(k)) and np.array_equal(out["task"][k:used], np.arange(used - k))
+    assert out["t1"][:k].max() <= out["t0"][k:used].min()
